@@ -112,6 +112,7 @@ PROTOTYPES = {
 }
 
 _lib = None
+_binding = None
 
 
 def lib() -> ctypes.CDLL:
@@ -129,6 +130,22 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+def torch_binding():
+    """The CPython extension (csrc/torch_binding.cpp) that the device-tensor wrappers call first: its functions
+    return None for a call they do not cover, which the wrapper then handles itself.  Raises if it has not been built."""
+    global _binding
+    if _binding is None:
+        lib()
+        try:
+            import torch  # noqa: F401  the extension uses torch's libraries
+            from . import _torch_binding
+        except ImportError as e:
+            raise RuntimeError(f"{PKG_DIR}/_torch_binding.so cannot be loaded ({e}): build it with "
+                               "`python -m rustorch_b200.build`") from e
+        _binding = _torch_binding
+    return _binding
 
 
 def error_string(status: int) -> str:

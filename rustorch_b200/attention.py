@@ -192,6 +192,9 @@ def _dense_view(t) -> bool:
     return True
 
 
+_MHA_BOUND = frozenset(("kv_lens", "key_keep", "scale", "return_lse", "q_offsets"))  # what the extension takes
+
+
 def mha_prefill_bf16(q, k, v, n_heads: int, n_kv_heads: Optional[int] = None, causal: bool = False, **kw):
     """Attention on activations in the layout the reference's modules keep them in: q [B,T,Hq*hd],
     k, v [B,S,Hkv*hd] bf16 CUDA tensors (crates/rustorch-nn/src/attention.rs:468-485 transposes them
@@ -199,6 +202,12 @@ def mha_prefill_bf16(q, k, v, n_heads: int, n_kv_heads: Optional[int] = None, ca
     repeats the KV heads).  The transposes and the repeat are folded into the TMA descriptors:
     returns (out [B,T,Hq*hd], lse [B,Hq,T]) without any full-tensor copy.
     """
+    if kw.keys() <= _MHA_BOUND:
+        r = (_lib._binding or _lib.torch_binding()).mha_prefill_bf16(
+            q, k, v, n_heads, n_kv_heads, causal, kw.get("kv_lens"), kw.get("key_keep"), kw.get("scale"),
+            kw.get("return_lse", True), kw.get("q_offsets"))
+        if r is not None:
+            return r
     n_kv_heads = n_heads if n_kv_heads is None else n_kv_heads
     B, T, E = q.shape
     S = k.shape[1]
@@ -225,6 +234,10 @@ def prefill_bf16(q, k, v, causal: bool = False, kv_lens=None, key_keep=None, sca
     when any of q, k, v, out is a strided view whose last dim is contiguous (e.g. a
     ``[B,T,H,hd]`` activation permuted to ``[B,H,T,hd]``): no transpose copy is made.
     """
+    r = (_lib._binding or _lib.torch_binding()).prefill_bf16(q, k, v, causal, kv_lens, key_keep, scale, out, lse, return_lse,
+                                                             q_offsets)
+    if r is not None:
+        return r
     import torch
     for name, t in (("q", q), ("k", k), ("v", v)):
         if not (t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 4):
@@ -285,6 +298,9 @@ def prefill_bf16(q, k, v, causal: bool = False, kv_lens=None, key_keep=None, sca
 def prefill_f32(q, k, v, causal: bool = False, kv_lens=None, key_keep=None, scale: Optional[float] = None,
                 q_offsets=None):
     """f32 CUDA-core forward on f32 CUDA tensors q [B,Hq,Nq,D], k/v [B,Hkv,Nkv,D] via ``rt_attn_prefill_f32``."""
+    r = (_lib._binding or _lib.torch_binding()).prefill_f32(q, k, v, causal, kv_lens, key_keep, scale, q_offsets)
+    if r is not None:
+        return r
     import torch
     B, Hq, Nq, D = q.shape
     _, Hkv, Nkv, _ = k.shape
@@ -309,6 +325,9 @@ def prefill_f32(q, k, v, causal: bool = False, kv_lens=None, key_keep=None, scal
 def backward_f32(q, k, v, out, d_out, lse, causal: bool = False, scale: Optional[float] = None):
     """(dq, dk, dv) on f32 CUDA tensors [B,H,N,D] via ``rt_attn_backward_f32``; ``out`` and ``lse`` are
     the results of ``prefill_f32`` on the same q, k, v, mask and scale."""
+    r = (_lib._binding or _lib.torch_binding()).backward_f32(q, k, v, out, d_out, lse, causal, scale)
+    if r is not None:
+        return r
     import torch
     B, H, N, D = q.shape
     for name, t in (("q", q), ("k", k), ("v", v), ("out", out), ("d_out", d_out)):
@@ -332,6 +351,9 @@ def backward_f32(q, k, v, out, d_out, lse, causal: bool = False, scale: Optional
 def backward_bf16(q, k, v, out, d_out, lse, causal: bool = False, scale: Optional[float] = None):
     """(dq, dk, dv) f32 from bf16 CUDA tensors [B,H,N,D] (D in {64,128}) via ``rt_attn_backward_bf16``;
     ``out`` and ``lse`` are the results of ``prefill_bf16`` on the same q, k, v, mask and scale."""
+    r = (_lib._binding or _lib.torch_binding()).backward_bf16(q, k, v, out, d_out, lse, causal, scale)
+    if r is not None:
+        return r
     import torch
     B, H, N, D = q.shape
     for name, t in (("q", q), ("k", k), ("v", v), ("out", out), ("d_out", d_out)):

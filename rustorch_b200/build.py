@@ -1,4 +1,5 @@
-"""Builds librustorch_attn.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds librustorch_attn.so (the C-ABI library) in-tree with nvcc for sm_100a, and _torch_binding.so, the
+CPython extension through which the Python wrappers call it.
 
     python -m rustorch_b200.build [--force] [--verbose]
 
@@ -16,6 +17,8 @@ import sys
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "librustorch_attn.so")
+BINDING_PATH = os.path.join(PKG_DIR, "_torch_binding.so")
+BINDING_SOURCE = os.path.join(CSRC, "torch_binding.cpp")
 SOURCES = ["api.cu", "decode.cu", "decode_tc.cu", "prefill_simt.cu", "prefill_tc.cu", "tc_selftest.cu", "decode_static.cu", "backward_simt.cu", "backward_tc.cu", "backward_tcgen05.cu"]
 
 NVCC_FLAGS = [
@@ -42,13 +45,37 @@ def needs_build() -> bool:
     if not os.path.exists(LIB_PATH):
         return True
     t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith(".cpp")] + [
         os.path.join(PKG_DIR, "..", "include", "rustorch_attn.h")]
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_binding(force: bool = False) -> str:
+    """g++ over torch_binding.cpp against torch's headers; linked to the C-ABI library next to it."""
+    header = os.path.join(PKG_DIR, "..", "include", "rustorch_attn.h")
+    if not force and os.path.exists(BINDING_PATH) and os.path.getmtime(BINDING_PATH) > max(
+            os.path.getmtime(BINDING_SOURCE), os.path.getmtime(header)):
+        return BINDING_PATH
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    cmd += [x for d in includes for x in ("-isystem", d)] + ["-o", BINDING_PATH, BINDING_SOURCE]
+    cmd += ["-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",
+            "-L" + PKG_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        sys.stderr.write(proc.stdout + proc.stderr)
+        raise RuntimeError("g++ failed building _torch_binding.so")
+    return BINDING_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
+        build_binding()
         return LIB_PATH
     cmd = [_nvcc()] + [f for f in NVCC_FLAGS if f != "--use_fast_math=false"]
     if verbose:
@@ -59,6 +86,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         sys.stderr.write(proc.stdout + proc.stderr)
     if proc.returncode != 0:
         raise RuntimeError("nvcc failed building librustorch_attn.so")
+    build_binding(force)
     return LIB_PATH
 
 

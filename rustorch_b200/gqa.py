@@ -204,6 +204,10 @@ def gqa_decode(q, k_cache, v_cache, kv_lens=None, kv_len: Optional[int] = None, 
     uniform ``kv_len``.  Returns (out [B,Hq,D] in ``out_dtype`` (bf16 default, or float32), lse or None).
     ``out`` / ``lse`` may be passed in (a decode loop reuses them: nothing is allocated per step).
     """
+    r = (_lib._binding or _lib.torch_binding()).gqa_decode(q, k_cache, v_cache, kv_lens, kv_len, kv_begin, kv_end, scale,
+                                                           out_dtype, return_lse, workspace, out, lse)
+    if r is not None:
+        return r
     import torch
     B, Hq, Hkv, D, max_seq = _guard_decode_args(q, k_cache, v_cache, kv_lens, workspace)
     if out is None:
@@ -327,9 +331,15 @@ def rope_inv_freq(head_dim: int, base: float = 10000.0, device="cuda"):
     return (1.0 / torch.pow(torch.tensor(float(base), dtype=torch.float32), 2.0 * k / head_dim)).to(device)
 
 
+_ROPE_STYLES = {"half_split": _lib.RT_ROPE_HALF_SPLIT, "adjacent": _lib.RT_ROPE_ADJACENT}
+
+
 def rope_kv_append(q, k_in, v_in, k_cache, v_cache, inv_freq, pos=None, positions=None, style: str = "half_split") -> None:
     """Rotary embedding of q (in place) and of the new K row + append of K, V at each sequence's position, one
     launch (``rt_rope_kv_append_bf16``).  q [B,Hq,D], k_in/v_in [B,Hkv,D], caches [B,Hkv,max_seq,D]."""
+    if (_lib._binding or _lib.torch_binding()).rope_kv_append(q, k_in, v_in, k_cache, v_cache, inv_freq, pos, positions,
+                                                              _ROPE_STYLES[style]):
+        return
     import torch
     B, Hq, Hkv, D, max_seq = _guard_decode_args(q, k_cache, v_cache)
     _guard("k_in", k_in, torch.bfloat16, like=q, shape=(B, Hkv, D))
@@ -341,6 +351,6 @@ def rope_kv_append(q, k_in, v_in, k_cache, v_cache, inv_freq, pos=None, position
                                            v_cache.data_ptr(), inv_freq.data_ptr(), B, Hq, Hkv, D, max_seq,
                                            0 if pos is None else int(pos),
                                            positions.data_ptr() if positions is not None else None,
-                                           {"half_split": _lib.RT_ROPE_HALF_SPLIT, "adjacent": _lib.RT_ROPE_ADJACENT}[style],
+                                           _ROPE_STYLES[style],
                                            _stream_ptr())
     _lib.check(rc, "rt_rope_kv_append_bf16")
