@@ -56,7 +56,7 @@ struct TcCfg {
     // (batch, query block) pairs the length-sorted schedule can hold (two uint16 per pair); what is left of
     // the 227 KB of shared memory at D = 128 bounds it there
     static constexpr int SCHED_CAP = (D == 128) ? 384 : 2048;
-    static constexpr int SMEM_BYTES = (2 + KS + VS) * TILE_BYTES + NBARS * 8 + 16 + 4 * SCHED_CAP + 1024;
+    static constexpr int SMEM_BYTES = (2 + KS + VS) * TILE_BYTES + NBARS * 8 + 48 + 4 * SCHED_CAP + 1024;
     static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB of shared memory a CTA can opt into");
     static constexpr uint32_t TMEM_COLS = 512;
     static constexpr uint32_t COL_S = 0, COL_O = 256;   // S: tile w, buffer b at COL_S + w*128 + b*64
@@ -79,6 +79,7 @@ struct TcParams {
     int sorted;        // length-sorted schedule (launches with per-batch kv_lens), see tc_item
     int stagger_clocks;  // single-tile items: head start of tile 0 over tile 1, in SM clocks
     int direct_out;    // one item per CTA: the epilogue stores its rows straight from registers (no staged tile, no TMA store)
+    int tighten;       // key_keep launches of one item per CTA: trailing hidden keys are found at start-up and not visited
     int single_tile;   // items are 128-row blocks whose 64-key steps alternate between the two tiles (small launches, see tc_item)
 };
 
@@ -144,11 +145,12 @@ struct TcItem {
 // pair side by side, and it is dealt to the CTAs boustrophedon (0..G-1, G-1..0, ...), heaviest first: the
 // persistent kernel's overlap of one item's set-up with the previous item's tail, and a balanced finish.
 template <bool kCausal, bool kSingle>
-__device__ __forceinline__ void tc_steps(const TcParams& p, int b, int q0, int& kv_hi, int& q_off, int& U0, int& U1) {
-    kv_hi = p.seq_kv;
+__device__ __forceinline__ void tc_steps(const TcParams& p, int b, int q0, int& kv_hi, int& q_off, int& U0, int& U1,
+                                         int keep_hi = 0x7fffffff) {
+    kv_hi = min(p.seq_kv, keep_hi);
     if (p.kv_lens) {
         const int l = p.kv_lens[b];
-        kv_hi = l < 0 ? 0 : (l < p.seq_kv ? l : p.seq_kv);
+        kv_hi = l < 0 ? 0 : (l < kv_hi ? l : kv_hi);
     }
     q_off = p.q_offsets ? p.q_offsets[b] : 0;   // query row i sits at key position i + q_off
     const int n_steps = (kv_hi + 63) / 64;      // 64-key steps that hold a visible key
@@ -162,7 +164,7 @@ __device__ __forceinline__ void tc_steps(const TcParams& p, int b, int q0, int& 
 }
 
 template <bool kCausal, bool kSingle>
-__device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16_t* sched) {
+__device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16_t* sched, int keep_hi = 0x7fffffff) {
     TcItem it;
     it.valid = false;
     int qb;
@@ -196,7 +198,7 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
     // Single-tile items: block qb covers rows [128 qb, 128 qb + 128); the item's origin is kept 128 rows
     // earlier so that the block sits where tile 1 sits in a two-tile item (TcItem::qrow).
     it.q0 = kSingle ? qb * 128 - 128 : qb * 256;
-    tc_steps<kCausal, kSingle>(p, it.b, it.q0, it.kv_hi, it.q_off, it.U0, it.U1);
+    tc_steps<kCausal, kSingle>(p, it.b, it.q0, it.kv_hi, it.q_off, it.U0, it.U1, keep_hi);
     it.n_tiles = kSingle ? it.U0 : (it.U1 + 1) / 2;
     return it;
 }
@@ -240,7 +242,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     uint64_t* done_bar = stage_full + 2;  // [1]
     uint64_t* merge_bar = done_bar + 1;   // [1]  single-tile items: both tiles have published their (max, sum)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(merge_bar + 1);
-    uint16_t* sched = reinterpret_cast<uint16_t*>(tmem_slot + 4);  // [SCHED_CAP] pair order, then [SCHED_CAP] step counts
+    uint16_t* sched = reinterpret_cast<uint16_t*>(tmem_slot + 12);  // (after 8 words of the keep-flag scan) [SCHED_CAP] pair order, then [SCHED_CAP] step counts
 
     // Broadcasting the warp index makes it provably warp-uniform, so role dispatch and the MMA
     // operands stay on the uniform datapath.
@@ -336,10 +338,30 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
     }
+    if (kKeep && p.tighten) {
+        // Keep flags mostly hide the tail of a sequence (its padding): the last kept key bounds the keys this CTA's
+        // only item visits.  At least one key stays, so that an item has steps here exactly if it has them without
+        // the bound (the preload above relies on that); a row that sees no kept key is recognised as before.
+        grid_dep_wait();
+        if (warp < 8) {
+            const uint8_t* keep = p.key_keep + (int64_t)(((int)blockIdx.x / p.slots_per_head) / p.heads) * p.keep_batch_stride;
+            int hi = 1;
+            for (int i = threadIdx.x; i < Nkv; i += 256)
+                if (__ldg(keep + i)) hi = i + 1;
+            hi = __reduce_max_sync(kFullMask, hi);
+            if (lane == 0) reinterpret_cast<int*>(tmem_slot + 4)[warp] = hi;
+        }
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    int keep_hi = 0x7fffffff;
+    if (kKeep && p.tighten) {
+        keep_hi = 1;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) keep_hi = max(keep_hi, reinterpret_cast<const int*>(tmem_slot + 4)[i]);
+    }
     grid_dep_wait();
     // The next kernel of the stream may be scheduled as SMs fall free (it waits as above before it reads or
     // writes anything): its launch latency and set-up hide behind the tail of this grid.
@@ -355,7 +377,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             // A single-tile item is its CTA's only item; Q and K tile 0 were requested during setup.  Each
             // issuer reads every tile once and asks for K tile u + 2 right after the PV of step u, so K runs
             // two tiles ahead of V in the request order: K1 | K2 V0 | K3 V1 | ...
-            const TcItem it = tc_item<kCausal, kSingle>(0, p, sched);
+            const TcItem it = tc_item<kCausal, kSingle>(0, p, sched, keep_hi);
             if (first_preloaded) {
                 bool ok = true;
                 int kg = 1, vg = 0;
@@ -398,7 +420,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             int na0 = 0, na1 = 0;  // items so far in which tile w took part (phase of its per-item barriers)
             bool ok = true;
             for (int j = 0; ok; ++j) {
-                const TcItem it = tc_item<kCausal, kSingle>(j, p, sched);
+                const TcItem it = tc_item<kCausal, kSingle>(j, p, sched, keep_hi);
                 if (it.end) break;
                 if (!it.valid || it.n_tiles == 0) continue;  // nothing to load
                 auto load_q = [&](int w, int na) {
@@ -487,7 +509,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             };
             bool ok = true;
             for (int j = 0; ok; ++j) {
-                const TcItem it = tc_item<kCausal, kSingle>(j, p, sched);
+                const TcItem it = tc_item<kCausal, kSingle>(j, p, sched, keep_hi);
                 if (it.end) break;
                 if (!it.valid || it.n_tiles == 0) continue;
                 const int n_u = it.steps(w);
@@ -598,7 +620,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         bool ok = true;
 
         for (int j = 0; ok; ++j) {
-            const TcItem it = tc_item<kCausal, kSingle>(j, p, sched);
+            const TcItem it = tc_item<kCausal, kSingle>(j, p, sched, keep_hi);
             if (it.end) break;
             if (!it.valid) continue;
             const int n_iter = it.steps(w);
@@ -625,6 +647,17 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             bool seen = false;  // the row has met a score that no mask hides
             for (int u = 0; u < n_iter; ++u) {
                 const int buf = u & 1;
+                const int col0 = (il ? 2 * u + w : u) * 64;
+                uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;
+                if (kKeep) {
+                    // Mask::Padding keep flags (mask.rs:44) of the step's 64 keys as two 32-bit words: each lane reads
+                    // two flags, issued before the wait for the scores so that their latency hides behind it.  (One
+                    // flag load per key in every thread, as this replaces, cost 6 x the rest of the step.)
+                    const int k0 = col0 + lane, k1 = k0 + 32;
+                    const bool f0 = k0 >= Nkv || __ldg(keep + k0) != 0, f1 = k1 >= Nkv || __ldg(keep + k1) != 0;
+                    keep0 = __ballot_sync(kFullMask, f0);
+                    keep1 = __ballot_sync(kFullMask, f1);
+                }
                 if (!__all_sync(kFullMask, mbar_wait(&s_full[w * 2 + buf], (uint32_t)((buf ? cs1 : cs0) + (u >> 1)) & 1u,
                                                      p.status, kToSFull))) {
                     ok = false;
@@ -650,7 +683,6 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 }
 
                 // ---- masks: keys beyond kv_hi, causal diagonal, keep flags
-                const int col0 = (il ? 2 * u + w : u) * 64;
                 int lim = kv_hi - 1 - col0;                       // last visible column in this step
                 if (kCausal) lim = min(lim, row + q_off - col0);
                 if (lim < 63) {
@@ -658,10 +690,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     for (int i = 0; i < 64; ++i)
                         if (i > lim) s[i] = 0xff800000u;  // -inf
                 }
-                if (kKeep) {  // Mask::Padding keep flags (mask.rs:44); every thread reads the same bytes
+                if (kKeep && (keep0 & keep1) != 0xffffffffu) {
 #pragma unroll
-                    for (int i = 0; i < 64; ++i)
-                        if (col0 + i < Nkv && __ldg(keep + col0 + i) == 0) s[i] = 0xff800000u;
+                    for (int i = 0; i < 32; ++i) {
+                        if (!(keep0 & (1u << i))) s[i] = 0xff800000u;
+                        if (!(keep1 & (1u << i))) s[32 + i] = 0xff800000u;
+                    }
                 }
 
                 // ---- row max (three-input max halves the instruction count)
@@ -1107,6 +1141,7 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
     const int64_t n_ctas = (persistent && p.n_slots > n_sm) ? n_sm : p.n_slots;
     p.direct_out = (n_ctas == p.n_slots && !p.paired && !p.sorted) ? 1 : 0;  // every CTA has exactly one item
     const bool keep = key_keep != nullptr;
+    p.tighten = (keep && p.direct_out && seq_kv > 0) ? 1 : 0;
 #define RT_TC_DISPATCH(DD)                                                                         \
     if (causal) {                                                                                  \
         return keep ? launch_tc<DD, true, true>(mq, mk, mv, mo, p, n_ctas, stream)                     \
