@@ -6,18 +6,15 @@
 //   P = exp(scale * Q K^T - LSE),  dV = P^T dO,  dP = dO V^T,
 //   dS = P o (dP - delta),  delta_i = sum_j P_ij dP_ij = dO_i . O_i,
 //   dQ = scale * dS K,  dK = scale * dS^T Q
-// evaluated tile by tile, so nothing of size N x N is stored.  Two deterministic passes (no
-// atomics): one warp per query row accumulates dQ_i over key tiles, then one warp per key row
-// accumulates dK_j and dV_j over query tiles; each pass recomputes the scores it needs.  The lane
-// index runs over the 32 rows of the opposite tile, which sit in shared memory with a padded
-// pitch.  A causal launch skips the tiles above the diagonal.
+// evaluated tile by tile, so nothing of size N x N is stored.  Deterministic, without atomics: a CTA owns 64 query
+// rows and accumulates dQ over the key tiles, or owns 64 key rows and accumulates dK and dV over the query tiles
+// (recomputing S and dP).  Both kinds run in one launch, so that one side's long rows fill the other side's tail.
+// The products are the register-tiled ones of simt_tile.cuh.  A causal launch skips the tiles above the diagonal.
 #include "common.cuh"
 #include "kernels.h"
+#include "simt_tile.cuh"
 
 namespace rt {
-
-constexpr int kBwdRows = 8;    // rows (warps) per CTA
-constexpr int kBwdTile = 32;   // rows of the opposite operand per tile (one per lane)
 
 struct BwdParams {
     const float *q, *k, *v, *out, *d_out, *lse;
@@ -40,135 +37,182 @@ __global__ void __launch_bounds__(256) bwd_delta_kernel(const float* __restrict_
     if (lane == 0) delta[row] = acc;
 }
 
-// Pass over the rows of one side (kQuerySide: a warp owns query row i and walks key tiles to form
-// dQ_i; otherwise it owns key row j and walks query tiles to form dK_j and dV_j).
-template <bool kQuerySide>
-__global__ void __launch_bounds__(kBwdRows * 32) bwd_pass_kernel(const BwdParams p) {
-    extern __shared__ float smem[];
+// One CTA's 64 rows of one side.  X1, X2 are its own rows of (Q, dO) or (K, V), Y1, Y2 the other side's tiles of
+// (K, V) or (Q, dO), 16 J rows at a time; col0 is the first of the NC x 32 gradient columns it accumulates.
+// Every step computes dP (Y2) before S (Y1) and accumulates with Y2 before Y1, so each single-buffered tile is
+// copied while a product that does not need it runs.  With G = 2 groups each takes every second tile of the other
+// side, with buffers and sums of its own; the first adds the second's sums at the end.
+template <int NC, int J, int G, bool kKeySide>
+__device__ __forceinline__ void bwd_rows(const BwdParams& p, float* smem, int64_t bh, int64_t own0, int col0, bool vec,
+                                         bool pairs) {
+    using namespace simt;
     const int D = p.dim;
-    const int P1 = D + 1;
-    float* tA = smem;                        // [32][D+1]  K tile (query side) / Q tile (key side)
-    float* tB = tA + kBwdTile * P1;          // [32][D+1]  V tile               / dO tile
-    float* rA = tB + kBwdTile * P1;          // [rows][D]  Q rows               / K rows
-    float* rB = rA + kBwdRows * D;           // [rows][D]  dO rows              / V rows
-    float* tLse = rB + kBwdRows * D;         // [32]  (key side) LSE of the tile's query rows
-    float* tDelta = tLse + kBwdTile;         // [32]  (key side) delta of the tile's query rows
+    const int group = G == 1 ? 0 : (int)threadIdx.x >> 7, tid = (int)threadIdx.x & (kGroup - 1);
+    const int x_tile = tile_floats(kRows, D), y_tile = tile_floats(16 * J, D);
+    float* X1 = smem;
+    float* X2 = X1 + x_tile;
+    float* Y1 = X2 + x_tile + group * (2 * y_tile + kWFloats);
+    float* Y2 = Y1 + y_tile;
+    float* Ws = Y2 + y_tile;
+    const Lane ln;
+    const Share share = Share::of<kGroup>(tid, D, vec), x_share = Share::of<kGroup * G>((int)threadIdx.x, D, vec);
+    const int64_t N = p.seq, base = bh * N * D;
+    const float* lse = p.lse + bh * N;
+    const float* delta = p.delta + bh * N;
+    const float* oth1 = (kKeySide ? p.q : p.k) + base;
+    const float* oth2 = (kKeySide ? p.d_out : p.v) + base;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t bh = blockIdx.y;
-    const int64_t N = p.seq;
-    const int64_t row0 = (int64_t)blockIdx.x * kBwdRows;
-    const int64_t r = row0 + warp;           // the row this warp owns
-    const bool row_valid = r < N;
-    const int64_t base = bh * N * D;
+    // the other side's rows that the own rows meet: keys up to the last own query, queries from the first own key on
+    const int64_t t_lo = (kKeySide && p.causal) ? own0 / (16 * J) * (16 * J) : 0;
+    const int64_t t_hi = (!kKeySide && p.causal && own0 + kRows < N) ? own0 + kRows : N;
 
-    const float* ownA = (kQuerySide ? p.q : p.k) + base;
-    const float* ownB = (kQuerySide ? p.d_out : p.v) + base;
-    const float* othA = (kQuerySide ? p.k : p.q) + base;
-    const float* othB = (kQuerySide ? p.v : p.d_out) + base;
+    const int64_t first = t_lo + group * 16 * J, step = (int64_t)G * 16 * J;
+    load_tile<kRows, kGroup * G>(X1, (kKeySide ? p.k : p.q) + base, own0, N, D, vec, x_share);
+    load_tile<kRows, kGroup * G>(X2, (kKeySide ? p.v : p.d_out) + base, own0, N, D, vec, x_share);
+    if (first < t_hi) load_tile<16 * J, kGroup>(Y2, oth2, first, N, D, vec, share);
+    cp_async_commit();
 
-    for (int i = threadIdx.x; i < kBwdRows * D; i += blockDim.x) {
-        const int64_t rr = row0 + i / D;
-        rA[i] = rr < N ? ownA[rr * D + i % D] : 0.f;
-        rB[i] = rr < N ? ownB[rr * D + i % D] : 0.f;
-    }
-    float own_lse = 0.f, own_delta = 0.f;
-    if (kQuerySide && row_valid) {
-        own_lse = p.lse[bh * N + r];
-        own_delta = p.delta[bh * N + r];
-    }
-
-    // tile range of the opposite side that this CTA's rows can see / be seen by
-    int64_t t_lo = 0, t_hi = N;
-    if (p.causal) {
-        if (kQuerySide) {
-            t_hi = row0 + kBwdRows < N ? row0 + kBwdRows : N;  // keys <= last query row of the CTA
-        } else {
-            t_lo = (row0 / kBwdTile) * kBwdTile;               // queries >= first key row of the CTA
-        }
-    }
-
-    float acc0[8], acc1[8];  // query side: dQ_i; key side: dK_j (acc0) and dV_j (acc1); d = lane + 32*t
+    // LSE in units of log2.  A row without a visible key has LSE = -inf: +inf in its place makes every probability 0.
+    auto lse2_of = [&](int64_t r) {
+        const float x = r < N ? lse[r] : INFINITY;
+        return x == -INFINITY ? INFINITY : x * kLog2e;
+    };
+    auto delta_of = [&](int64_t r) { return r < N ? delta[r] : 0.f; };
+    const float c2 = p.scale * kLog2e;
+    float r_lse[kKeySide ? 1 : 8], r_delta[kKeySide ? 1 : 8];
+    if (!kKeySide) {
 #pragma unroll
-    for (int t = 0; t < 8; ++t) acc0[t] = acc1[t] = 0.f;
-
-    for (int64_t t0 = t_lo; t0 < t_hi; t0 += kBwdTile) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < kBwdTile * D; i += blockDim.x) {
-            const int rr = i / D, d = i % D;
-            const bool in = t0 + rr < N;
-            tA[rr * P1 + d] = in ? othA[(t0 + rr) * D + d] : 0.f;
-            tB[rr * P1 + d] = in ? othB[(t0 + rr) * D + d] : 0.f;
+        for (int i = 0; i < 8; ++i) {
+            r_lse[i] = lse2_of(own0 + ln.g + 8 * i);
+            r_delta[i] = delta_of(own0 + ln.g + 8 * i);
         }
-        if (!kQuerySide && threadIdx.x < kBwdTile) {
-            const bool in = t0 + threadIdx.x < N;
-            tLse[threadIdx.x] = in ? p.lse[bh * N + t0 + threadIdx.x] : 0.f;
-            tDelta[threadIdx.x] = in ? p.delta[bh * N + t0 + threadIdx.x] : 0.f;
-        }
-        __syncthreads();
-        if (!row_valid) continue;
-
-        const int64_t o = t0 + lane;  // the opposite row this lane handles
-        const int64_t qi = kQuerySide ? r : o, kj = kQuerySide ? o : r;
-        const float* a_own = rA + warp * D;
-        const float* b_own = rB + warp * D;
-        const float* a_oth = tA + lane * P1;
-        const float* b_oth = tB + lane * P1;
-        // s = q_i . k_j ; dp = dO_i . v_j  (query side: own = (q, dO), other = (k, v); key side: own = (k, v))
-        float s = 0.f, dp = 0.f;
-        for (int d = 0; d < D; ++d) {
-            s = fmaf(a_own[d], a_oth[d], s);
-            dp = fmaf(b_own[d], b_oth[d], dp);
-        }
-        const float lse = kQuerySide ? own_lse : tLse[lane];
-        const float delta = kQuerySide ? own_delta : tDelta[lane];
-        const bool visible = o < N && !(p.causal && kj > qi) && lse != -INFINITY;
-        const float prob = visible ? expf(s * p.scale - lse) : 0.f;
-        const float ds = prob * (dp - delta) * p.scale;
-
-        if (kQuerySide) {
-            // dQ_i += sum_j dS_ij K_j
-            for (int jj = 0; jj < kBwdTile; ++jj) {
-                const float w = __shfl_sync(kFullMask, ds, jj);
-                const float* krow = tA + jj * P1;
+    }
+    float2 z1[4][2 * NC], z2[kKeySide ? 4 : 1][2 * NC];  // dQ, or dK and dV
 #pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    const int d = lane + 32 * t;
-                    if (d < D) acc0[t] = fmaf(w, krow[d], acc0[t]);
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 2 * NC; ++c) z1[r][c] = z2[kKeySide ? r : 0][c] = make_float2(0.f, 0.f);
+
+    cp_async_wait<0>();
+    __syncthreads();  // both groups have copied their share of the own rows
+    for (int64_t t0 = first; t0 < t_hi; t0 += step) {
+        const bool more = t0 + step < t_hi;
+        float c_lse[kKeySide ? J : 1], c_delta[kKeySide ? J : 1];
+        if (kKeySide) {
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                c_lse[j] = lse2_of(t0 + ln.h + 16 * j);
+                c_delta[j] = delta_of(t0 + ln.h + 16 * j);
+            }
+        }
+        cp_async_wait<0>();
+        group_sync(group);  // Y2 is visible, the last step's Y1 is free
+        load_tile<16 * J, kGroup>(Y1, oth1, t0, N, D, vec, share);
+        cp_async_commit();
+        float dp[8][J], pr[8][J];
+        product<J>(dp, X2, Y2, D, ln);
+        cp_async_wait<0>();
+        group_sync(group);  // Y1 is visible (and, on the query side, Y2 free)
+        if (!kKeySide && more) {
+            load_tile<16 * J, kGroup>(Y2, oth2, t0 + step, N, D, vec, share);
+            cp_async_commit();
+        }
+        product<J>(pr, X1, Y1, D, ln);
+
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < J; ++j)
+                pr[i][j] = exp2f(fmaf(pr[i][j], c2, -(kKeySide ? c_lse[j] : r_lse[i])));
+        if (t0 + 16 * J > N || (p.causal && (kKeySide ? t0 < own0 + kRows : t0 + 16 * J > own0))) {
+            const int hi = (int)(N - t0 < 16 * J ? N - t0 : 16 * J);
+            const int diag = (int)(own0 - t0);  // within a tile of zero wherever the causal mask cuts
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < J; ++j) {
+                    const int own = ln.g + 8 * i + diag, oth = ln.h + 16 * j;
+                    if (oth >= hi || (p.causal && (kKeySide ? own > oth : oth > own))) pr[i][j] = 0.f;
                 }
-            }
-        } else {
-            // dK_j += sum_i dS_ij Q_i ; dV_j += sum_i P_ij dO_i
-            for (int ii = 0; ii < kBwdTile; ++ii) {
-                const float w = __shfl_sync(kFullMask, ds, ii);
-                const float pw = __shfl_sync(kFullMask, prob, ii);
-                const float* qrow = tA + ii * P1;
-                const float* dorow = tB + ii * P1;
+        }
 #pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    const int d = lane + 32 * t;
-                    if (d < D) {
-                        acc0[t] = fmaf(w, qrow[d], acc0[t]);
-                        acc1[t] = fmaf(pw, dorow[d], acc1[t]);
-                    }
-                }
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < J; ++j) dp[i][j] = pr[i][j] * (dp[i][j] - (kKeySide ? c_delta[j] : r_delta[i]));
+        if constexpr (kKeySide) {
+            accumulate<J, NC>(z2, pr, Y2 + col0, D, Ws, ln);  // dV += P^T dO
+            group_sync(group);                                // Y2 is free
+            if (more) {
+                load_tile<16 * J, kGroup>(Y2, oth2, t0 + step, N, D, vec, share);
+                cp_async_commit();
             }
         }
+        accumulate<J, NC>(z1, dp, Y1 + col0, D, Ws, ln);  // dQ += dS K, or dK += dS^T Q
     }
 
-    if (!row_valid) return;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        const int d = lane + 32 * t;
-        if (d < D) {
-            if (kQuerySide) {
-                p.dq[base + r * D + d] = acc0[t];
-            } else {
-                p.dk[base + r * D + d] = acc0[t];
-                p.dv[base + r * D + d] = acc1[t];
-            }
+    if (G == 2) {
+        __syncthreads();  // both are done with their tiles; the exchange starts at the first group's Y1
+        float2* ex = reinterpret_cast<float2*>(X2 + x_tile);
+        if (group == 1) {
+            put(ex, z1, tid);
+            if constexpr (kKeySide) put(ex + 8 * NC * kGroup, z2, tid);
         }
+        __syncthreads();
+        if (group == 1) return;
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 2 * NC; ++c) {
+                z1[r][c] = __fadd2_rn(z1[r][c], ex[(r * 2 * NC + c) * kGroup + tid]);
+                if constexpr (kKeySide) z2[r][c] = __fadd2_rn(z2[r][c], ex[(8 * NC + r * 2 * NC + c) * kGroup + tid]);
+            }
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int64_t r = own0 + ln.g + 8 * i;
+        if (r >= N) continue;
+        store_row<NC>((kKeySide ? p.dk : p.dq) + base + r * D, z1, i, p.scale, col0, D, pairs, ln);
+        if constexpr (kKeySide) store_row<NC>(p.dv + base + r * D, z2, i, 1.f, col0, D, pairs, ln);
+    }
+}
+
+// CTA order: rank (0 = most other-side tiles under a causal mask), then side, column group, head.
+// Against the kernel that gave every own row to one warp (a shared-memory load per multiply-add): B=2 H=8 N=1000 D=64
+// causal 1814 -> 205 us, B=4 H=16 N=1024 D=64 12.1 -> 1.47 ms (41 TFLOP/s executed), B=4 H=16 N=161 D=80 312 -> 63 us.
+// Scalar multiply-adds in place of the packed ones were 4 % slower, one group per CTA (two CTAs an SM) 15 % at N=1000.
+template <int NC, int J, int G>
+__global__ void __launch_bounds__(simt::kGroup * G, 1)
+bwd_tiled_kernel(const BwdParams p, const bool vec, const bool pairs, const int n_tiles, const int n_bh, const int groups) {
+    extern __shared__ __align__(16) float smem[];
+    const int x = (int)blockIdx.x;
+    const int bh = x % n_bh, rest = x / n_bh, col0 = rest % groups * (NC * 32), side = rest / groups & 1,
+              rank = rest / groups / 2;
+    if (side == 0)
+        bwd_rows<NC, J, G, true>(p, smem, bh, (int64_t)rank * simt::kRows, col0, vec, pairs);
+    else
+        bwd_rows<NC, J, G, false>(p, smem, bh, (int64_t)(p.causal ? n_tiles - 1 - rank : rank) * simt::kRows, col0, vec,
+                                  pairs);
+}
+
+template <int NC, int J, int G>
+static cudaError_t launch_bwd_tiled(const BwdParams& p, int64_t bh, cudaStream_t stream) {
+    auto bytes = [](int dim) {
+        return sizeof(float) * (2 * (size_t)simt::tile_floats(simt::kRows, dim) +
+                                G * (2 * (size_t)simt::tile_floats(16 * J, dim) + simt::kWFloats));
+    };
+    cudaError_t e = set_max_dynamic_smem_once<bwd_tiled_kernel<NC, J, G>>((int)bytes(G == 1 ? 256 : NC * 32));
+    if (e != cudaSuccess) return e;
+    const int64_t n_tiles = (p.seq + simt::kRows - 1) / simt::kRows;
+    const int groups = (p.dim + NC * 32 - 1) / (NC * 32);
+    const int64_t n = 2 * n_tiles * bh * groups;
+    if (n > 0x7fffffff) return cudaErrorInvalidValue;
+    const uintptr_t in = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) |
+                         reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.d_out);
+    const uintptr_t outs = reinterpret_cast<uintptr_t>(p.dq) | reinterpret_cast<uintptr_t>(p.dk) | reinterpret_cast<uintptr_t>(p.dv);
+    const bool vec = p.dim % 4 == 0 && (in & 15) == 0, pairs = p.dim % 2 == 0 && (outs & 7) == 0;
+    bwd_tiled_kernel<NC, J, G><<<(unsigned)n, simt::kGroup * G, bytes(p.dim), stream>>>(p, vec, pairs, (int)n_tiles,
+                                                                                         (int)bh, groups);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_backward_f32(const float* q, const float* k, const float* v, const float* out, const float* d_out,
@@ -182,15 +226,13 @@ cudaError_t launch_backward_f32(const float* q, const float* k, const float* v, 
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     BwdParams p{q, k, v, out, d_out, lse, dq, dk, dv, delta_ws, seq, dim, causal, scale};
-    const size_t smem = sizeof(float) * ((size_t)2 * kBwdTile * (dim + 1) + (size_t)2 * kBwdRows * dim + 2 * kBwdTile);
-    e = cudaFuncSetAttribute(bwd_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(bwd_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    dim3 grid((unsigned)((seq + kBwdRows - 1) / kBwdRows), (unsigned)bh);
-    bwd_pass_kernel<true><<<grid, kBwdRows * 32, smem, stream>>>(p);
-    bwd_pass_kernel<false><<<grid, kBwdRows * 32, smem, stream>>>(p);
-    return cudaGetLastError();
+    // Tiles of 64 x 64 while the scores of both products fit the registers next to the gradients, 64 x 32 beyond; a
+    // head dim above 128 is accumulated in two column groups of 128, and its tiles leave no room for a second group.
+    if (dim <= 32) return launch_bwd_tiled<1, 4, 2>(p, bh, stream);
+    if (dim <= 64) return launch_bwd_tiled<2, 4, 2>(p, bh, stream);
+    if (dim <= 96) return launch_bwd_tiled<3, 2, 2>(p, bh, stream);
+    if (dim <= 128) return launch_bwd_tiled<4, 2, 2>(p, bh, stream);
+    return launch_bwd_tiled<4, 2, 1>(p, bh, stream);
 }
 
 }  // namespace rt

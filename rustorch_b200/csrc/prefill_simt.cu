@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "simt_tile.cuh"
 
 namespace rt {
 
@@ -131,187 +132,174 @@ __global__ void __launch_bounds__(kSimtRows * 32) prefill_f32_kernel(const SimtP
 }
 
 // ---------------------------------------------------------------------------------------------
-// Register-tiled variant: one CTA of 256 threads (16 x 16) owns 64 query rows and walks the keys in
-// tiles of 64.  Q and K sit transposed in shared memory ([d][row], [d][key]) so that the score
-// product reads one 16-byte vector of each per 16 multiply-adds (thread (ty, tx) holds the 4 x 4
-// block rows 4 ty.., keys 4 tx..); the probabilities go through shared memory ([row][key]) and the
-// P V product reads 4 keys x (4 rows of P + NG vectors of V) per 64 NG multiply-adds.  Same recurrence,
-// masks and NaN rules as the kernel above; NG = ceil(D / 64) groups of 64 output columns.
-constexpr int kTileRows = 64, kTileKeys = 64, kTilePad = 68;  // 68: rows stay 16-byte aligned, 4-bank skew
-
-template <int NG>
-__global__ void __launch_bounds__(256) prefill_f32_tiled_kernel(const SimtParams p) {
+// Register-tiled variant: a CTA owns 64 query rows and walks the keys in tiles of 64; see simt_tile.cuh for the
+// split of the two products.  Same recurrence, masks and NaN rules as the kernel above.  With G = 2 groups each has
+// its own K and V buffers and its own running maximum, sum and output, merged at the end: at these sizes (a few
+// hundred row blocks) the launch lasts as long as its longest block, and two groups walk that in half the steps.
+// Head dims above 128 leave no room for the second group's tiles.  K and V have one buffer each per group: K of the
+// next tile is copied while P V runs, V while Q K^T runs, so two group barriers per tile order everything.  The row
+// sum stays per thread until the end.  NC = ceil(D / 32) column groups of the output.
+// Against the 256-thread kernel with 4 x 4 scores a thread that this replaces (scalar loads transposed into shared
+// memory with 16-way conflicts): B=1 H=8 N=2048 D=64 causal 371 -> 120 us (36 TFLOP/s), B=2 H=16 N=1000 D=128 causal
+// 520 -> 232 us, B=4 H=16 N=1024 D=64 656 -> 435 us (40 TFLOP/s of the FP32 pipe's 74).
+template <int NC, int G>
+__global__ void __launch_bounds__(simt::kGroup * G, 1)
+prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, const int64_t row_blocks) {
+    using namespace simt;
     extern __shared__ __align__(16) float smem[];
-    const int D = p.dim;
-    constexpr int DP = NG * 64;
-    float* Qt = smem;                         // [D][68]   Q transposed, scaled
-    float* Kt = Qt + (size_t)D * kTilePad;    // [D][68]   K transposed
-    float* Vs = Kt + (size_t)D * kTilePad;    // [64][DP]  V, columns >= D zero
-    float* Ps = Vs + (size_t)kTileKeys * DP;  // [64][68]  probabilities [row][key]
+    const int group = G == 1 ? 0 : (int)threadIdx.x >> 7, tid = (int)threadIdx.x & (kGroup - 1);
+    const int D = p.dim, tile = tile_floats(kRows, D);
+    float* Qs = smem;
+    float* Ks = Qs + tile + group * (2 * tile + kWFloats);
+    float* Vs = Ks + tile;
+    float* Ws = Vs + tile;
+    const Lane ln;
+    const Share share = Share::of<kGroup>(tid, D, vec), q_share = Share::of<kGroup * G>((int)threadIdx.x, D, vec);
 
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int64_t b = blockIdx.z, hq = blockIdx.y;
-    const int64_t hkv = hq / (p.heads_q / p.heads_kv);
-    const int64_t row0 = (int64_t)(gridDim.x - 1 - blockIdx.x) * kTileRows;  // heaviest causal blocks first
-
-    const float* qptr = p.q + ((b * p.heads_q + hq) * p.seq_q) * D;
+    // CTA order: under a causal mask the longest row blocks of all heads first
+    const int64_t n_bh = (int64_t)gridDim.x / row_blocks, x = blockIdx.x;
+    const int64_t bh = p.causal ? x % n_bh : x / row_blocks;
+    const int64_t row0 = (p.causal ? row_blocks - 1 - x / n_bh : x % row_blocks) * kRows;
+    const int64_t b = bh / p.heads_q, hq = bh % p.heads_q, hkv = hq / (p.heads_q / p.heads_kv);
     const float* kptr = p.k + ((b * p.heads_kv + hkv) * p.seq_kv) * D;
     const float* vptr = p.v + ((b * p.heads_kv + hkv) * p.seq_kv) * D;
     const uint8_t* keep = p.key_keep ? p.key_keep + b * p.keep_batch_stride : nullptr;
-
-    for (int i = tid; i < kTileRows * D; i += 256) {
-        const int r = i / D, d = i % D;
-        Qt[d * kTilePad + r] = (row0 + r < p.seq_q) ? qptr[(row0 + r) * D + d] * p.scale : 0.f;
-    }
 
     int64_t k_hi = p.seq_kv;
     if (p.kv_lens && p.kv_lens[b] < k_hi) k_hi = p.kv_lens[b] < 0 ? 0 : p.kv_lens[b];
     const int64_t q_off = p.q_offsets ? p.q_offsets[b] : 0;  // query row i sits at key position i + q_off
     int64_t k_loop = k_hi;
     if (p.causal) {
-        int64_t last = row0 + kTileRows;  // keys <= position of the last query row of the CTA
+        int64_t last = row0 + kRows;  // keys <= position of the last query row of the CTA
         if (last > p.seq_q) last = p.seq_q;
         last += q_off;
         if (last < 0) last = 0;
         if (last < k_loop) k_loop = last;
     }
 
-    float m[4], l[4], o[4][NG][4];
+    const float c2 = p.scale * kLog2e;
+    float m[8], l[8];  // maximum (log2 units) and this thread's share of the sum
+    float2 z[4][2 * NC];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 8; ++i) {
         m[i] = -INFINITY;
         l[i] = 0.f;
-#pragma unroll
-        for (int g = 0; g < NG; ++g)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) o[i][g][c] = 0.f;
     }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 2 * NC; ++c) z[r][c] = make_float2(0.f, 0.f);
 
-    for (int64_t kj = 0; kj < k_loop; kj += kTileKeys) {
-        __syncthreads();  // the previous tile's K, V and P are no longer read
-        for (int i = tid; i < kTileKeys * D; i += 256) {
-            const int r = i / D, d = i % D;
-            const bool in = kj + r < k_hi;
-            Kt[d * kTilePad + r] = in ? kptr[(kj + r) * D + d] : 0.f;
-            Vs[r * DP + d] = in ? vptr[(kj + r) * D + d] : 0.f;
+    const int64_t first = (int64_t)group * kRows, step = (int64_t)G * kRows;
+    load_tile<kRows, kGroup * G>(Qs, p.q + (bh * p.seq_q) * D, row0, p.seq_q, D, vec, q_share);
+    if (first < k_loop) load_tile<kRows, kGroup>(Ks, kptr, first, k_hi, D, vec, share);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();  // both groups have copied their share of Q
+    for (int64_t kj = first; kj < k_loop; kj += step) {
+        cp_async_wait<0>();
+        group_sync(group);  // this tile's K is visible and nobody reads the last tile's V any more
+        load_tile<kRows, kGroup>(Vs, vptr, kj, k_hi, D, vec, share);
+        cp_async_commit();
+        float s[8][4];
+        product<4>(s, Qs, Ks, D, ln);
+        cp_async_wait<0>();
+        group_sync(group);  // V is visible, K is free
+        if (kj + step < k_loop) {
+            load_tile<kRows, kGroup>(Ks, kptr, kj + step, k_hi, D, vec, share);
+            cp_async_commit();
         }
-        if (D < DP) {
-            const int extra = DP - D;
-            for (int i = tid; i < kTileKeys * extra; i += 256) Vs[(i / extra) * DP + D + i % extra] = 0.f;
-        }
-        __syncthreads();
-
-        // ---- S = (scale Q) K^T, 4 x 4 per thread
-        float s[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-#pragma unroll 4
-        for (int d = 0; d < D; ++d) {
-            const float4 q4 = *reinterpret_cast<const float4*>(Qt + d * kTilePad + ty * 4);
-            const float4 k4 = *reinterpret_cast<const float4*>(Kt + d * kTilePad + tx * 4);
-            const float qa[4] = {q4.x, q4.y, q4.z, q4.w}, ka[4] = {k4.x, k4.y, k4.z, k4.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) s[i][j] = fmaf(qa[i], ka[j], s[i][j]);
-        }
-
-        // ---- masks, online softmax (the 16 threads of a row group agree through shuffles)
-        bool masked[4][4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int64_t key = kj + tx * 4 + j;
-            const bool off = key >= k_hi || (keep && key < p.seq_kv && !keep[key]);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                masked[i][j] = off || (p.causal && key > row0 + ty * 4 + i + q_off);
-                if (masked[i][j]) s[i][j] = -INFINITY;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float m_tile = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
-#pragma unroll
-            for (int off = 8; off; off >>= 1) m_tile = fmaxf(m_tile, __shfl_xor_sync(kFullMask, m_tile, off));
-            const float m_new = fmaxf(m[i], m_tile);
-            const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-            const float alpha = (m[i] == -INFINITY) ? 0.f : expf(m[i] - m_use);
-            float psum = 0.f;
+        // ---- masks, in tiles that the length, the diagonal or flags cut
+        if (keep || kj + kRows > k_hi || (p.causal && kj + kRows - 1 > row0 + q_off)) {
+            const int hi = (int)(k_hi - kj < kRows ? k_hi - kj : kRows);
+            const int64_t d64 = row0 + q_off - kj;
+            const int diag = (int)(d64 < -kRows ? -kRows : d64 > kRows ? kRows : d64);  // tile row r sees keys <= r + diag
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                s[i][j] = masked[i][j] ? 0.f : expf(s[i][j] - m_use);
-                psum += s[i][j];
+                const int key = ln.h + 16 * j;
+                const bool off = key >= hi || (keep && !keep[kj + key]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (off || (p.causal && key > ln.g + 8 * i + diag)) s[i][j] = -INFINITY;
             }
+        }
+        // ---- online softmax in units of log2; the 16 lanes of a row agree on the maximum through shuffles
+        float2 alpha[4];
 #pragma unroll
-            for (int off = 8; off; off >>= 1) psum += __shfl_xor_sync(kFullMask, psum, off);
-            l[i] = l[i] * alpha + psum;
+        for (int i = 0; i < 8; ++i) {
+            const float mt = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
+            const float m_new = fmaxf(m[i], row_max(mt) * c2);
+            const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+            const float a = exp2f(m[i] - m_use);  // 0 while m is -inf
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = exp2f(fmaf(s[i][j], c2, -m_use));  // masked: 0
+            l[i] = l[i] * a + ((s[i][0] + s[i][1]) + (s[i][2] + s[i][3]));
             m[i] = m_new;
+            if (i & 1) alpha[i >> 1].y = a;
+            else alpha[i >> 1].x = a;
+        }
 #pragma unroll
-            for (int g = 0; g < NG; ++g)
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) o[i][g][c] *= alpha;
-            *reinterpret_cast<float4*>(Ps + (ty * 4 + i) * kTilePad + tx * 4) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+            for (int c = 0; c < 2 * NC; ++c) z[r][c] = __fmul2_rn(z[r][c], alpha[r]);
+        accumulate<4, NC>(z, s, Vs, D, Ws, ln);
+    }
+
+    // ---- the two groups' partial rows: the second hands over (max, per-thread sum, output), the first merges
+    if (G == 2) {
+        __syncthreads();  // both are done with their tiles; the exchange starts at the first group's K
+        float2* ex = reinterpret_cast<float2*>(Qs + tile);
+        if (group == 1) {
+            put(ex, z, tid);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ex[(8 * NC + i) * kGroup + tid] = make_float2(m[i], l[i]);
         }
         __syncthreads();
-
-        // ---- O += P V: rows 4 ty.., columns 64 g + 4 tx..
-#pragma unroll 2
-        for (int kk = 0; kk < kTileKeys; kk += 4) {
-            float pa[4][4];
+        if (group == 1) return;
+        float2 f0[4], f1[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 t = *reinterpret_cast<const float4*>(Ps + (ty * 4 + i) * kTilePad + kk);
-                pa[i][0] = t.x; pa[i][1] = t.y; pa[i][2] = t.z; pa[i][3] = t.w;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int g = 0; g < NG; ++g) {
-                    const float4 v4 = *reinterpret_cast<const float4*>(Vs + (kk + u) * DP + g * 64 + tx * 4);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        o[i][g][0] = fmaf(pa[i][u], v4.x, o[i][g][0]);
-                        o[i][g][1] = fmaf(pa[i][u], v4.y, o[i][g][1]);
-                        o[i][g][2] = fmaf(pa[i][u], v4.z, o[i][g][2]);
-                        o[i][g][3] = fmaf(pa[i][u], v4.w, o[i][g][3]);
-                    }
-                }
+        for (int i = 0; i < 8; ++i) {
+            const float2 o = ex[(8 * NC + i) * kGroup + tid];
+            const float mm = fmaxf(m[i], o.x), m_use = (mm == -INFINITY) ? 0.f : mm;
+            const float a = exp2f(m[i] - m_use), c = exp2f(o.x - m_use);
+            l[i] = l[i] * a + o.y * c;  // (a NaN sum stays one: NaN * 0)
+            m[i] = mm;
+            if (i & 1) { f0[i >> 1].y = a; f1[i >> 1].y = c; }
+            else { f0[i >> 1].x = a; f1[i >> 1].x = c; }
         }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 2 * NC; ++c)
+                z[r][c] = __ffma2_rn(f0[r], z[r][c], __fmul2_rn(f1[r], ex[(r * 2 * NC + c) * kGroup + tid]));
     }
 
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int64_t qi = row0 + ty * 4 + i;
+    for (int i = 0; i < 8; ++i) {
+        const float sum = row_sum(l[i]);
+        const int64_t qi = row0 + ln.g + 8 * i;
         if (qi >= p.seq_q) continue;
-        float* dst = p.out + ((b * p.heads_q + hq) * p.seq_q + qi) * D;
-        const bool ok = (l[i] > 0.f) && isfinite(l[i]);  // cpu_forward.rs:411
-        const float inv = ok ? 1.f / l[i] : 0.f;
-#pragma unroll
-        for (int g = 0; g < NG; ++g)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int d = g * 64 + tx * 4 + c;
-                if (d < D) dst[d] = ok ? o[i][g][c] * inv : NAN;
-            }
-        if (p.lse && tx == 0)
-            p.lse[(b * p.heads_q + hq) * p.seq_q + qi] =
-                (l[i] > 0.f) ? m[i] + logf(l[i]) : (l[i] == 0.f ? -INFINITY : NAN);
+        const bool ok = (sum > 0.f) && isfinite(sum);  // cpu_forward.rs:411
+        store_row<NC>(p.out + (bh * p.seq_q + qi) * D, z, i, ok ? 1.f / sum : NAN, 0, D, pairs, ln);
+        if (p.lse && ln.h == 0)
+            p.lse[bh * p.seq_q + qi] = (sum > 0.f) ? fmaf(m[i], kLn2, logf(sum)) : (sum == 0.f ? -INFINITY : NAN);
     }
 }
 
-template <int NG>
+template <int NC, int G>
 static cudaError_t launch_tiled(const SimtParams& p, int64_t batch, cudaStream_t stream) {
-    const size_t smem = sizeof(float) * (2 * (size_t)p.dim * kTilePad + (size_t)kTileKeys * NG * 64 +
-                                         (size_t)kTileRows * kTilePad);
-    cudaError_t e = cudaFuncSetAttribute(prefill_f32_tiled_kernel<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    auto bytes = [](int dim) {
+        return sizeof(float) * ((1 + 2 * G) * (size_t)simt::tile_floats(simt::kRows, dim) + G * (size_t)simt::kWFloats);
+    };
+    // the limit of the widest head dim of this instantiation, so that it is set once
+    cudaError_t e = set_max_dynamic_smem_once<prefill_f32_tiled_kernel<NC, G>>((int)bytes(NC * 32));
     if (e != cudaSuccess) return e;
-    const int64_t row_blocks = (p.seq_q + kTileRows - 1) / kTileRows;
-    if (row_blocks > 0x7fffffff || p.heads_q > 65535 || batch > 65535) return cudaErrorInvalidValue;
-    dim3 grid((unsigned)row_blocks, (unsigned)p.heads_q, (unsigned)batch);
-    prefill_f32_tiled_kernel<NG><<<grid, 256, smem, stream>>>(p);
+    const int64_t row_blocks = (p.seq_q + simt::kRows - 1) / simt::kRows, n = row_blocks * p.heads_q * batch;
+    if (n > 0x7fffffff) return cudaErrorInvalidValue;
+    const uintptr_t in = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v);
+    const bool vec = p.dim % 4 == 0 && (in & 15) == 0;
+    const bool pairs = p.dim % 2 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 7) == 0;
+    prefill_f32_tiled_kernel<NC, G><<<(unsigned)n, simt::kGroup * G, bytes(p.dim), stream>>>(p, vec, pairs, row_blocks);
     return cudaGetLastError();
 }
 
@@ -325,16 +313,17 @@ cudaError_t launch_prefill_f32(const float* q, const float* k, const float* v, f
                  keep_batch_stride, scale};
     // The register-tiled kernel is the path for 16 query rows and more; a decode-shaped call (a few rows against
     // a long cache) would waste most of its 64-row tile and keeps the warp-per-row kernel, which
-    // RT_ATTN_PREFILL_F32_IMPL=rows selects for every shape (comparisons).  The tiled kernel applies the scale
-    // to Q once, the other one to every score.
+    // RT_ATTN_PREFILL_F32_IMPL=rows selects for every shape (comparisons).
     static const bool rows_impl = [] {
         const char* e = getenv("RT_ATTN_PREFILL_F32_IMPL");
         return e && e[0] == 'r';
     }();
     if (!rows_impl && dim <= 256 && seq_q >= 16) {
-        if (dim <= 64) return launch_tiled<1>(p, batch, stream);
-        if (dim <= 128) return launch_tiled<2>(p, batch, stream);
-        return launch_tiled<4>(p, batch, stream);
+        if (dim <= 32) return launch_tiled<1, 2>(p, batch, stream);
+        if (dim <= 64) return launch_tiled<2, 2>(p, batch, stream);
+        if (dim <= 96) return launch_tiled<3, 2>(p, batch, stream);
+        if (dim <= 128) return launch_tiled<4, 2>(p, batch, stream);
+        return launch_tiled<8, 1>(p, batch, stream);
     }
     const size_t smem = sizeof(float) * ((size_t)kSimtKeys * (dim + 1) + (size_t)kSimtKeys * dim +
                                          (size_t)kSimtRows * dim);

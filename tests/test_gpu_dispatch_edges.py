@@ -23,3 +23,23 @@ def test_keep_flags_with_hidden_tails(oracle, D, N, causal):
     _, ref, ref_lse = oracle.flash_forward_ext(q, k, v, causal=causal, keep=keep)
     util.check_output(out, ref, label=f"keep tails N{N} D{D} causal={causal}")
     util.check_lse(lse, ref_lse)
+
+
+@pytest.mark.parametrize("N", [1, 17, 64, 65, 130, 200])
+@pytest.mark.parametrize("D", [1, 7, 32, 33, 64, 80, 96, 100, 128, 129, 200, 256])
+def test_f32_forward_and_backward_tiles(oracle, N, D):
+    """The register-tiled f32 kernels where their tiles, column groups, 16-byte copies and two-group split end."""
+    import torch
+    import rustorch_b200 as rt
+    for causal in (False, True):
+        q, k, v, do = (oracle.fill_normal((1, 2, N, D), s) for s in (1, 2, 3, 4))
+        t = [util.to_cuda(x) for x in (q, k, v, do)]
+        out, lse = rt.prefill_f32(*t[:3], causal=causal)
+        got = rt.backward_f32(*t[:3], out, t[3], lse, causal=causal)
+        torch.cuda.synchronize()
+        _, ref, ref_lse = oracle.flash_forward_ext(q, k, v, causal=causal)
+        assert np.abs(util.to_np(out) - ref).max() < 1e-4
+        assert np.abs(util.to_np(lse) - ref_lse).max() < 1e-4
+        _, *grads = oracle.flash_backward(q, k, v, do, causal=causal)
+        for name, a, b in zip(("dq", "dk", "dv"), got, grads):
+            assert np.abs(util.to_np(a) - b).max() < 2e-4 * max(1.0, np.abs(b).max()), (name, causal)
