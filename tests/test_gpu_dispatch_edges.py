@@ -43,3 +43,28 @@ def test_f32_forward_and_backward_tiles(oracle, N, D):
         _, *grads = oracle.flash_backward(q, k, v, do, causal=causal)
         for name, a, b in zip(("dq", "dk", "dv"), got, grads):
             assert np.abs(util.to_np(a) - b).max() < 2e-4 * max(1.0, np.abs(b).max()), (name, causal)
+
+
+@pytest.mark.parametrize("precision", ["f32", "bf16"])
+@pytest.mark.parametrize("B,H,N", [(1, 1, 1), (1, 2, 300), (3, 5, 1000), (1, 40, 2100)])
+def test_host_entry_staged_equals_pinned(precision, B, H, N):
+    """Pageable slices (staging threads, conversion on the host) and pinned ones (copied as they are, conversion on
+    the device) give the same bits: one piece, several chunks, and more pieces than the ring has slots.  The inputs
+    hold values whose bf16 rounding is special."""
+    import torch
+    import rustorch_b200 as rt
+    D, n = 64, B * H * N * 64
+    r = np.random.default_rng(7)
+    q, k, v = (r.standard_normal(n, dtype=np.float32) for _ in range(3))
+    v[:10] = [1.00390625, 1.01171875, -0.0, 1e-40, 3e38, -1.0, 65504.0, 1e-30, 0.99609375, 2.0]
+    shape, mask = rt.AttentionShape.new(B, H, N, D), rt.Mask.causal()
+    out = np.empty_like(q)
+    rt.flash_forward_masked(shape, q, k, v, mask, out, precision)
+    pinned = [torch.empty(n, dtype=torch.float32, pin_memory=True).numpy() for _ in range(4)]
+    for p, x in zip(pinned, (q, k, v)):
+        p[:] = x
+    rt.flash_forward_masked(shape, *pinned[:3], mask, pinned[3], precision)
+    assert np.array_equal(out.view(np.uint32), pinned[3].view(np.uint32))
+    mixed = np.empty_like(q)
+    rt.flash_forward_masked(shape, q, pinned[1], v, mask, mixed, precision)
+    assert np.array_equal(out.view(np.uint32), mixed.view(np.uint32))
