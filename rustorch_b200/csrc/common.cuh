@@ -53,4 +53,69 @@ __device__ __forceinline__ float fast_log2(float x) {
     return y;
 }
 
+// How a decode launch cuts its sequences into chunks, one CTA each; see pick_split for the rule.
+enum { kSplitFixed = 0, kSplitEven, kSplitShare };
+struct DecodeSplit {
+    int n_chunks;  // chunks of a sequence at most
+    int chunk;     // kSplitFixed: tokens per chunk (grid: chunk, KV head, sequence)
+    int mode;      // kSplitEven: n_chunks equal parts of every sequence's own length (same grid)
+                   // kSplitShare: chunks of one size for all `batch` <= 32 sequences, about `target` of them in all,
+    int batch;     //              dealt to a flat grid of `ctas` CTAs
+    int ctas;
+    float target;
+};
+
+// The chunk of the calling CTA: tokens [lo, hi) of the sequence's visible range.
+struct DecodeChunk {
+    int b, kvh, idx, lo, hi;
+    int rest;  // kSplitShare: chunks after the sequence's last, which the CTA with the last marks empty for the merge
+    bool none;  // kSplitShare: a CTA beyond the last chunk
+};
+
+__device__ __forceinline__ int round_up_64(int x) { return max(64, (x + 63) & ~63); }
+
+// Called by all threads of a warp; every warp comes to the same answer on its own.  visible_of(b): tokens of sequence b.
+template <class VisibleOf>
+__device__ __forceinline__ DecodeChunk find_chunk(const DecodeSplit& sp, int n_kv, VisibleOf&& visible_of) {
+    DecodeChunk c;
+    c.none = false;
+    c.rest = 0;
+    if (sp.mode != kSplitShare) {
+        c.idx = blockIdx.x, c.kvh = blockIdx.y, c.b = blockIdx.z;
+        const int visible = visible_of(c.b);
+        const int size = sp.mode == kSplitFixed ? sp.chunk : round_up_64((visible + sp.n_chunks - 1) / sp.n_chunks);
+        c.lo = c.idx * size;
+        c.hi = min(c.lo + size, visible);
+        return c;
+    }
+    // Lane b holds sequence b: the sum of the lengths gives the chunk size, a scan of the chunk counts the place of
+    // every sequence in the list of chunks (sequence, KV head, chunk).
+    const int lane = threadIdx.x & 31;
+    const int visible = lane < sp.batch ? visible_of(lane) : 0;
+    float total = (float)visible;
+#pragma unroll
+    for (int off = 16; off; off >>= 1) total += __shfl_xor_sync(kFullMask, total, off);
+    const int share = (int)ceilf(total * (float)n_kv / sp.target);
+    const int size = round_up_64(max(share, (visible + sp.n_chunks - 1) / sp.n_chunks));
+    const int n = max(1, (visible + size - 1) / size), mine = lane < sp.batch ? n * n_kv : 0;
+    int end = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(kFullMask, end, off);
+        if (lane >= off) end += y;
+    }
+    const int want = blockIdx.x;
+    const unsigned owner = __ballot_sync(kFullMask, want >= end - mine && want < end);
+    c.none = owner == 0;
+    c.b = owner ? __ffs(owner) - 1 : 0;
+    const int at = want - __shfl_sync(kFullMask, end - mine, c.b), size_b = __shfl_sync(kFullMask, size, c.b),
+              n_b = __shfl_sync(kFullMask, n, c.b), visible_b = __shfl_sync(kFullMask, visible, c.b);
+    c.kvh = at / n_b;
+    c.idx = at - c.kvh * n_b;
+    c.lo = c.idx * size_b;
+    c.hi = min(c.lo + size_b, visible_b);
+    if (c.idx == n_b - 1) c.rest = sp.n_chunks - n_b;
+    return c;
+}
+
 }  // namespace rt

@@ -50,7 +50,7 @@ struct DecodeParams {
     int64_t kv_begin, kv_end;
     int64_t max_seq;
     int n_heads, n_kv;
-    int chunk, n_chunks;
+    DecodeSplit split;
     int64_t rows;  // B * Hq
     int64_t of_stride, lse_stride;  // floats between consecutive rows of out_f32 / lse (D and 1 unless packed)
     float scale_log2;
@@ -66,21 +66,23 @@ __global__ void __launch_bounds__(128) gqa_decode_splitkv_kernel(const DecodePar
     __shared__ float sm_l[NG][G];
     __shared__ __align__(16) float sm_o[NG][G][D];
 
-    const int chunk_idx = blockIdx.x;
-    const int kvh = blockIdx.y;
-    const int b = blockIdx.z;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gi = lane / LPT;   // lane-group within the warp
     const int lig = lane % LPT;  // lane within the group: owns dims [lig*8, lig*8+8)
-    const int64_t row0 = (int64_t)b * p.n_heads + (int64_t)kvh * G;  // first output row of the group
-    const bool direct = (p.n_chunks == 1);
+    const bool direct = (p.split.n_chunks == 1);
 
-    int64_t len = p.kv_lens ? (int64_t)p.kv_lens[b] : p.kv_len_uniform;
-    if (len > p.max_seq) len = p.max_seq;
-    int64_t hi = (p.kv_end >= 0 && p.kv_end < len) ? p.kv_end : len;
-    const int64_t c0 = p.kv_begin + (int64_t)chunk_idx * p.chunk;
-    int64_t c1 = c0 + p.chunk;
-    if (c1 > hi) c1 = hi;
+    const DecodeChunk ck = find_chunk(p.split, p.n_kv, [&](int seq) {  // tokens of a sequence inside the launch's range
+        int64_t len = p.kv_lens ? (int64_t)p.kv_lens[seq] : p.kv_len_uniform;
+        if (len > p.max_seq) len = p.max_seq;
+        if (p.kv_end >= 0 && p.kv_end < len) len = p.kv_end;
+        return len > p.kv_begin ? (int)(len - p.kv_begin) : 0;
+    });
+    if (ck.none) return;
+    const int chunk_idx = ck.idx, kvh = ck.kvh, b = ck.b;
+    const int64_t row0 = (int64_t)b * p.n_heads + (int64_t)kvh * G;  // first output row of the group
+    const int64_t c0 = p.kv_begin + ck.lo, c1 = p.kv_begin + ck.hi;
+    for (int i = tid; i < ck.rest * G; i += 128)
+        p.part_lse[(int64_t)(chunk_idx + 1 + i / G) * p.rows + row0 + i % G] = -INFINITY;
 
     if (c0 >= c1) {  // nothing visible in this chunk: identity partial
         if (direct) {
@@ -797,7 +799,7 @@ int decode_num_chunks(int64_t batch, int n_kv, int64_t max_seq) {
 
 template <int D, int G>
 static cudaError_t launch_decode_dg(const DecodeParams& p, int64_t batch, cudaStream_t stream) {
-    dim3 grid(p.n_chunks, p.n_kv, (unsigned)batch);
+    const dim3 grid = p.split.mode == kSplitShare ? dim3(p.split.ctas) : dim3(p.split.n_chunks, p.n_kv, (unsigned)batch);
     gqa_decode_splitkv_kernel<D, G><<<grid, 128, 0, stream>>>(p);
     return cudaGetLastError();
 }
@@ -811,6 +813,55 @@ static cudaError_t launch_decode_d(const DecodeParams& p, int group, int64_t bat
         case 8: return launch_decode_dg<D, 8>(p, batch, stream);
     }
     return cudaErrorInvalidValue;
+}
+
+// The split of one launch.  Its chunk count stays within what rt_gqa_decode_workspace_bytes sized the scratch for.
+//  * As many (sequence, KV head) groups as resident CTAs (1, 2 or 4 per SM by head dim) or more: whole sequences up to
+//    4096 tokens, which need no partials and no merge; the next CTA starts as one ends, so a last wave that is nearly
+//    empty costs less than cutting every sequence (600 groups of up to 512 tokens, D = 128: 51 -> 19 us; 900 of up to
+//    1500, D = 256: 299 -> 142 us).  Longer ones keep chunks of at most 1024 tokens: an 8192-token CTA would end 20 us
+//    after the others.
+//  * 64 groups and more of at most 256 KB of K and V: also whole.  That is 5 us for one CTA, less than a merge costs.
+//  * Fewer groups: one wave, about slots / groups chunks per sequence.  Per-sequence lengths are only known on the
+//    device.  From 40 MB on (6 us at the HBM rate) and up to 32 sequences, chunks of one size for all of them, so that
+//    every CTA streams equally long (D = 64, 112 groups of 1000 to 4096 tokens: 27 -> 13 us; 8 sequences of 500 to 4000
+//    over 8 KV heads, D = 128: 17.6 -> 14.0 us); the scan of the lengths costs 0.4 us, so smaller launches cut every
+//    sequence into equal parts of its own, or, up to 2048 tokens and for larger batches, at fixed places.
+static DecodeSplit pick_split(int64_t batch, int n_kv, int head_dim, int64_t max_seq, int64_t span, bool ragged) {
+    DecodeSplit sp{};
+    sp.chunk = decode_chunk_tokens(batch, n_kv, max_seq);
+    const int64_t groups = batch * (int64_t)n_kv, slots = (int64_t)sm_count() * (head_dim == 64 ? 4 : head_dim == 128 ? 2 : 1);
+    const int64_t whole = (span + 63) / 64 * 64, group_bytes = span * head_dim * 4;
+    if (groups >= slots || (groups >= 2 * (int64_t)sm_count() && span > 4096)) {
+        if (span <= 4096) sp.chunk = (int)whole;
+    } else if (groups >= 64 && group_bytes <= (256 << 10)) {
+        sp.chunk = (int)whole;
+    } else {
+        const int64_t most = decode_num_chunks(batch, n_kv, max_seq);
+        int64_t parts = slots / groups;
+        // at one CTA per SM a group per CTA leaves SMs idle, or all of them to one long CTA: two waves of shorter ones
+        if (head_dim == 64 && parts == 2) parts = 1;  // two CTAs per SM do as well as four here and need no merge
+        const bool twice = head_dim == 256 && parts == 1 && ((7 * groups <= 5 * slots && span > 1024) || span > 4096);
+        if (twice) parts = 2 * slots / groups;
+        if (parts > most) parts = most;
+        const int64_t want = ((span + parts - 1) / parts + 63) / 64 * 64;
+        if (want <= (1 << 20)) sp.chunk = (int)want;
+        if (ragged && batch <= 32 && parts > 1 && !twice && span < (1 << 30)) {
+            if (groups * group_bytes >= (40 << 20)) {
+                const int64_t n = (span + 63) / 64;
+                sp.mode = kSplitShare;
+                sp.n_chunks = (int)(n < most ? n : most);
+                sp.batch = (int)batch;
+                // a sequence's last chunk is half empty on average; at most groups chunks are started beyond the target
+                sp.target = (float)(slots - groups / 2);
+                sp.ctas = (int)(slots + groups - groups / 2);
+                return sp;
+            }
+            if (span > 2048) sp.mode = kSplitEven;
+        }
+    }
+    sp.n_chunks = (int)((span + sp.chunk - 1) / sp.chunk);
+    return sp;
 }
 
 cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void* out_bf16, float* out_f32,
@@ -834,25 +885,12 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
     p.max_seq = max_seq;
     p.n_heads = n_heads;
     p.n_kv = n_kv;
-    p.chunk = decode_chunk_tokens(batch, n_kv, max_seq);
     // The visible range can be no longer than this; chunks past it would all be empty.
     int64_t span = max_seq - kv_begin;
     if (!kv_lens && kv_len_uniform - kv_begin < span) span = kv_len_uniform - kv_begin;
     if (kv_end >= 0 && kv_end - kv_begin < span) span = kv_end - kv_begin;
     if (span < 1) span = 1;
-    // A few long sequences (fewer (sequence, KV head) groups than resident CTAs): one wave of longer chunks
-    // streams as fast as several waves of short ones and leaves a fraction of the partials to merge
-    // (one sequence of 131072 positions: 37 chunks instead of 147).  The chunk only ever grows here, so the
-    // chunk count stays within what rt_gqa_decode_workspace_bytes sized the scratch for.
-    {
-        const int64_t groups = batch * (int64_t)n_kv, slots = (int64_t)sm_count() * 2;
-        if (groups < slots) {
-            const int64_t per_group = slots / groups;
-            const int64_t want = ((span + per_group - 1) / per_group + 63) / 64 * 64;
-            if (want > p.chunk && want <= (1 << 20)) p.chunk = (int)want;
-        }
-    }
-    p.n_chunks = (int)((span + p.chunk - 1) / p.chunk);
+    p.split = pick_split(batch, n_kv, head_dim, max_seq, span, kv_lens != nullptr);
     p.rows = batch * n_heads;
     p.of_stride = of_stride > 0 ? of_stride : head_dim;
     p.lse_stride = lse_stride > 0 ? lse_stride : 1;
@@ -866,15 +904,15 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
     bool merged = false;
     if (tail) {  // the caller merges the chunk partials itself (split-KV row exchange)
         counters = nullptr;
-        tail->n_chunks = p.n_chunks;
+        tail->n_chunks = p.split.n_chunks;
         tail->part_o = p.part_o;
         tail->part_lse = p.part_lse;
     }
     cudaError_t e = cudaErrorNotSupported;
     if (decode_use_tensor_cores())
         e = launch_gqa_decode_tc(q, k, v, out_bf16, out_f32, lse, batch, n_heads, n_kv, head_dim, max_seq, kv_lens,
-                                 kv_len_uniform, kv_begin, kv_end, scale, p.part_o, p.part_lse, counters, p.chunk,
-                                 p.n_chunks, p.of_stride, p.lse_stride, &merged, push, stream);
+                                 kv_len_uniform, kv_begin, kv_end, scale, p.part_o, p.part_lse, counters, p.split,
+                                 p.of_stride, p.lse_stride, &merged, push, stream);
     if (e == cudaErrorNotSupported) {  // a cache too large for 32-bit TMA row coordinates, or RT_ATTN_DECODE_IMPL=simt
         switch (head_dim) {
             case 64: e = launch_decode_d<64>(p, group, batch, stream); break;
@@ -885,8 +923,8 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
     }
     if (e != cudaSuccess) return e;
     if (merged && push && push->world > 0 && pushed) *pushed = true;  // delivered by the decode kernel itself
-    if (p.n_chunks > 1 && !merged && !tail) {
-        e = launch_merge_partials(p.part_o, p.part_lse, p.n_chunks, p.rows, head_dim, head_dim, 1, p.out_bf16, p.out_f32, lse,
+    if (p.split.n_chunks > 1 && !merged && !tail) {
+        e = launch_merge_partials(p.part_o, p.part_lse, p.split.n_chunks, p.rows, head_dim, head_dim, 1, p.out_bf16, p.out_f32, lse,
                                   stream, nullptr, push, p.of_stride, p.lse_stride);
         if (e != cudaSuccess) return e;
         if (push && pushed) *pushed = true;

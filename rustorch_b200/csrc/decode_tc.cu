@@ -40,7 +40,7 @@ struct DecodeTcParams {
     int64_t kv_begin, kv_end;
     int64_t max_seq;
     int n_heads, n_kv;
-    int chunk, n_chunks;
+    DecodeSplit split;
     int64_t rows;
     int64_t of_stride, lse_stride;  // floats between consecutive rows of out_f32 / lse
     float scale_log2;
@@ -66,7 +66,7 @@ __device__ __forceinline__ void finish_group(const DecodeTcParams& p, int b, int
     __shared__ float s_red[4][G];
     constexpr int VPL = D / 32;  // dims per lane
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = p.n_chunks;
+    const int n = p.split.n_chunks;
     __threadfence();
     __syncthreads();
     if (tid == 0) s_last = (atomicAdd(&p.counters[b * p.n_kv + kvh], 1) == n - 1);
@@ -252,11 +252,9 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::RING_BYTES);
 
-    const int chunk_idx = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tig = lane & 3;  // mma fragment coordinates: g = head row, tig = column pair
-    const int64_t row0 = (int64_t)b * p.n_heads + (int64_t)kvh * G;
-    const bool direct = (p.n_chunks == 1);
+    const bool direct = (p.split.n_chunks == 1);
 
     // Launched with programmatic stream serialisation, the CTA may be resident before the kernel ahead of it in
     // the stream has finished (the append of this token's K and V rows, the previous step's merge): this
@@ -264,12 +262,18 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     // Nothing is read from global memory before it.
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    int64_t len = p.kv_lens ? (int64_t)p.kv_lens[b] : p.kv_len_uniform;
-    if (len > p.max_seq) len = p.max_seq;
-    const int64_t hi = (p.kv_end >= 0 && p.kv_end < len) ? p.kv_end : len;
-    const int64_t c0 = p.kv_begin + (int64_t)chunk_idx * p.chunk;
-    int64_t c1 = c0 + p.chunk;
-    if (c1 > hi) c1 = hi;
+    const DecodeChunk ck = find_chunk(p.split, p.n_kv, [&](int seq) {  // tokens of a sequence inside the launch's range
+        int64_t len = p.kv_lens ? (int64_t)p.kv_lens[seq] : p.kv_len_uniform;
+        if (len > p.max_seq) len = p.max_seq;
+        if (p.kv_end >= 0 && p.kv_end < len) len = p.kv_end;
+        return len > p.kv_begin ? (int)(len - p.kv_begin) : 0;
+    });
+    if (ck.none) return;
+    const int chunk_idx = ck.idx, kvh = ck.kvh, b = ck.b;
+    const int64_t row0 = (int64_t)b * p.n_heads + (int64_t)kvh * G;  // first output row of the group
+    const int64_t c0 = p.kv_begin + ck.lo, c1 = p.kv_begin + ck.hi;
+    for (int i = tid; i < ck.rest * G; i += 128)
+        p.part_lse[(int64_t)(chunk_idx + 1 + i / G) * p.rows + row0 + i % G] = -INFINITY;
 
     if (c0 >= c1) {  // nothing visible in this chunk: identity partial
         launch_dependents();
@@ -517,7 +521,7 @@ static cudaError_t launch_dg(const CUtensorMap& mk, const CUtensorMap& mv, const
         return !(e && e[0] == '0');
     }();
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.n_chunks, p.n_kv, (unsigned)batch);
+    cfg.gridDim = p.split.mode == kSplitShare ? dim3(p.split.ctas) : dim3(p.split.n_chunks, p.n_kv, (unsigned)batch);
     cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = DecodeTcCfg<D>::SMEM_BYTES;
     cfg.stream = stream;
@@ -548,7 +552,7 @@ static cudaError_t launch_d(const CUtensorMap& mk, const CUtensorMap& mv, const 
 cudaError_t launch_gqa_decode_tc(const void* q, const void* k, const void* v, void* out_bf16, float* out_f32,
                                  float* lse, int64_t batch, int n_heads, int n_kv, int head_dim, int64_t max_seq,
                                  const int32_t* kv_lens, int64_t kv_len_uniform, int64_t kv_begin, int64_t kv_end,
-                                 float scale, float* part_o, float* part_lse, int* counters, int chunk, int n_chunks,
+                                 float scale, float* part_o, float* part_lse, int* counters, const DecodeSplit& split,
                                  int64_t of_stride, int64_t lse_stride, bool* merged, const MergePush* push,
                                  cudaStream_t stream) {
     *merged = false;
@@ -572,8 +576,8 @@ cudaError_t launch_gqa_decode_tc(const void* q, const void* k, const void* v, vo
     p.max_seq = max_seq;
     p.n_heads = n_heads;
     p.n_kv = n_kv;
-    p.chunk = chunk;
-    p.n_chunks = n_chunks;
+    p.split = split;
+    const int n_chunks = split.n_chunks;
     p.rows = batch * n_heads;
     p.of_stride = of_stride;
     p.lse_stride = lse_stride;
@@ -607,7 +611,8 @@ cudaError_t launch_gqa_decode_tc(const void* q, const void* k, const void* v, vo
     constexpr int kMaxFusedChunks = 8;
     const bool many_ctas = batch * n_kv * (int64_t)n_chunks >= 4 * (int64_t)sm_count();
     const bool batched = n_chunks <= kMaxFusedChunks && many_ctas && !pushing;
-    p.counters = (n_chunks > 1 && fits && (batched || push_ok) && !fused_off) ? counters : nullptr;
+    // (kSplitShare: no fixed number of chunks per group to count to)
+    p.counters = (n_chunks > 1 && split.mode != kSplitShare && fits && (batched || push_ok) && !fused_off) ? counters : nullptr;
     p.push = MergePush{};
     if (p.counters) {
         cudaError_t e = cudaMemsetAsync(p.counters, 0, sizeof(int) * (size_t)batch * n_kv, stream);

@@ -68,3 +68,36 @@ def test_host_entry_staged_equals_pinned(precision, B, H, N):
     mixed = np.empty_like(q)
     rt.flash_forward_masked(shape, q, pinned[1], v, mask, mixed, precision)
     assert np.array_equal(out.view(np.uint32), mixed.view(np.uint32))
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,D,S,lens", [
+    (40, 16, 8, 128, 200, (0, 200)),      # at least as many groups as CTAs: whole sequences
+    (40, 8, 8, 64, 300, (1, 300)),        # 64 groups and more, little each: whole
+    (3, 16, 8, 128, 4096, (0, 4096)),     # shares of all tokens, one sequence empty
+    (32, 4, 2, 64, 2600, (5, 2600)),      # the same with a full warp of sequences
+    (2, 8, 1, 256, 2100, (2050, 2099)),   # equal parts of every sequence
+    (5, 4, 2, 128, 1000, (63, 65)),       # fixed parts, most of them empty
+    (90, 1, 1, 256, 1100, (900, 1100)),   # D = 256: two waves
+])
+def test_decode_splits(oracle, B, Hq, Hkv, D, S, lens):
+    """One launch of each rule of the decode split, with lengths at the ends of its range, whole and as a KV range."""
+    import torch
+    import rustorch_b200 as rt
+    r = np.random.default_rng(5)
+    n = r.integers(lens[0], lens[1] + 1, B).astype(np.int32)
+    n[0], n[-1] = lens
+    q = util.normal_bf16(oracle, (B, Hq, D), 1)
+    k, v = (util.normal_bf16(oracle, (B, Hkv, S, D), s) for s in (2, 3))
+    dq, dk, dv, dn = *(util.to_cuda_bf16(x) for x in (q, k, v)), util.to_cuda(n)
+    out, lse = rt.gqa_decode(dq, dk, dv, kv_lens=dn)
+    torch.cuda.synchronize()
+    _, ref, ref_lse = oracle.gqa_decode_cache(q, k, v, n)
+    util.check_output(util.to_np(out), ref, label="whole")
+    util.check_lse(util.to_np(lse), ref_lse)
+    cut = S // 3
+    parts = [rt.gqa_decode(dq, dk, dv, kv_lens=dn, kv_begin=a, kv_end=b, out_dtype=torch.float32)
+             for a, b in ((0, cut), (cut, S))]
+    out, lse = rt.merge_partials(torch.stack([p[0].reshape(B * Hq, D) for p in parts]),
+                                 torch.stack([p[1].reshape(B * Hq) for p in parts]))
+    util.check_output(util.to_np(out).reshape(B, Hq, D), ref, label="range")
+    util.check_lse(util.to_np(lse).reshape(B, Hq), ref_lse)
