@@ -75,7 +75,8 @@ struct TcParams {
     int* status;       // device status word (bounded-wait expiry codes)
     int64_t o_stride_b, o_stride_h, o_stride_row;  // element strides of the output (inner dim contiguous)
     int n_qb;          // 256-row blocks per head
-    int slots_per_head, n_slots, paired;  // static schedule, see tc_item
+    int n_items, units;  // static schedule, see tc_item: items of the launch, (batch, query head) pairs
+    int rounds, tail_head, tail_skip, n_tail;  // paired rounds, and the blocks that they leave
     int sorted;        // length-sorted schedule (launches with per-batch kv_lens), see tc_item
     int stagger_clocks;  // single-tile items: head start of tile 0 over tile 1, in SM clocks
     int direct_out;    // one item per CTA: the epilogue stores its rows straight from registers (no staged tile, no TMA store)
@@ -129,12 +130,16 @@ struct TcItem {
     __device__ __forceinline__ int qrow(int w, bool single) const { return q0 + ((w || single) ? 128 : 0); }
 };
 
-// Static schedule.  The (batch, head)-major slot list is dealt round-robin to the CTAs, so the
-// CTAs running at one time work on a few neighbouring heads and share their K/V in L2.  In
-// paired mode a slot holds the 256-row blocks r and n_qb-1-r of one head, heavy one first: under
-// a causal mask every slot then costs the same, and the CTAs finish together.  A launch with fewer
-// 256-row blocks than 3/4 of the SMs uses 128-row items instead (single_tile): twice the CTAs, and inside
-// a CTA the item's 64-key steps alternate between the two tiles (tile 0 takes the even steps = the first
+// Static schedule.  Under a causal mask the 256-row block of rank n_qb-1 of a head costs n_qb times the first one, so
+// what a launch costs over its work is the balance of the CTAs' lists.  Level t holds the t-th heaviest block of
+// every head; the levels one after the other are dealt to the CTAs boustrophedon (0..G-1, G-1..0, ...), heaviest
+// first.  Without a mask the blocks go out head after head, the ragged last ones (a tile or two of fewer rows: cheaper)
+// at the end.  Where the K/V of all heads exceed L2, `rounds` paired rounds come first: a slot holds the blocks r and
+// n_qb-1-r of one head, so all slots of a round cost the same and its CTAs work on a few neighbouring heads and share
+// their K/V in L2; only the heads left over are dealt by levels.  (Pairs alone left the last round half empty: B=2
+// H=32 N=2409 D=128 141 us against 118, B=4 H=12 N=1794 D=64 62 / 51, B=14 H=16 N=584 D=64 52 / 41.)
+// A launch with fewer 256-row blocks than 3/4 of the SMs uses 128-row items instead (single_tile): twice the CTAs,
+// and inside a CTA the item's 64-key steps alternate between the two tiles (tile 0 takes the even steps = the first
 // half of every 128-key K/V tile, tile 1 the odd ones), each with its own running max, sum and accumulator;
 // the epilogue merges the two partial results straight out of TMEM and stores the rows directly (no staged
 // tile: such a CTA has no further item).  Both softmax warpgroups and both MMA issuers then work on the one
@@ -157,6 +162,7 @@ __device__ __forceinline__ void tc_steps(const TcParams& p, int b, int q0, int& 
     const int last0 = q0 + 127 + q_off, last1 = last0 + 128;  // last key each tile's last row may see
     U0 = !kCausal ? n_steps : (last0 < 0 ? 0 : min(n_steps, last0 / 64 + 1));
     U1 = !kCausal ? n_steps : (last1 < 0 ? 0 : min(n_steps, last1 / 64 + 1));
+    if (!kSingle && q0 + 128 >= p.seq) U1 = 0;  // the second tile of a ragged last block holds no row
     if (kSingle) {  // the block's U1 steps are dealt alternately: even ones to tile 0, odd ones to tile 1
         U0 = (U1 + 1) >> 1;
         U1 = U1 >> 1;
@@ -170,25 +176,55 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
     int qb;
     if (p.sorted) {
         const int G = (int)gridDim.x;
-        it.end = (int64_t)j * G >= (int64_t)p.n_slots;
+        it.end = (int64_t)j * G >= (int64_t)p.n_items;
         if (it.end) return it;
         const int pos = j * G + ((j & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x);
-        if (pos >= p.n_slots) return it;
+        if (pos >= p.n_items) return it;
         const int pair = sched[pos / p.heads];
         qb = pair % p.n_qb;
         it.b = pair / p.n_qb;
         it.h = pos % p.heads;
         it.bh = it.b * p.heads + it.h;
     } else {
-        const int slot = (int)blockIdx.x + (p.paired ? (j >> 1) : j) * (int)gridDim.x;
-        it.end = slot >= p.n_slots;
-        if (it.end) return it;
-        it.bh = slot / p.slots_per_head;
-        const int r = slot % p.slots_per_head;
-        qb = p.n_qb - 1 - r;
-        if (p.paired && (j & 1)) {
-            if (r == qb) return it;  // the middle block of an odd count has no partner
-            qb = r;
+        const int G = (int)gridDim.x;
+        it.end = false;
+        if (kCausal && j < 2 * p.rounds) {
+            const int slot = (int)blockIdx.x + (j >> 1) * G, per_head = (p.n_qb + 1) >> 1, r = slot % per_head;
+            it.bh = slot / per_head;
+            qb = p.n_qb - 1 - r;
+            if (j & 1) {
+                if (r == qb) return it;  // the middle block of an odd count has no partner
+                qb = r;
+            }
+        } else {
+            const int jt = kCausal ? j - 2 * p.rounds : j;
+            it.end = jt * G >= p.n_tail;
+            if (it.end) return it;
+            const int pos = jt * G + ((jt & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x);
+            if (pos >= p.n_tail) return it;
+            if (kCausal) {
+                // level t: the t-th heaviest block of every head left; the head that the rounds end in is missing
+                // from the first and last tail_skip levels
+                const int full = p.units - p.tail_head - 1, mid = p.tail_skip * full,
+                          hi = mid + (p.n_qb - 2 * p.tail_skip) * (full + 1);
+                int t;
+                if (pos < mid) {
+                    t = pos / full;
+                    it.bh = p.tail_head + 1 + pos % full;
+                } else if (pos < hi) {
+                    t = p.tail_skip + (pos - mid) / (full + 1);
+                    it.bh = p.tail_head + (pos - mid) % (full + 1);
+                } else {
+                    t = p.n_qb - p.tail_skip + (pos - hi) / full;
+                    it.bh = p.tail_head + 1 + (pos - hi) % full;
+                }
+                qb = p.n_qb - 1 - t;
+            } else {
+                // head after head; the lighter ragged blocks last
+                const int whole = p.seq / (kSingle ? 128 : 256), n_whole = p.units * whole;
+                it.bh = pos < n_whole ? pos / whole : pos - n_whole;
+                qb = pos < n_whole ? pos % whole : whole;
+            }
         }
         it.b = it.bh / p.heads;
         it.h = it.bh % p.heads;
@@ -199,7 +235,7 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
     // earlier so that the block sits where tile 1 sits in a two-tile item (TcItem::qrow).
     it.q0 = kSingle ? qb * 128 - 128 : qb * 256;
     tc_steps<kCausal, kSingle>(p, it.b, it.q0, it.kv_hi, it.q_off, it.U0, it.U1, keep_hi);
-    it.n_tiles = kSingle ? it.U0 : (it.U1 + 1) / 2;
+    it.n_tiles = kSingle ? it.U0 : (max(it.U0, it.U1) + 1) / 2;
     return it;
 }
 
@@ -260,7 +296,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // Rank sort of the (batch, query block) pairs by their step count, descending, ties by index:
         // every CTA computes the same table.
         uint16_t* cost = sched + C::SCHED_CAP;
-        const int n_pairs = p.n_slots / p.heads;
+        const int n_pairs = p.n_items / p.heads;
         for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
             int kv_hi, q_off, U0, U1;
             tc_steps<kCausal, kSingle>(p, i / p.n_qb, (i % p.n_qb) * 256, kv_hi, q_off, U0, U1);
@@ -344,7 +380,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // the bound (the preload above relies on that); a row that sees no kept key is recognised as before.
         grid_dep_wait();
         if (warp < 8) {
-            const uint8_t* keep = p.key_keep + (int64_t)(((int)blockIdx.x / p.slots_per_head) / p.heads) * p.keep_batch_stride;
+            const uint8_t* keep = p.key_keep + (int64_t)tc_item<kCausal, kSingle>(0, p, sched).b * p.keep_batch_stride;
             int hi = 1;
             for (int i = threadIdx.x; i < Nkv; i += 256)
                 if (__ldg(keep + i)) hi = i + 1;
@@ -1088,12 +1124,15 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
     p.scale_log2 = scale * kLog2e;
     p.status = device_status_ptr();
     if (!p.status) return cudaErrorInvalidSymbol;
-    // Schedule (tc_item).  A causal launch without per-batch lengths has a known cost per item, so
-    // it runs one CTA per SM over a static list in which the 256-row blocks of a head are paired
-    // heavy + light: every CTA gets the same work and the per-item set-up overlaps the previous
-    // item.  Other launches (uniform items, or lengths only the device knows) use one CTA per item
-    // and leave the balancing to the hardware scheduler.  RT_ATTN_PREFILL_SCHED=persistent|percta
-    // overrides the choice.
+    // Schedule (tc_item).  A launch whose items' costs the host knows (no per-batch lengths, and no keep flags unless
+    // a causal mask already orders the items) and that has more items than SMs runs one CTA per SM over a static
+    // list: the set-up of an item overlaps the item before.  With per-batch lengths the list is sorted on the
+    // device.  Other launches use one CTA per item and leave the balancing to the hardware scheduler.
+    // A causal launch whose K and V stay in L2 deals out whole levels, which balances best; a larger one works
+    // through paired rounds, in which the CTAs share a few heads' K/V, down to the last one or two, and deals only
+    // the rest by levels.  (Levels throughout cost 12 % on B=4 H=32 N=4096 D=128, 268 MB of K and V, at full clocks; at
+    // 52 to 140 MB the two are within 1.5 %; at 30 MB and below levels win by up to 18 %.)
+    constexpr int64_t kLevelsKvBytes = 96ll << 20;
     const int n_sm = sm_count();
     // RT_ATTN_PREFILL_TILES=1|2 and RT_ATTN_PREFILL_SCHED=persistent|percta override the choices below
     // (read once per process).
@@ -1124,22 +1163,31 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
     const int64_t n_items = bh * n_qb;
     if (n_items > 0x3fffffff) return cudaErrorInvalidValue;
     p.n_qb = (int)n_qb;
-    bool persistent = causal && kv_lens == nullptr && n_items >= 2 * (int64_t)n_sm && !p.single_tile;
+    bool persistent = kv_lens == nullptr && (causal || key_keep == nullptr) && n_items > (int64_t)n_sm && !p.single_tile;
     if (env_sched == 1 && !p.single_tile) persistent = true;  // a single-tile item is its CTA's only item (the merge reuses barriers)
     if (env_sched == 2) persistent = false;
-    p.paired = (persistent && n_items >= 2 * (int64_t)n_sm) ? 1 : 0;
     // Per-batch lengths: the length-sorted persistent schedule, if its table fits (tc_item).
     p.sorted = 0;
-    if (kv_lens != nullptr && !p.single_tile && env_sched != 2 && n_items >= 2 * (int64_t)n_sm &&
+    if (kv_lens != nullptr && !p.single_tile && env_sched != 2 && n_items > (int64_t)n_sm &&
         batch * n_qb <= (dim == 128 ? TcCfg<128>::SCHED_CAP : TcCfg<64>::SCHED_CAP) && batch * n_qb <= 65535) {
         p.sorted = 1;
-        p.paired = 0;
         persistent = true;
     }
-    p.slots_per_head = p.paired ? (int)((n_qb + 1) / 2) : (int)n_qb;
-    p.n_slots = (int)(bh * p.slots_per_head);
-    const int64_t n_ctas = (persistent && p.n_slots > n_sm) ? n_sm : p.n_slots;
-    p.direct_out = (n_ctas == p.n_slots && !p.paired && !p.sorted) ? 1 : 0;  // every CTA has exactly one item
+    const int64_t n_ctas = (persistent && n_items > n_sm) ? n_sm : n_items;
+    p.n_items = (int)n_items;
+    p.units = (int)bh;
+    p.rounds = p.tail_head = p.tail_skip = 0;
+    p.n_tail = (int)n_items;
+    if (causal && n_ctas < n_items && !p.sorted) {
+        const int64_t per_head = (n_qb + 1) / 2, all = bh * per_head / n_ctas;
+        const int64_t kv_bytes = batch * heads_kv * seq_kv * dim * 4;
+        p.rounds = (kv_bytes > kLevelsKvBytes && all > 1) ? (int)(all - 1) : 0;
+        const int64_t taken = p.rounds * n_ctas;
+        p.tail_head = (int)(taken / per_head);
+        p.tail_skip = (int)(taken % per_head);
+        p.n_tail = p.tail_head == bh ? 0 : (int)((bh - p.tail_head) * n_qb - 2 * p.tail_skip);
+    }
+    p.direct_out = n_ctas == n_items ? 1 : 0;  // every CTA has exactly one item
     const bool keep = key_keep != nullptr;
     p.tighten = (keep && p.direct_out && seq_kv > 0) ? 1 : 0;
 #define RT_TC_DISPATCH(DD)                                                                         \

@@ -101,3 +101,29 @@ def test_decode_splits(oracle, B, Hq, Hkv, D, S, lens):
                                  torch.stack([p[1].reshape(B * Hq) for p in parts]))
     util.check_output(util.to_np(out).reshape(B, Hq, D), ref, label="range")
     util.check_lse(util.to_np(lse).reshape(B, Hq), ref_lse)
+
+
+@pytest.mark.parametrize("B,H,N,D,causal,part", [
+    (28, 20, 1200, 64, True, 7),     # more K/V than L2: paired rounds that end inside a head, levels for the rest
+    (26, 16, 1100, 128, True, 13),   # the same, last tile of a head without rows
+    (12, 16, 300, 64, True, 4),      # levels only; the parts fall below one item per SM
+    (20, 16, 777, 64, False, 5),     # head after head, ragged blocks last
+    (3, 50, 130, 128, False, 3),     # one block more than SMs
+])
+def test_prefill_schedules(B, H, N, D, causal, part):
+    """Every block is visited once whatever the schedule: a launch gives what launches over parts of its batch give."""
+    import torch
+    import rustorch_b200 as rt
+    torch.manual_seed(3)
+    q, k, v = (torch.randn(B, H, N, D, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    out, lse = rt.prefill_bf16(q, k, v, causal=causal)
+    for b in range(0, B, part):
+        o, l = rt.prefill_bf16(*(x[b:b + part] for x in (q, k, v)), causal=causal)
+        assert torch.allclose(out[b:b + part].float(), o.float(), rtol=1e-2, atol=1e-2)
+        assert torch.allclose(lse[b:b + part], l, rtol=1e-5, atol=1e-4)
+    s = q[-1].float() @ k[-1].float().transpose(1, 2) / D ** 0.5
+    if causal:
+        s = s.masked_fill(torch.ones(N, N, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    ref = torch.softmax(s, -1) @ v[-1].float()
+    assert float((out[-1].float() - ref).norm() / ref.norm()) < 1e-2
+    assert torch.allclose(lse[-1], torch.logsumexp(s, -1), rtol=1e-4, atol=1e-3)
