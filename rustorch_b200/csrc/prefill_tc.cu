@@ -28,6 +28,7 @@
 // The normalised O tile is staged in the tile's own (by then idle) Q buffer and leaves through
 // TMA stores.  Every mbarrier wait is bounded; on expiry the kernel records a code in the device
 // status word, drains its own copies and MMAs, frees TMEM and returns.
+#include <algorithm>
 #include <cuda.h>
 #include <cstdlib>
 #include <cstring>
@@ -76,6 +77,7 @@ struct TcParams {
     int64_t o_stride_b, o_stride_h, o_stride_row;  // element strides of the output (inner dim contiguous)
     int n_qb;          // 256-row blocks per head
     int n_items, units;  // static schedule, see tc_item: items of the launch, (batch, query head) pairs
+    int by_level;      // single-tile items: level after level instead of head after head
     int rounds, tail_head, tail_skip, n_tail;  // paired rounds, and the blocks that they leave
     int sorted;        // length-sorted schedule (launches with per-batch kv_lens), see tc_item
     int stagger_clocks;  // single-tile items: head start of tile 0 over tile 1, in SM clocks
@@ -138,12 +140,13 @@ struct TcItem {
 // n_qb-1-r of one head, so all slots of a round cost the same and its CTAs work on a few neighbouring heads and share
 // their K/V in L2; only the heads left over are dealt by levels.  (Pairs alone left the last round half empty: B=2
 // H=32 N=2409 D=128 141 us against 118, B=4 H=12 N=1794 D=64 62 / 51, B=14 H=16 N=584 D=64 52 / 41.)
-// A launch with fewer 256-row blocks than 3/4 of the SMs uses 128-row items instead (single_tile): twice the CTAs,
+// Small launches use 128-row items instead (single_tile, see prefer_single_tile): twice the CTAs,
 // and inside a CTA the item's 64-key steps alternate between the two tiles (tile 0 takes the even steps = the first
 // half of every 128-key K/V tile, tile 1 the odd ones), each with its own running max, sum and accumulator;
 // the epilogue merges the two partial results straight out of TMEM and stores the rows directly (no staged
 // tile: such a CTA has no further item).  Both softmax warpgroups and both MMA issuers then work on the one
-// block, which nearly halves the critical path of a small problem.
+// block, which nearly halves the critical path of a small problem.  More such items than SMs are started level by
+// level as well, heaviest first (H=8 N=4096 D=128: 53 us head after head, 37 by levels).
 // Sorted mode (per-batch kv_lens, where an item's cost is only known on the device): every CTA ranks the
 // (batch, query block) pairs by their step count at start-up (the same deterministic sort in every CTA, so
 // no queue, no atomics and no scratch memory are needed), the item list is that order with all heads of a
@@ -174,7 +177,15 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
     TcItem it;
     it.valid = false;
     int qb;
-    if (p.sorted) {
+    if (kSingle) {  // the CTA's only item
+        it.end = j > 0;
+        if (it.end) return it;
+        const int n = p.by_level ? p.units : p.n_qb, a = (int)blockIdx.x / n, r = (int)blockIdx.x % n;
+        it.bh = p.by_level ? r : a;
+        qb = p.n_qb - 1 - (p.by_level ? a : r);
+        it.b = it.bh / p.heads;
+        it.h = it.bh % p.heads;
+    } else if (p.sorted) {
         const int G = (int)gridDim.x;
         it.end = (int64_t)j * G >= (int64_t)p.n_items;
         if (it.end) return it;
@@ -221,7 +232,7 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
                 qb = p.n_qb - 1 - t;
             } else {
                 // head after head; the lighter ragged blocks last
-                const int whole = p.seq / (kSingle ? 128 : 256), n_whole = p.units * whole;
+                const int whole = p.seq / 256, n_whole = p.units * whole;
                 it.bh = pos < n_whole ? pos / whole : pos - n_whole;
                 qb = pos < n_whole ? pos % whole : whole;
             }
@@ -1090,6 +1101,38 @@ static cudaError_t launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const
                          : launch_tc_s<D, kCausal, kKeep, false>(mq, mk, mv, mo, p, n_ctas, stream);
 }
 
+// Whether a launch runs faster on 128-row items (one per CTA, keys split inside it) than on 256-row items (one CTA per
+// SM works through several).  The first have twice the CTAs and half the time per key, the second less total work:
+// each is priced as the longer of its heaviest item and its share of all items.  Costs in us, from launches
+// of either kind timed over B*H = 8..448, N = 37..4096: per 128 keys and per item.  (They picked
+// the faster kind or one within 10 % of it on 57 of 57 shapes, within 3 % on 54; the block-count rule that this
+// replaces took 33 us instead of 23 on H=16 N=1795 D=128, 49 / 27 on H=8 N=3500 D=64, 99 / 74 on a 97-row chunk
+// against 10190 keys.)  Lengths that only the device knows are taken at their largest.
+static bool prefer_single_tile(int64_t bh, int64_t seq, int64_t seq_kv, int64_t dim, bool causal, bool offsets, int n_sm) {
+    const int64_t n1 = (seq + 127) / 128, n2 = (seq + 255) / 256;
+    if (bh * n2 >= 8 * (int64_t)n_sm) return false;  // many items: the lower total wins, and no loop over long heads
+    const double key1 = dim == 128 ? 1.0 : 0.84, item1 = dim == 128 ? 4.8 : 4.2;  // 128-row items
+    const double key2 = dim == 128 ? 2.0 : 1.7, key2_one = 1.1, item2 = 3.0, first2 = 2.5;  // 256-row items
+    const int64_t all = (seq_kv + 127) / 128, off = (causal && offsets && seq_kv > seq) ? seq_kv - seq : 0;
+    auto tiles = [&](int64_t row_end) { return causal ? std::min(all, (off + std::min(row_end, seq) + 127) / 128) : all; };
+    double sum1 = 0, max1 = 0, sum2 = 0, max2 = 0;
+    for (int64_t i = 0; i < n1; ++i) {
+        const double c = (double)tiles((i + 1) * 128) * key1 + item1;
+        sum1 += c;
+        max1 = std::max(max1, c);
+    }
+    for (int64_t i = 0; i < n2; ++i) {
+        const double c = (double)tiles((i + 1) * 256) * (i * 256 + 128 >= seq ? key2_one : key2) + item2;
+        sum2 += c;
+        max2 = std::max(max2, c);
+    }
+    // equal items come in whole waves; a causal list is dealt out to within about 8 %
+    auto span = [&](double sum, double mx, int64_t n) {
+        return causal ? std::max(mx, 1.08 * sum * (double)bh / n_sm) : mx * (double)((bh * n + n_sm - 1) / n_sm);
+    };
+    return span(sum1, max1, n1) < span(sum2, max2, n2) + first2;
+}
+
 cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void* out, float* lse, int64_t batch,
                               int64_t heads, int64_t heads_kv, int64_t seq, int64_t seq_kv, int dim,
                               const TensorStrides& sq, const TensorStrides& sk, const TensorStrides& sv,
@@ -1144,14 +1187,7 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
         const char* s = getenv("RT_ATTN_PREFILL_SCHED");
         return (s && !strcmp(s, "persistent")) ? 1 : (s && !strcmp(s, "percta")) ? 2 : 0;
     }();
-    // 128-row items (key split inside the CTA) for launches of fewer 256-row blocks than 3/4 of the SMs, and for
-    // long sequences up to the point where the persistent schedule takes over: with 64 and more key steps per
-    // block the finer items pack the causal imbalance better than they lose per step (measured on B=1 H=8 / 16,
-    // N=4096, D=128: 58.6 / 93.7 us against 62.4 / 98.4; at N=2048 the two are level or 256-row items win).
-    const int64_t n_blocks256 = bh * ((seq + 255) / 256);
-    p.single_tile = (seq > 128 && (n_blocks256 * 4 < 3 * (int64_t)n_sm ||
-                                   (n_blocks256 < 2 * (int64_t)n_sm && seq_kv >= 4096 && causal && kv_lens == nullptr)))
-                        ? 1 : 0;
+    p.single_tile = prefer_single_tile(bh, seq, seq_kv, dim, causal, q_offsets != nullptr, n_sm) ? 1 : 0;
     static const int env_stagger = [] {
         const char* s = getenv("RT_ATTN_PREFILL_STAGGER");
         return s ? atoi(s) : 900;
@@ -1178,6 +1214,7 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
     p.units = (int)bh;
     p.rounds = p.tail_head = p.tail_skip = 0;
     p.n_tail = (int)n_items;
+    p.by_level = n_items > n_sm ? 1 : 0;
     if (causal && n_ctas < n_items && !p.sorted) {
         const int64_t per_head = (n_qb + 1) / 2, all = bh * per_head / n_ctas;
         const int64_t kv_bytes = batch * heads_kv * seq_kv * dim * 4;

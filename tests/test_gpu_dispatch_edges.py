@@ -109,6 +109,8 @@ def test_decode_splits(oracle, B, Hq, Hkv, D, S, lens):
     (12, 16, 300, 64, True, 4),      # levels only; the parts fall below one item per SM
     (20, 16, 777, 64, False, 5),     # head after head, ragged blocks last
     (3, 50, 130, 128, False, 3),     # one block more than SMs
+    (6, 16, 1000, 128, True, 2),     # the parts: more 128-row items than SMs, by levels
+    (4, 16, 100, 64, True, 1),       # one ragged 128-row item per head
 ])
 def test_prefill_schedules(B, H, N, D, causal, part):
     """Every block is visited once whatever the schedule: a launch gives what launches over parts of its batch give."""
