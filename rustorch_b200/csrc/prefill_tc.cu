@@ -80,6 +80,7 @@ struct TcParams {
     int by_level;      // single-tile items: level after level instead of head after head
     int rounds, tail_head, tail_skip, n_tail;  // paired rounds, and the blocks that they leave
     int sorted;        // length-sorted schedule (launches with per-batch kv_lens), see tc_item
+    int keep_tab;      // sorted schedule with key_keep: index of the per-batch step bounds behind the order in the table, else 0
     int stagger_clocks;  // single-tile items: head start of tile 0 over tile 1, in SM clocks
     int direct_out;    // one item per CTA: the epilogue stores its rows straight from registers (no staged tile, no TMA store)
     int tighten;       // key_keep launches of one item per CTA: trailing hidden keys are found at start-up and not visited
@@ -196,6 +197,7 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
         it.b = pair / p.n_qb;
         it.h = pos % p.heads;
         it.bh = it.b * p.heads + it.h;
+        if (p.keep_tab) keep_hi = 64 * sched[p.keep_tab + it.b];
     } else {
         const int G = (int)gridDim.x;
         it.end = false;
@@ -308,9 +310,30 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // every CTA computes the same table.
         uint16_t* cost = sched + C::SCHED_CAP;
         const int n_pairs = p.n_items / p.heads;
+        if (kKeep && p.keep_tab) {
+            // The last kept key of every batch bounds its steps as a length would: each warp looks for it from the
+            // end, 256 flags at a time (hidden tails beyond 4096 keys are not searched further).  At least one
+            // step stays, so that rows without a kept key are recognised as in the other schedules.
+            for (int b = warp; b < n_pairs / p.n_qb; b += 12) {
+                const uint8_t* keep = p.key_keep + (int64_t)b * p.keep_batch_stride;
+                int hi = 0, end = Nkv;
+                for (int round = 0; round < 16 && end > 0 && hi == 0; ++round, end -= 256) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int k = end - 1 - (i * 32 + lane);
+                        if (k >= 0 && __ldg(keep + k) != 0) hi = max(hi, k + 1);
+                    }
+                    hi = __reduce_max_sync(kFullMask, hi);
+                }
+                hi = max(hi, max(end, 1));  // end: where the search stopped
+                if (lane == 0) sched[p.keep_tab + b] = (uint16_t)((hi + 63) / 64);
+            }
+            __syncthreads();
+        }
         for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
             int kv_hi, q_off, U0, U1;
-            tc_steps<kCausal, kSingle>(p, i / p.n_qb, (i % p.n_qb) * 256, kv_hi, q_off, U0, U1);
+            const int keep_hi = (kKeep && p.keep_tab) ? 64 * sched[p.keep_tab + i / p.n_qb] : 0x7fffffff;
+            tc_steps<kCausal, kSingle>(p, i / p.n_qb, (i % p.n_qb) * 256, kv_hi, q_off, U0, U1, keep_hi);
             cost[i] = (uint16_t)min(U0 + U1, 65535);
         }
         __syncthreads();
@@ -1202,11 +1225,16 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
     bool persistent = kv_lens == nullptr && (causal || key_keep == nullptr) && n_items > (int64_t)n_sm && !p.single_tile;
     if (env_sched == 1 && !p.single_tile) persistent = true;  // a single-tile item is its CTA's only item (the merge reuses barriers)
     if (env_sched == 2) persistent = false;
-    // Per-batch lengths: the length-sorted persistent schedule, if its table fits (tc_item).
-    p.sorted = 0;
-    if (kv_lens != nullptr && !p.single_tile && env_sched != 2 && n_items > (int64_t)n_sm &&
-        batch * n_qb <= (dim == 128 ? TcCfg<128>::SCHED_CAP : TcCfg<64>::SCHED_CAP) && batch * n_qb <= 65535) {
+    // Per-batch lengths: the length-sorted persistent schedule, if its table fits (tc_item).  Keep flags are the same
+    // with a length that every CTA has to look up first, about 0.7 us for 12 sequences; an item saves 3 us of set-up,
+    // so at least 12 blocks per sequence are asked for.  (B=8 H=12 N=777 D=64 with padding: 45 us one CTA per item.)
+    p.sorted = p.keep_tab = 0;
+    const int64_t n_pairs = batch * n_qb, cap = dim == 128 ? TcCfg<128>::SCHED_CAP : TcCfg<64>::SCHED_CAP;
+    const bool keep_sorted = key_keep != nullptr && heads * n_qb >= 12 && n_pairs + batch <= cap && seq_kv <= 4000000 && seq_kv > 0;
+    if ((kv_lens != nullptr || keep_sorted) && !p.single_tile && env_sched != 2 && n_items > (int64_t)n_sm &&
+        n_pairs <= cap && n_pairs <= 65535) {
         p.sorted = 1;
+        p.keep_tab = keep_sorted ? (int)n_pairs : 0;
         persistent = true;
     }
     const int64_t n_ctas = (persistent && n_items > n_sm) ? n_sm : n_items;

@@ -129,3 +129,31 @@ def test_prefill_schedules(B, H, N, D, causal, part):
     ref = torch.softmax(s, -1) @ v[-1].float()
     assert float((out[-1].float() - ref).norm() / ref.norm()) < 1e-2
     assert torch.allclose(lse[-1], torch.logsumexp(s, -1), rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("B,H,N,Nkv,D,causal", [(9, 12, 600, 600, 64, False), (9, 12, 600, 600, 128, True),
+                                                 (6, 30, 200, 9000, 64, False), (13, 12, 257, 300, 128, False)])
+def test_keep_flags_sorted(B, H, N, Nkv, D, causal):
+    """Keep flags in the sorted schedule (tails of every length, beyond the searched 4096 keys too, holes, nothing kept)."""
+    import torch
+    import rustorch_b200 as rt
+    torch.manual_seed(4)
+    q = torch.randn(B, H, N, D, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(B, H, Nkv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    keep = torch.ones(B, Nkv, device="cuda", dtype=torch.uint8)
+    for b, hidden in enumerate([0, 1, 64, Nkv - 1, 300, Nkv // 2][:B]):
+        keep[b, Nkv - hidden:] = 0
+    keep[1, 5:90] = 0
+    keep[2] = 0
+    out, lse = rt.prefill_bf16(q, k, v, causal=causal, key_keep=keep)
+    for b in range(B):
+        s = q[b].float() @ k[b].float().transpose(1, 2) / D ** 0.5
+        s = s.masked_fill(keep[b] == 0, float("-inf"))
+        if causal:
+            s = s.masked_fill(torch.ones(N, Nkv, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+        ref = torch.softmax(s, -1) @ v[b].float()
+        dead = torch.isinf(s).all(-1)
+        assert torch.equal(torch.isnan(out[b]).all(-1), dead) and torch.equal(lse[b] == float("-inf"), dead)
+        x, y = out[b].float()[~dead], ref[~dead]
+        assert float((x - y).norm()) <= 1e-2 * float(y.norm())
+        assert torch.allclose(lse[b][~dead], torch.logsumexp(s, -1)[~dead], rtol=1e-4, atol=1e-3)
