@@ -29,6 +29,7 @@
 // TMA stores.  Every mbarrier wait is bounded; on expiry the kernel records a code in the device
 // status word, drains its own copies and MMAs, frees TMEM and returns.
 #include <algorithm>
+#include <atomic>
 #include <cuda.h>
 #include <cstdlib>
 #include <cstring>
@@ -84,6 +85,7 @@ struct TcParams {
     int stagger_clocks;  // single-tile items: head start of tile 0 over tile 1, in SM clocks
     int direct_out;    // one item per CTA: the epilogue stores its rows straight from registers (no staged tile, no TMA store)
     int tighten;       // key_keep launches of one item per CTA: trailing hidden keys are found at start-up and not visited
+    int split;         // CTAs (one cluster) that share the keys of a single-tile item
     int single_tile;   // items are 128-row blocks whose 64-key steps alternate between the two tiles (small launches, see tc_item)
 };
 
@@ -118,6 +120,28 @@ __device__ __forceinline__ float2 exp2_poly2(float2 x) {
 // than that costs more issue slots on the FMA pipe than it frees on the MUFU pipe).
 __host__ __device__ constexpr bool poly_pair(int q) { return (q & 3) == 3; }
 
+// All threads of the cluster: their shared-memory writes before it are visible to all after it.  (Threads that have
+// exited count as arrived; every wait on the way here is bounded.)
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// The address in CTA `rank` of the cluster of what lies at `a` in this one.
+__device__ __forceinline__ uint32_t map_cluster(uint32_t a, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float2 ld_cluster_f2(uint32_t a) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -126,6 +150,7 @@ struct TcItem {
     int bh, b, h, h_kv, q0, kv_hi, q_off;  // bh = b * heads + h indexes LSE; h_kv is the KV head h reads
     int U0, U1;    // 64-key steps of each Q tile; scalars, so nothing is indexed dynamically
     int n_tiles;   // 128-key K/V tiles to load
+    int t0;        // first of them (split items: each CTA of the cluster takes its own run of tiles)
     bool end;      // the list is exhausted
     bool valid;    // false: this position of the list holds no item
     __device__ __forceinline__ int steps(int w) const { return w ? U1 : U0; }
@@ -141,7 +166,7 @@ struct TcItem {
 // n_qb-1-r of one head, so all slots of a round cost the same and its CTAs work on a few neighbouring heads and share
 // their K/V in L2; only the heads left over are dealt by levels.  (Pairs alone left the last round half empty: B=2
 // H=32 N=2409 D=128 141 us against 118, B=4 H=12 N=1794 D=64 62 / 51, B=14 H=16 N=584 D=64 52 / 41.)
-// Small launches use 128-row items instead (single_tile, see prefer_single_tile): twice the CTAs,
+// Small launches use 128-row items instead (single_tile, see choose_items): twice the CTAs,
 // and inside a CTA the item's 64-key steps alternate between the two tiles (tile 0 takes the even steps = the first
 // half of every 128-key K/V tile, tile 1 the odd ones), each with its own running max, sum and accumulator;
 // the epilogue merges the two partial results straight out of TMEM and stores the rows directly (no staged
@@ -155,7 +180,7 @@ struct TcItem {
 // persistent kernel's overlap of one item's set-up with the previous item's tail, and a balanced finish.
 template <bool kCausal, bool kSingle>
 __device__ __forceinline__ void tc_steps(const TcParams& p, int b, int q0, int& kv_hi, int& q_off, int& U0, int& U1,
-                                         int keep_hi = 0x7fffffff) {
+                                         int keep_hi = 0x7fffffff, int* t0 = nullptr) {
     kv_hi = min(p.seq_kv, keep_hi);
     if (p.kv_lens) {
         const int l = p.kv_lens[b];
@@ -167,6 +192,11 @@ __device__ __forceinline__ void tc_steps(const TcParams& p, int b, int q0, int& 
     U0 = !kCausal ? n_steps : (last0 < 0 ? 0 : min(n_steps, last0 / 64 + 1));
     U1 = !kCausal ? n_steps : (last1 < 0 ? 0 : min(n_steps, last1 / 64 + 1));
     if (!kSingle && q0 + 128 >= p.seq) U1 = 0;  // the second tile of a ragged last block holds no row
+    if (kSingle && t0) {  // this CTA's share of the steps
+        const int per = ((U1 + 1) / 2 + p.split - 1) / p.split;
+        *t0 = ((int)blockIdx.x % p.split) * per;
+        U1 = max(0, min(U1 - 2 * *t0, 2 * per));
+    }
     if (kSingle) {  // the block's U1 steps are dealt alternately: even ones to tile 0, odd ones to tile 1
         U0 = (U1 + 1) >> 1;
         U1 = U1 >> 1;
@@ -177,11 +207,12 @@ template <bool kCausal, bool kSingle>
 __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16_t* sched, int keep_hi = 0x7fffffff) {
     TcItem it;
     it.valid = false;
+    it.t0 = 0;
     int qb;
     if (kSingle) {  // the CTA's only item
         it.end = j > 0;
         if (it.end) return it;
-        const int n = p.by_level ? p.units : p.n_qb, a = (int)blockIdx.x / n, r = (int)blockIdx.x % n;
+        const int n = p.by_level ? p.units : p.n_qb, item = (int)blockIdx.x / p.split, a = item / n, r = item % n;
         it.bh = p.by_level ? r : a;
         qb = p.n_qb - 1 - (p.by_level ? a : r);
         it.b = it.bh / p.heads;
@@ -247,9 +278,54 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
     // Single-tile items: block qb covers rows [128 qb, 128 qb + 128); the item's origin is kept 128 rows
     // earlier so that the block sits where tile 1 sits in a two-tile item (TcItem::qrow).
     it.q0 = kSingle ? qb * 128 - 128 : qb * 256;
-    tc_steps<kCausal, kSingle>(p, it.b, it.q0, it.kv_hi, it.q_off, it.U0, it.U1, keep_hi);
+    tc_steps<kCausal, kSingle>(p, it.b, it.q0, it.kv_hi, it.q_off, it.U0, it.U1, keep_hi, kSingle ? &it.t0 : nullptr);
     it.n_tiles = kSingle ? it.U0 : (max(it.U0, it.U1) + 1) / 2;
     return it;
+}
+
+// The rows of a split item: thread i of the 256 takes 4 columns of every (1024 / D)-th row of this CTA's 128 / C rows
+// from the shared memory of all C CTAs, merges them and stores them.  All of a thread's remote loads are in flight
+// together (read row by row, the 0.7 us of each round trip added 5 us to an item).
+template <int D, int C>
+__device__ __forceinline__ void merge_cluster(const TcParams& p, const TcItem& it, uint32_t parts, uint32_t stats) {
+    constexpr int kPer = 128 / C * (D / 4) / 256;
+    const int row0 = (int)blockIdx.x % C * (128 / C);
+    float2 ml[kPer][C];
+    float4 x[kPer][C];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int i = threadIdx.x + k * 256, row = row0 + i / (D / 4), ch = i % (D / 4);
+#pragma unroll
+        for (int r = 0; r < C; ++r) {
+            ml[k][r] = ld_cluster_f2(map_cluster(stats + row * 8, r));
+            x[k][r] = ld_cluster_f4(map_cluster(parts + row * (D * 4) + ((ch ^ (row & 7)) << 4), r));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int i = threadIdx.x + k * 256, ch = i % (D / 4), row = it.qrow(1, true) + row0 + i / (D / 4);
+        float m = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int r = 0; r < C; ++r) m = fmaxf(m, ml[k][r].x);
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < C; ++r)
+            if (ml[k][r].x > -INFINITY) {
+                const float f = fast_exp2((ml[k][r].x - m) * p.scale_log2);
+                l += f * ml[k][r].y;
+                o = make_float4(o.x + f * x[k][r].x, o.y + f * x[k][r].y, o.z + f * x[k][r].z, o.w + f * x[k][r].w);
+            }
+        const bool seen = m > -INFINITY, valid = seen && l > 0.f;
+        const float inv = valid ? 1.f / l : 0.f;
+        if (row < p.seq) {
+            *reinterpret_cast<uint2*>(p.out + it.b * p.o_stride_b + it.h * p.o_stride_h + (int64_t)row * p.o_stride_row + ch * 4) =
+                valid ? make_uint2(float2_to_bf16x2(o.x * inv, o.y * inv), float2_to_bf16x2(o.z * inv, o.w * inv))
+                      : make_uint2(0x7fc07fc0u, 0x7fc07fc0u);
+            if (ch == 0 && p.lse)
+                p.lse[(int64_t)it.bh * p.seq + row] =
+                    valid ? (m * p.scale_log2 + fast_log2(l)) * kLn2 : (seen ? NAN : -INFINITY);
+        }
+    }
 }
 
 // Pipeline, per Q tile w and 64-key step u (buffer b = u & 1):
@@ -262,7 +338,7 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
 // (o_free: the next item's first PV may overwrite it), stages it in the Q buffer (stage_full),
 // one thread stores it (q_empty: the next item's Q may land).  A tile that sees no key in an
 // item takes no part in these (its rows are written as NaN directly).
-template <int D, bool kCausal, bool kKeep, bool kSingle>
+template <int D, bool kCausal, bool kKeep, bool kSingle, bool kSplit>
 __global__ void __launch_bounds__(384, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -387,7 +463,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 mbar_arrive_expect_tx(&k_full[0], TILE);
 #pragma unroll
                 for (int s = 0; s < C::NSUB; ++s)
-                    tma_load_4d(sK + s * SUB, &tm_k, &k_full[0], s * 64, 0, it.h_kv, it.b);
+                    tma_load_4d(sK + s * SUB, &tm_k, &k_full[0], s * 64, it.t0 * 128, it.h_kv, it.b);
             }
             for (int w = 0; w < 2 && !kSingle; ++w) {
                 if (it.steps(w) == 0) continue;
@@ -460,7 +536,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     mbar_arrive_expect_tx(&k_full[ks], TILE);
 #pragma unroll
                     for (int s = 0; s < C::NSUB; ++s)
-                        tma_load_4d(sK + ks * TILE + s * SUB, &tm_k, &k_full[ks], s * 64, t * 128, it.h_kv, it.b);
+                        tma_load_4d(sK + ks * TILE + s * SUB, &tm_k, &k_full[ks], s * 64, (it.t0 + t) * 128, it.h_kv, it.b);
                     ++kg;
                     return true;
                 };
@@ -475,7 +551,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     mbar_arrive_expect_tx(&v_full[vs], TILE);
 #pragma unroll
                     for (int s = 0; s < C::NSUB; ++s)
-                        tma_load_4d(sV + vs * TILE + s * SUB, &tm_v, &v_full[vs], s * 64, t * 128, it.h_kv, it.b);
+                        tma_load_4d(sV + vs * TILE + s * SUB, &tm_v, &v_full[vs], s * 64, (it.t0 + t) * 128, it.h_kv, it.b);
                     ++vg;
                 }
                 // Drain: every copy this thread issued must have landed before the CTA may exit.
@@ -675,6 +751,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             wait(done_bar, 0, kToDone);
         }
       }  // warp 11 idle: it only completes the warpgroup for setmaxnreg
+      if constexpr (kSplit) {
+          __syncwarp();
+          cluster_sync_all();
+          cluster_sync_all();
+      }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
         // ============================================================== softmax / epilogue warps
@@ -701,7 +782,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
             // The tile sees no key: NaN rows, LSE = -inf (cpu_forward.rs:411-420).  A single-tile item whose
             // other tile has a step still goes through the merge below with an empty partial result.
-            if (n_iter == 0 && !(il && it.n_tiles > 0)) {
+            if (n_iter == 0 && !kSplit && !(il && it.n_tiles > 0)) {
                 if (row < N && !(il && w == 0)) {
                     uint4* dst = reinterpret_cast<uint4*>(p.out + it.b * p.o_stride_b + it.h * p.o_stride_h +
                                                           (int64_t)row * p.o_stride_row);
@@ -717,7 +798,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             bool seen = false;  // the row has met a score that no mask hides
             for (int u = 0; u < n_iter; ++u) {
                 const int buf = u & 1;
-                const int col0 = (il ? 2 * u + w : u) * 64;
+                const int col0 = (il ? 2 * (it.t0 + u) + w : u) * 64;
                 uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;
                 if (kKeep) {
                     // Mask::Padding keep flags (mask.rs:44) of the step's 64 keys as two 32-bit words: each lane reads
@@ -888,7 +969,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 const float l_all = f_own * l + f_oth * l_o;
                 const bool valid = seen_any && (l_all > 0.f);
                 const float inv = valid ? 1.f / l_all : 0.f;
-                const float a_own = f_own * inv, a_oth = f_oth * inv;
+                const float a_own = kSplit ? f_own : f_own * inv, a_oth = kSplit ? f_oth : f_oth * inv;
                 const bool has_own = n_iter > 0, has_oth = it.steps(1 - w) > 0;  // an idle tile's accumulator was never written
                 // The merged half rows go straight to global memory (64 or 128 contiguous bytes per thread): the CTA
                 // has no further item, and a staged tile, its barrier and a TMA store would only lengthen the
@@ -898,6 +979,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 for (int cq = 0; cq < D / 64; ++cq) {
                     const int ch = w * (D / 64) + cq;
                     uint32_t oa[32], ob[32];
+                    float part[32];
                     if (has_own) tmem_ld32(tO + ch * 32, oa);
                     if (has_oth) tmem_ld32(tO_other + ch * 32, ob);
                     tc_wait_ld();
@@ -913,11 +995,22 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                             const float x1 = (has_own ? __uint_as_float(oa[e + 1]) * a_own : 0.f) +
                                              (has_oth ? __uint_as_float(ob[e + 1]) * a_oth : 0.f);
                             pw[i] = valid ? float2_to_bf16x2(x0, x1) : 0x7fc07fc0u;
+                            if constexpr (kSplit) part[e] = x0, part[e + 1] = x1;
                         }
-                        if (row < N) *reinterpret_cast<uint4*>(dst + ch * 32 + v4 * 8) = pack;
+                        if (!kSplit && row < N) *reinterpret_cast<uint4*>(dst + ch * 32 + v4 * 8) = pack;
+                    }
+                    if constexpr (kSplit) {
+                        // This CTA's partial row, relative to m_all, in f32 over the K ring (every MMA of the CTA has
+                        // retired): 16-byte chunks swizzled by the row, so that 8 lanes' rows meet 8 bank groups.
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            *reinterpret_cast<float4*>(sK + row_in_tile * (D * 4) + (((ch * 8 + i) ^ (row_in_tile & 7)) << 4)) =
+                                make_float4(part[4 * i], part[4 * i + 1], part[4 * i + 2], part[4 * i + 3]);
                     }
                 }
-                if (w == 1 && p.lse && row < N)
+                if (kSplit && w == 1)
+                    reinterpret_cast<float2*>(sV)[row_in_tile] = make_float2(seen_any ? m_all : -INFINITY, l_all);
+                if (!kSplit && w == 1 && p.lse && row < N)
                     p.lse[(int64_t)bh * N + row] =
                         valid ? (m_all * c + fast_log2(l_all)) * kLn2 : (seen_any ? NAN : -INFINITY);
             } else {
@@ -978,6 +1071,18 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             cs0 += (n_iter + 1) / 2;
             cs1 += n_iter / 2;
             co += n_iter;
+        }
+        if constexpr (kSplit) {
+            // ---- the cluster's partial rows: CTA r reads its 128 / split rows from every CTA's shared memory, merges them
+            // as above and stores them.  (A CTA that gave up on a wait still meets the barriers.)
+            cluster_sync_all();
+            const TcItem it = tc_item<kCausal, kSingle>(0, p, sched, keep_hi);
+            if (ok) {
+                if (p.split == 2) merge_cluster<D, 2>(p, it, smem_u32(sK), smem_u32(sV));
+                else if (p.split == 4) merge_cluster<D, 4>(p, it, smem_u32(sK), smem_u32(sV));
+                else merge_cluster<D, 8>(p, it, smem_u32(sK), smem_u32(sV));
+            }
+            cluster_sync_all();  // no CTA leaves while its partial rows are being read
         }
     }
 
@@ -1088,11 +1193,11 @@ bool make_tensor_map_bf16_3d(CUtensorMap* map, const void* base, int64_t bh, int
     return encode_bf16_map_cached(map, 3, base, dims, strides, box);
 }
 
-template <int D, bool kCausal, bool kKeep, bool kSingle>
+template <int D, bool kCausal, bool kKeep, bool kSingle, bool kSplit>
 static cudaError_t launch_tc_s(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                              const TcParams& p, int64_t n_ctas, cudaStream_t stream) {
-    auto kern = prefill_tc_kernel<D, kCausal, kKeep, kSingle>;
-    cudaError_t e = set_max_dynamic_smem_once<prefill_tc_kernel<D, kCausal, kKeep, kSingle>>(TcCfg<D>::SMEM_BYTES);
+    auto kern = prefill_tc_kernel<D, kCausal, kKeep, kSingle, kSplit>;
+    cudaError_t e = set_max_dynamic_smem_once<prefill_tc_kernel<D, kCausal, kKeep, kSingle, kSplit>>(TcCfg<D>::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     // RT_ATTN_PREFILL_PDL=0|1 forces programmatic stream serialization off or on.
     static const int env_pdl = [] {
@@ -1101,7 +1206,7 @@ static cudaError_t launch_tc_s(const CUtensorMap& mq, const CUtensorMap& mk, con
     }();
     // Measured: the overlap pays for short single-tile launches (up to 1 us of 9-16 us); for long ones the
     // dependency wait costs as much as the launch gap it hides.
-    const bool pdl = env_pdl >= 0 ? env_pdl == 1 : (kSingle && p.seq_kv <= 1024);
+    const bool pdl = !kSplit && (env_pdl >= 0 ? env_pdl == 1 : (kSingle && p.seq_kv <= 1024));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_ctas);
     cfg.blockDim = dim3(384);
@@ -1114,46 +1219,100 @@ static cudaError_t launch_tc_s(const CUtensorMap& mq, const CUtensorMap& mk, con
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
+    if constexpr (kSplit) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)p.split;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
     return cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, mo, p);
 }
 
 template <int D, bool kCausal, bool kKeep>
 static cudaError_t launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                              const TcParams& p, int64_t n_ctas, cudaStream_t stream) {
-    return p.single_tile ? launch_tc_s<D, kCausal, kKeep, true>(mq, mk, mv, mo, p, n_ctas, stream)
-                         : launch_tc_s<D, kCausal, kKeep, false>(mq, mk, mv, mo, p, n_ctas, stream);
+    if constexpr (!kKeep)
+        if (p.split > 1) return launch_tc_s<D, kCausal, false, true, true>(mq, mk, mv, mo, p, n_ctas * p.split, stream);
+    return p.single_tile ? launch_tc_s<D, kCausal, kKeep, true, false>(mq, mk, mv, mo, p, n_ctas, stream)
+                         : launch_tc_s<D, kCausal, kKeep, false, false>(mq, mk, mv, mo, p, n_ctas, stream);
 }
 
-// Whether a launch runs faster on 128-row items (one per CTA, keys split inside it) than on 256-row items (one CTA per
-// SM works through several).  The first have twice the CTAs and half the time per key, the second less total work:
-// each is priced as the longer of its heaviest item and its share of all items.  Costs in us, from launches
-// of either kind timed over B*H = 8..448, N = 37..4096: per 128 keys and per item.  (They picked
-// the faster kind or one within 10 % of it on 57 of 57 shapes, within 3 % on 54; the block-count rule that this
-// replaces took 33 us instead of 23 on H=16 N=1795 D=128, 49 / 27 on H=8 N=3500 D=64, 99 / 74 on a 97-row chunk
-// against 10190 keys.)  Lengths that only the device knows are taken at their largest.
-static bool prefer_single_tile(int64_t bh, int64_t seq, int64_t seq_kv, int64_t dim, bool causal, bool offsets, int n_sm) {
+// CTAs that clusters of `split` CTAs can have resident on the current device: GPCs hold whole clusters only, and how many
+// depends on the part (this one: 74 clusters of 2, 33 of 4, 15 of 8).  Asked once per device and size.
+static int cluster_slots(int split) {
+    static std::atomic<int> known[64][3];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::atomic<int>& slot = known[dev][split == 2 ? 0 : split == 4 ? 1 : 2];
+    int n = slot.load(std::memory_order_relaxed);
+    if (n > 0) return n - 1;
+    auto kern = prefill_tc_kernel<128, true, false, true, true>;
+    if (set_max_dynamic_smem_once<prefill_tc_kernel<128, true, false, true, true>>(TcCfg<128>::SMEM_BYTES) != cudaSuccess) return 0;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)split;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(split * 256));
+    cfg.blockDim = dim3(384);
+    cfg.dynamicSmemBytes = TcCfg<128>::SMEM_BYTES;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    slot.store(n * split + 1, std::memory_order_relaxed);
+    return n * split;
+}
+
+// What a launch's items are: 0 for 256-row items (one CTA per SM works through several), 1 for 128-row items (one per
+// CTA, keys split inside it), 2, 4 or 8 for 128-row items whose keys a cluster of so many CTAs shares.  The second
+// kind has twice the CTAs and half the time per key, the third a shorter chain still for launches that leave SMs idle
+// (a prompt chunk against a long cache), the first the least total work: each is priced as the longer of
+// its heaviest CTA and the SMs' share of all CTAs.  Costs in us, from launches timed over B*H = 8..448, N = 37..4096:
+// per 128 keys, per item, and for the merge across a cluster.
+// (Clusters: B=2 H=16/2 123 rows against 8400 keys D=128 50 -> 23 us, H=8/1 64 rows against 2048 keys 18 -> 11, H=4/1
+// 100 rows against 20000 keys D=64 130 -> 24.)  (Between the first two they picked the faster kind
+// or one within 10 % of it on 57 of 57 shapes, within 3 % on 54; the block-count rule that this replaces took
+// 33 us instead of 23 on H=16 N=1795 D=128, 49 / 27 on H=8 N=3500 D=64.)  Lengths that only the
+// device knows are taken at their largest.
+static int choose_items(int64_t bh, int64_t seq, int64_t seq_kv, int64_t dim, bool causal, bool offsets, bool may_split, int n_sm) {
     const int64_t n1 = (seq + 127) / 128, n2 = (seq + 255) / 256;
-    if (bh * n2 >= 8 * (int64_t)n_sm) return false;  // many items: the lower total wins, and no loop over long heads
-    const double key1 = dim == 128 ? 1.0 : 0.84, item1 = dim == 128 ? 4.8 : 4.2;  // 128-row items
-    const double key2 = dim == 128 ? 2.0 : 1.7, key2_one = 1.1, item2 = 3.0, first2 = 2.5;  // 256-row items
+    if (bh * n2 >= 8 * (int64_t)n_sm) return 0;  // many items: the lower total wins, and no loop over long heads
+    const double key1 = dim == 128 ? 1.0 : 0.84, item1 = dim == 128 ? 4.8 : 4.2, merge = 4.0;  // 128-row items
+    const double key2 = dim == 128 ? 2.0 : 1.7, key2_one = 1.1, item2 = 3.0, first2 = 2.5;     // 256-row items
     const int64_t all = (seq_kv + 127) / 128, off = (causal && offsets && seq_kv > seq) ? seq_kv - seq : 0;
     auto tiles = [&](int64_t row_end) { return causal ? std::min(all, (off + std::min(row_end, seq) + 127) / 128) : all; };
-    double sum1 = 0, max1 = 0, sum2 = 0, max2 = 0;
-    for (int64_t i = 0; i < n1; ++i) {
-        const double c = (double)tiles((i + 1) * 128) * key1 + item1;
-        sum1 += c;
-        max1 = std::max(max1, c);
-    }
+    // equal CTAs come in whole waves; a causal list is dealt out to within about 8 %
+    auto span = [&](double sum, double mx, int64_t n, int slots) {
+        return causal ? std::max(mx, 1.08 * sum * (double)bh / slots) : mx * (double)((bh * n + slots - 1) / slots);
+    };
+    double sum = 0, mx = 0;
     for (int64_t i = 0; i < n2; ++i) {
         const double c = (double)tiles((i + 1) * 256) * (i * 256 + 128 >= seq ? key2_one : key2) + item2;
-        sum2 += c;
-        max2 = std::max(max2, c);
+        sum += c;
+        mx = std::max(mx, c);
     }
-    // equal items come in whole waves; a causal list is dealt out to within about 8 %
-    auto span = [&](double sum, double mx, int64_t n) {
-        return causal ? std::max(mx, 1.08 * sum * (double)bh / n_sm) : mx * (double)((bh * n + n_sm - 1) / n_sm);
-    };
-    return span(sum1, max1, n1) < span(sum2, max2, n2) + first2;
+    double best = span(sum, mx, n2, n_sm) + first2;
+    int kind = 0;
+    for (int split = 1; split <= (may_split ? 8 : 1); split *= 2) {
+        sum = mx = 0;
+        for (int64_t i = 0; i < n1; ++i) {
+            const double c = (double)((tiles((i + 1) * 128) + split - 1) / split) * key1 + item1 + (split > 1 ? merge : 0);
+            sum += c * split;
+            mx = std::max(mx, c);
+        }
+        // a second wave of clusters starts only when whole clusters end (10 us and more a wave)
+        if (split > 1 && (bh * n1 * split > n_sm || bh * n1 * split > cluster_slots(split))) break;
+        const double t = span(sum, mx, n1 * split, n_sm);
+        if (t < best) {
+            best = t;
+            kind = split;
+        }
+    }
+    return kind;
 }
 
 cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void* out, float* lse, int64_t batch,
@@ -1210,7 +1369,9 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
         const char* s = getenv("RT_ATTN_PREFILL_SCHED");
         return (s && !strcmp(s, "persistent")) ? 1 : (s && !strcmp(s, "percta")) ? 2 : 0;
     }();
-    p.single_tile = prefer_single_tile(bh, seq, seq_kv, dim, causal, q_offsets != nullptr, n_sm) ? 1 : 0;
+    const int kind = choose_items(bh, seq, seq_kv, dim, causal, q_offsets != nullptr, key_keep == nullptr && env_tiles == 0, n_sm);
+    p.single_tile = kind > 0 ? 1 : 0;
+    p.split = kind > 1 ? kind : 1;
     static const int env_stagger = [] {
         const char* s = getenv("RT_ATTN_PREFILL_STAGGER");
         return s ? atoi(s) : 900;
@@ -1242,7 +1403,7 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
     p.units = (int)bh;
     p.rounds = p.tail_head = p.tail_skip = 0;
     p.n_tail = (int)n_items;
-    p.by_level = n_items > n_sm ? 1 : 0;
+    p.by_level = n_items * p.split > n_sm ? 1 : 0;
     if (causal && n_ctas < n_items && !p.sorted) {
         const int64_t per_head = (n_qb + 1) / 2, all = bh * per_head / n_ctas;
         const int64_t kv_bytes = batch * heads_kv * seq_kv * dim * 4;

@@ -157,3 +157,34 @@ def test_keep_flags_sorted(B, H, N, Nkv, D, causal):
         x, y = out[b].float()[~dead], ref[~dead]
         assert float((x - y).norm()) <= 1e-2 * float(y.norm())
         assert torch.allclose(lse[b][~dead], torch.logsumexp(s, -1)[~dead], rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nkv,D,causal,lens", [
+    (1, 4, 2, 100, 9000, 64, True, (9000,)),          # 8 CTAs an item
+    (2, 16, 2, 123, 8400, 128, True, (2100, 8400)),   # 4, one sequence much shorter
+    (1, 33, 33, 1, 3000, 128, False, (2999,)),        # 4, as many clusters as fit
+    (1, 74, 37, 128, 4097, 64, False, (4097,)),       # 2
+    (3, 8, 8, 200, 5000, 128, False, (0, 1, 5000)),   # shares without a key, and a sequence without one
+    (5, 4, 2, 70, 3000, 64, True, (70, 128, 129, 1500, 3000)),
+])
+def test_prefill_clusters(B, Hq, Hkv, Nq, Nkv, D, causal, lens):
+    """Items whose keys a cluster of CTAs shares."""
+    import torch
+    import rustorch_b200 as rt
+    torch.manual_seed(6)
+    q = torch.randn(B, Hq, Nq, D, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(B, Hkv, Nkv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    n = torch.tensor(lens, device="cuda", dtype=torch.int32)
+    off = torch.tensor([max(0, x - Nq) for x in lens], device="cuda", dtype=torch.int32)
+    out, lse = rt.prefill_bf16(q, k, v, causal=causal, kv_lens=n, q_offsets=off if causal else None)
+    for b in range(B):
+        if lens[b] == 0:
+            assert bool(torch.isnan(out[b]).all()) and bool((lse[b] == float("-inf")).all())
+            continue
+        kb, vb = (x[b, :, :lens[b]].float().repeat_interleave(Hq // Hkv, 0) for x in (k, v))
+        s = q[b].float() @ kb.transpose(1, 2) / D ** 0.5
+        if causal:
+            s = s.masked_fill(torch.ones(Nq, lens[b], dtype=torch.bool, device="cuda").triu(int(off[b]) + 1), float("-inf"))
+        ref = torch.softmax(s, -1) @ vb
+        assert float((out[b].float() - ref).norm() / ref.norm()) < 1e-2
+        assert torch.allclose(lse[b], torch.logsumexp(s, -1), rtol=1e-4, atol=1e-3)
