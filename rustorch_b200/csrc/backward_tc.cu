@@ -87,6 +87,8 @@ template <int D>
 __global__ void __launch_bounds__(256) bwd_delta_bf16_kernel(const __nv_bfloat16* __restrict__ out,
                                                              const __nv_bfloat16* __restrict__ d_out,
                                                              float* __restrict__ delta, int64_t rows) {
+    // The backward kernel's CTAs may start their set-up as soon as all of this grid's are running.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr int LPR = D / 8;        // lanes per row
     constexpr int RPW = 32 / LPR;     // rows per warp and pass
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

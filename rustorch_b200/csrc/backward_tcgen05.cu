@@ -4,7 +4,8 @@
 // 96-189) with the saved row statistics in place of the N x N probability matrix:
 //   P = exp(scale * Q K^T - LSE),  dP = dO V^T,  dS = P o (dP - delta),  delta_i = dO_i . O_i,
 //   dV = P^T dO,  dQ = scale * dS K,  dK = scale * dS^T Q.
-// Two deterministic passes (no atomics, fixed summation order) share one kernel template.  A CTA owns
+// Two deterministic passes (no atomics, fixed summation order) run in one launch, each on its own CTAs, one per SM, which
+// work through a list of tiles (tile_schedule.cuh).  For each tile a CTA takes
 // 128 rows of one side, keeps them in shared memory, and walks the other side in 64-row steps that TMA
 // streams through a four-slot ring:
 //   query side: own X1 = Q_i, X2 = dO_i;  per key tile (Y1 = K_j, Y2 = V_j)
@@ -23,7 +24,12 @@
 // MMAs of step u+2 occupy the tensor pipe (the forward kernel pipelines S and P the same way).
 // TMEM (512 columns): buffer b of step u (b = u & 1) holds T1 at [128 b, 128 b + 64) and T2 at
 // [128 b + 64, 128 b + 128); accumulators from 256 (dQ, or dV then dK), D columns each; P^T / dS (bf16)
-// overwrite 32 of the columns of T1 / T2.  320 threads: warps 0-7 element-wise work and the final read-out,
+// overwrite 32 of the columns of T1 / T2.
+// From one tile to the next the pipeline does not drain: the next own rows load once the last score MMAs have read the
+// present ones, and the next tile's first score MMAs run while the accumulators are read out (through shared memory
+// and TMA stores).  One CTA per tile, with its set-up, first loads and read-out exposed each time, took 651 us on
+// B=4 H=32 N=2048 D=128 causal (498 now), 45 on B=1 H=32 N=658 D=64 (24), 46 on B=4 H=8 N=625 D=128 (25).
+//  320 threads: warps 0-7 element-wise work and the final read-out,
 // two threads per own row (warp w owns rows 32 (w % 4).. and the 32 score columns of half w / 4; its bf16
 // results go back into the first 16 of its OWN columns, so the two threads of a row never touch each other's
 // inputs, and the accumulating MMAs take K elements 0-31 from columns [0,16) and 32-63 from [32,48));
@@ -31,10 +37,12 @@
 // Every mbarrier wait is bounded; on expiry the kernel records a code in the device status word and
 // leaves through the common teardown.
 #include <cuda.h>
+#include <algorithm>
 #include <cstdlib>
 
 #include "kernels.h"
 #include "tc_ptx.cuh"
+#include "tile_schedule.cuh"
 
 namespace rt {
 
@@ -45,7 +53,12 @@ bool make_tensor_map_bf16_4d(CUtensorMap* map, const void* base, int64_t batch, 
 
 namespace {
 
-enum { kToBwdX = 201, kToBwdYFull, kToBwdYEmpty, kToBwdT, kToBwdA, kToBwdAcc, kToBwdDrain, kToBwdStat };
+enum { kToBwdX = 201, kToBwdYFull, kToBwdYEmpty, kToBwdT, kToBwdA, kToBwdAcc, kToBwdDrain, kToBwdStat, kToBwdXEmpty, kToBwdAlign };
+
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Q, K, V and dO up to this size are taken to stay in L2 (126 MB) with their gradients passing through.
+constexpr int64_t kLevelsBytes = 96ll << 20;
 
 template <int D>
 struct BwdCfg {
@@ -55,76 +68,94 @@ struct BwdCfg {
     static constexpr int HALF_BYTES = 64 * D * 2;   // 64 other-side rows: NSUB sub-tiles of 64 rows x 128 bytes
     static constexpr int HSUB_BYTES = 64 * 64 * 2;
     static constexpr int STAGES = 4;                // ring slots, each (Y1 | Y2) of one 64-row step
-    static constexpr int NBARS = 1 + 2 * STAGES + 6;
+    static constexpr int STAGE_OUT = 8 * 32 * 128;  // per element-wise warp: 32 rows x 32 f32 columns on their way out
+    static constexpr int NBARS = 2 + 2 * STAGES + 6;
     static constexpr int STAT_BYTES = 2 * 2 * 128 * 4;  // two slots of LSE * log2(e) and delta of a 128-row other tile
-    static constexpr int SMEM_BYTES = 2 * TILE_BYTES + STAGES * 2 * HALF_BYTES + STAT_BYTES + NBARS * 8 + 16 + 1024;
+    static constexpr int SMEM_BYTES = 2 * TILE_BYTES + STAGES * 2 * HALF_BYTES + STAGE_OUT + STAT_BYTES + NBARS * 8 + 16;
     static constexpr uint32_t COL_T = 0, COL_ACC = 256;  // T1 of buffer b at COL_T + 128 b, T2 64 columns further
+    static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB of shared memory a CTA can opt into");
 };
 
 struct Bwd5Params {
     const float* lse;    // [B*H, N]
     const float* delta;  // [B*H, N]
-    float* out1;         // query side: dQ; key side: dV   ([B*H, N, D] f32)
-    float* out2;         // key side: dK
     int seq, heads;
     int causal;
     float scale, scale_log2;
     int* status;
-    int head_group;      // heads per group of the CTA order
+    int q_ctas;          // CTAs of the query side; the rest of the grid is the key side's
+    LevelSchedule list[2];  // the query side's and the key side's 128-row tiles
+};
+
+// One 128-row tile of a CTA's own side.
+struct BwdItem {
+    int bh, b, h;
+    int own0;     // first own row
+    int s_lo;     // first other-side 64-row step (even)
+    int n_u;      // steps
 };
 
 template <int D, bool kKeySide>
-__global__ void __launch_bounds__(320, 1)
-bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
-                   const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
-                   const Bwd5Params p) {
+__device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtensorMap* tm_x2, const CUtensorMap* tm_y1,
+                                         const CUtensorMap* tm_y2, const CUtensorMap* tm_o1, const CUtensorMap* tm_o2,
+                                         const Bwd5Params& p, uint8_t* smem, int warp, int lane, int cta, int n_ctas) {
     using C = BwdCfg<D>;
     constexpr int TILE = C::TILE_BYTES, SUB = C::SUB_BYTES, STAGES = C::STAGES, HALFT = C::HALF_BYTES, HSUB = C::HSUB_BYTES;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sX1 = smem;
     uint8_t* sX2 = sX1 + TILE;
     uint8_t* sY = sX2 + TILE;  // [STAGES][Y1 | Y2], 64 rows each
-    float* stat = reinterpret_cast<float*>(sY + STAGES * 2 * HALFT);  // [2][lse2[128] | delta[128]]
+    uint8_t* sOut = sY + STAGES * 2 * HALFT;
+    float* stat = reinterpret_cast<float*>(sOut + C::STAGE_OUT);  // [2][lse2[128] | delta[128]]
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(stat) + C::STAT_BYTES);
-    uint64_t* x_full = bars;                // [1]
-    uint64_t* y_full = x_full + 1;          // [STAGES]
+    uint64_t* x_full = bars;                // [1] one phase per item
+    uint64_t* x_empty = x_full + 1;         // [1] one phase per item: its last score MMAs have retired
+    uint64_t* y_full = x_empty + 1;         // [STAGES]
     uint64_t* y_empty = y_full + STAGES;    // [STAGES]
     uint64_t* t_full = y_empty + STAGES;    // [2] per buffer, one phase per use: T1, T2 are in TMEM
     uint64_t* a_full = t_full + 2;          // [2] per buffer, one phase per use: the bf16 A operands are in TMEM
-    uint64_t* acc_done = a_full + 2;        // [1] the last accumulating MMA has retired
-    uint64_t* stat_bar = acc_done + 1;      // [1] one phase per step: the column statistics are in shared memory
+    uint64_t* acc_done = a_full + 2;        // [1] one phase per item: its last accumulating MMA has retired
+    uint64_t* stat_bar = acc_done + 1;      // [1] one phase per other tile: the column statistics are in shared memory
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stat_bar + 1);
 
-    const int warp = __shfl_sync(kFullMask, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int N = p.seq;
-    const int n_tiles = (N + 127) / 128;
-    // heaviest tiles first: under a causal mask the query side's last tiles and the key side's first tiles
-    // walk the most other-side tiles
-    // CTA order: heads in groups of p.head_group (RT_ATTN_BACKWARD_HEAD_GROUP, default 4); inside a group tile rank r (0 = heaviest) of every head comes
-    // before rank r + 1.  A group's Q, K, V, dO (a few MB per head) stay in L2 while its CTAs run, and the grid's
-    // last wave holds the group's lightest tiles instead of a head's heaviest.
-    const int kHeadGroup = p.head_group;
-    const int n_bh = (int)gridDim.x / n_tiles;
-    const int grp = (int)blockIdx.x / (kHeadGroup * n_tiles);
-    const int rem = (int)blockIdx.x - grp * kHeadGroup * n_tiles;
-    const int in_grp = min(kHeadGroup, n_bh - grp * kHeadGroup);
-    const int rank = rem / in_grp;
-    const int own = kKeySide ? rank : (p.causal ? n_tiles - 1 - rank : rank);
-    const int bh = grp * kHeadGroup + rem % in_grp, b = bh / p.heads, h = bh % p.heads;
-    const int own0 = own * 128;
-    // other-side tiles [t_lo, t_hi)
-    const int t_lo = (kKeySide && p.causal) ? own : 0;
-    const int t_hi = (!kKeySide && p.causal) ? own + 1 : n_tiles;
-    const int n_steps = t_hi - t_lo;  // other-side tiles; each is two 64-row steps
-    const int n_u = 2 * n_steps;
+    const LevelSchedule& list = p.list[kKeySide ? 1 : 0];
+    // Entry j of the CTA's list and on to the next that holds a tile (all roles walk the same list).  Heaviest first:
+    // under a causal mask the query side's last tiles and the key side's first tiles walk the most steps.
+    auto fetch = [&](int& j, BwdItem& it) {
+        for (;;) {
+            bool end = false, valid;
+            int rank = 0;
+            if (p.causal) {
+                valid = level_item(list, j, cta, n_ctas, it.bh, rank, end);
+            } else {
+                const int pos = j * n_ctas + cta;
+                end = pos >= list.units * list.n;
+                valid = !end;
+                it.bh = pos / list.n;
+                rank = pos % list.n;
+            }
+            ++j;
+            if (end) return false;
+            if (!valid) continue;
+            const int own = (kKeySide || !p.causal) ? rank : list.n - 1 - rank;
+            it.b = it.bh / p.heads;
+            it.h = it.bh % p.heads;
+            it.own0 = own * 128;
+            const int all = (N + 63) / 64;
+            it.s_lo = (kKeySide && p.causal) ? 2 * own : 0;
+            it.n_u = ((!kKeySide && p.causal) ? min(all, 2 * own + 2) : all) - it.s_lo;
+            return true;
+        }
+    };
 
     if (warp == 8 && lane == 0) {
-        prefetch_tensormap(&tm_x1);
-        prefetch_tensormap(&tm_x2);
-        prefetch_tensormap(&tm_y1);
-        prefetch_tensormap(&tm_y2);
+        prefetch_tensormap(tm_x1);
+        prefetch_tensormap(tm_x2);
+        prefetch_tensormap(tm_y1);
+        prefetch_tensormap(tm_y2);
+        prefetch_tensormap(tm_o1);
         mbar_init(x_full, 1);
+        mbar_init(x_empty, 1);
         for (int i = 0; i < STAGES; ++i) {
             mbar_init(&y_full[i], 1);
             mbar_init(&y_empty[i], 1);
@@ -146,33 +177,44 @@ bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_dep_wait();  // delta is the previous kernel's output; the set-up above overlaps that kernel
 
     if (warp == 8) {
         // ============================================================== TMA producer
         if (lane == 0) {
-            mbar_arrive_expect_tx(x_full, 2 * TILE);
+            int g = 0, k = 0;  // steps requested so far (ring position and phase), items begun
+            bool ok = true;
+            BwdItem it;
+            for (int j = 0; ok && fetch(j, it); ++k) {
+                if (k > 0 && !mbar_wait(x_empty, (uint32_t)(k - 1) & 1u, p.status, kToBwdXEmpty)) break;
+                mbar_arrive_expect_tx(x_full, 2 * TILE);
 #pragma unroll
-            for (int s = 0; s < C::NSUB; ++s) {
-                tma_load_4d(sX1 + s * SUB, &tm_x1, x_full, s * 64, own0, h, b);
-                tma_load_4d(sX2 + s * SUB, &tm_x2, x_full, s * 64, own0, h, b);
-            }
-            int issued = 0;
-            for (int u = 0; u < n_u; ++u) {
-                const int st = u % STAGES;
-                if (u >= STAGES && !mbar_wait(&y_empty[st], (uint32_t)(u / STAGES - 1) & 1u, p.status, kToBwdYEmpty)) break;
-                mbar_arrive_expect_tx(&y_full[st], 2 * HALFT);
-                uint8_t* dst = sY + st * 2 * HALFT;
-                const int r0 = (t_lo + (u >> 1)) * 128 + (u & 1) * 64;
+                for (int s = 0; s < C::NSUB; ++s)
 #pragma unroll
-                for (int s = 0; s < C::NSUB; ++s) {
-                    tma_load_4d(dst + s * HSUB, &tm_y1, &y_full[st], s * 64, r0, h, b);
-                    tma_load_4d(dst + HALFT + s * HSUB, &tm_y2, &y_full[st], s * 64, r0, h, b);
+                    for (int r = 0; r < 2; ++r) {
+                        tma_load_4d(sX1 + s * SUB + r * HSUB, tm_x1, x_full, s * 64, it.own0 + r * 64, it.h, it.b);
+                        tma_load_4d(sX2 + s * SUB + r * HSUB, tm_x2, x_full, s * 64, it.own0 + r * 64, it.h, it.b);
+                    }
+                for (int u = 0; u < it.n_u; ++u) {
+                    const int st = g % STAGES;
+                    if (g >= STAGES && !mbar_wait(&y_empty[st], (uint32_t)(g / STAGES - 1) & 1u, p.status, kToBwdYEmpty)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_arrive_expect_tx(&y_full[st], 2 * HALFT);
+                    uint8_t* dst = sY + st * 2 * HALFT;
+                    const int r0 = (it.s_lo + u) * 64;
+#pragma unroll
+                    for (int s = 0; s < C::NSUB; ++s) {
+                        tma_load_4d(dst + s * HSUB, tm_y1, &y_full[st], s * 64, r0, it.h, it.b);
+                        tma_load_4d(dst + HALFT + s * HSUB, tm_y2, &y_full[st], s * 64, r0, it.h, it.b);
+                    }
+                    ++g;
                 }
-                issued = u + 1;
             }
             // Drain: every copy this thread issued must have landed before the CTA may exit.
-            mbar_wait(x_full, 0, p.status, kToBwdDrain);
-            for (int u = max(0, issued - STAGES); u < issued; ++u)
+            if (k > 0) mbar_wait(x_full, (uint32_t)(k - 1) & 1u, p.status, kToBwdDrain);
+            for (int u = max(0, g - STAGES); u < g; ++u)
                 mbar_wait(&y_full[u % STAGES], (uint32_t)(u / STAGES) & 1u, p.status, kToBwdDrain);
         }
     } else if (warp == 9) {
@@ -191,8 +233,8 @@ bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
         auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
             return __all_sync(kFullMask, mbar_wait(bar, parity, p.status, code));
         };
-        // T1 = X1 Y1^T, T2 = X2 Y2^T over the 64 other-side rows of step u, into buffer u & 1 (they overwrite
-        // the A operands of step u - 2: the pipe runs this thread's MMAs in issue order, after the accumulating
+        // T1 = X1 Y1^T, T2 = X2 Y2^T over the 64 other-side rows of step u (counted over all items), into buffer u & 1
+        // (they overwrite the A operands of step u - 2: the pipe runs this thread's MMAs in issue order, after the accumulating
         // MMAs of that step)
         auto issue_T = [&](int u) {
             const int st = u % STAGES;
@@ -211,102 +253,126 @@ bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
                 if (leader) mma_ss(t2, dx2 + offx, y2 + offy, idesc_t, kk > 0);
             }
         };
-        bool ok = wait(x_full, 0, kToBwdX);
         auto wait_rows = [&](int u) {  // the rows of step u have landed
             const bool got = wait(&y_full[u % STAGES], (uint32_t)(u / STAGES) & 1u, kToBwdYFull);
             tc_fence_after();
             return got;
         };
-        if (ok && n_u > 0) {
-            ok = wait_rows(0);
-            if (ok) {
-                issue_T(0);
-                commit(&t_full[0]);
-                ok = wait_rows(1);
+        int g = 0;  // the item's first step
+        bool ok = true;
+        BwdItem it;
+        for (int j = 0, k = 0; ok && fetch(j, it); ++k) {
+            // The item's first score MMAs follow the previous item's last accumulating ones and run while the element-wise
+            // warps read those accumulators out; their next results, which the first accumulating MMAs here
+            // wait for, come after that.
+            const int n_u = it.n_u;
+            ok = wait(x_full, (uint32_t)k & 1u, kToBwdX);
+            for (int u = 0; u < min(2, n_u) && ok; ++u) {
+                ok = wait_rows(g + u);
+                if (!ok) break;
+                issue_T(g + u);
+                commit(&t_full[(g + u) & 1]);
+                if (u == n_u - 1) commit(x_empty);
             }
-            if (ok) {
-                issue_T(1);
-                commit(&t_full[1]);
+            for (int u = 0; u < n_u && ok; ++u) {
+                const int gu = g + u, st = gu % STAGES;
+                if (!wait(&a_full[gu & 1], (uint32_t)(gu >> 1) & 1u, kToBwdA)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint64_t y1 = dy_mn + (uint64_t)((st * 2 * HALFT) >> 4), y2 = y1 + (uint64_t)(HALFT >> 4);
+                const uint32_t t1 = tT + (gu & 1) * 128, t2 = t1 + 64;
+                const uint32_t acc0 = u > 0 ? 1u : 0u;
+                if (kKeySide) {
+                    // dV += P^T dO (A = P^T in the first 32 columns of T1, B = Y2 = dO), dK += dS^T Q (A in T2, B = Y1 = Q)
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        if (leader)
+                            mma_ts(tAcc, t1 + kk * 8 + (kk >= 2 ? 16 : 0), y2 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        if (leader)
+                            mma_ts(tAcc + D, t2 + kk * 8 + (kk >= 2 ? 16 : 0), y1 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
+                } else {
+                    // dQ += dS K (A = dS in the first 32 columns of T2, B = Y1 = K)
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        if (leader)
+                            mma_ts(tAcc, t2 + kk * 8 + (kk >= 2 ? 16 : 0), y1 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
+                }
+                commit(&y_empty[st]);  // the step's rows are free once these MMAs (and the score MMAs before them) retire
+                if (u == n_u - 1) commit(acc_done);
+                if (u + 2 < n_u) {
+                    if (!wait_rows(gu + 2)) {
+                        ok = false;
+                        break;
+                    }
+                    issue_T(gu + 2);
+                    commit(&t_full[gu & 1]);
+                    if (u + 2 == n_u - 1) commit(x_empty);
+                }
             }
+            g += n_u;
         }
-        for (int u = 0; u < n_u && ok; ++u) {
-            const int st = u % STAGES;
-            if (!wait(&a_full[u & 1], (uint32_t)(u >> 1) & 1u, kToBwdA)) break;
-            tc_fence_after();
-            const uint64_t y1 = dy_mn + (uint64_t)((st * 2 * HALFT) >> 4), y2 = y1 + (uint64_t)(HALFT >> 4);
-            const uint32_t t1 = tT + (u & 1) * 128, t2 = t1 + 64;
-            const uint32_t acc0 = u > 0 ? 1u : 0u;
-            if (kKeySide) {
-                // dV += P^T dO (A = P^T in the first 32 columns of T1, B = Y2 = dO), dK += dS^T Q (A in T2, B = Y1 = Q)
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    if (leader)
-                        mma_ts(tAcc, t1 + kk * 8 + (kk >= 2 ? 16 : 0), y2 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    if (leader)
-                        mma_ts(tAcc + D, t2 + kk * 8 + (kk >= 2 ? 16 : 0), y1 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
-            } else {
-                // dQ += dS K (A = dS in the first 32 columns of T2, B = Y1 = K)
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    if (leader)
-                        mma_ts(tAcc, t2 + kk * 8 + (kk >= 2 ? 16 : 0), y1 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
-            }
-            commit(&y_empty[st]);  // the step's rows are free once these MMAs (and the score MMAs before them) retire
-            if (u + 2 < n_u) {
-                if (!wait_rows(u + 2)) break;
-                issue_T(u + 2);
-                commit(&t_full[u & 1]);
-            }
-            if (u == n_u - 1) commit(acc_done);
-        }
-        if (n_u == 0) commit(acc_done);
     } else {
         // ============================================================== element-wise warps (two threads per own row)
         const int half = warp >> 2;  // which 32 of a step's 64 score columns
         const int r = (warp & 3) * 32 + lane;
-        const int own_row = own0 + r;
         const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
         const uint32_t tT = tmem_base + lane_sel + C::COL_T;
         const uint32_t tAcc = tmem_base + lane_sel + C::COL_ACC;
+        uint8_t* const stage = sOut + warp * 4096;
         const float c = p.scale_log2;
-        const int64_t stat_base = (int64_t)bh * N;
+        // LSE (as log2; +inf, which makes every probability 0, for absent queries and rows without a visible key) and
+        // delta of one query.  Requested a tile (key side) or an item (query side) ahead.
+        float raw_lse = 0.f, raw_delta = 0.f;
+        auto request = [&](const BwdItem& it, int qi) {
+            raw_lse = qi < N ? __ldg(p.lse + (int64_t)it.bh * N + qi) : INFINITY;
+            raw_delta = qi < N ? __ldg(p.delta + (int64_t)it.bh * N + qi) : 0.f;
+        };
+        auto lse2 = [&] { return (raw_lse > -INFINITY && raw_lse < INFINITY) ? raw_lse * kLog2e : INFINITY; };
+        int j = 0, g = 0, gt = 0;  // list entry, first step of the item, other tiles so far (key side)
+        BwdItem it, nx;
+        bool ok = true, more = fetch(j, it);
+        if (more) request(it, kKeySide ? it.s_lo * 64 + r : it.own0 + r);
+        for (int k = 0; more && ok; ++k, it = nx) {
+        more = fetch(j, nx);
+        const int own_row = it.own0 + r, n_u = it.n_u;
         float my_lse2 = 0.f, my_delta = 0.f;  // query side: this row's statistics
-        if (!kKeySide && own_row < N) {
-            const float x = p.lse[stat_base + own_row];
-            my_lse2 = (x > -INFINITY && x < INFINITY) ? x * kLog2e : INFINITY;  // no visible key (or NaN): P = 0
-            my_delta = p.delta[stat_base + own_row];
+        if (!kKeySide) {
+            my_lse2 = lse2();
+            my_delta = raw_delta;
+            if (more) request(nx, nx.own0 + r);
         }
-        bool ok = true;
         for (int u = 0; u < n_u && ok; ++u) {
-            const int t = u >> 1, st = t & 1, buf = u & 1;
-            const int other0 = (t_lo + t) * 128 + buf * 64;  // first other-side row of this step
-            float* s_lse2 = stat + st * 256;
+            const int step = it.s_lo + u, buf = (g + u) & 1, sub = step & 1;
+            const int other0 = step * 64;  // first other-side row of this step
+            float* s_lse2 = stat + (gt & 1) * 256;
             float* s_delta = s_lse2 + 128;
-            if (kKeySide && buf == 0) {
+            if (kKeySide && sub == 0) {
                 // the statistics of this tile's 128 queries (columns); the slot was last read two tiles ago, and
                 // every thread has passed the a_full arrivals of that tile's successor by now
                 if (half == 0) {
-                    const int qi = other0 + r;
-                    const float x = qi < N ? p.lse[stat_base + qi] : INFINITY;
-                    s_lse2[r] = (x > -INFINITY && x < INFINITY) ? x * kLog2e : INFINITY;  // +inf -> P = 0
-                    s_delta[r] = qi < N ? p.delta[stat_base + qi] : 0.f;
+                    s_lse2[r] = lse2();
+                    s_delta[r] = raw_delta;
+                    if (u + 2 < n_u) request(it, other0 + 128 + r);
+                    else if (more) request(nx, nx.s_lo * 64 + r);
                 }
                 mbar_arrive(stat_bar);  // an mbarrier rather than bar.sync, so that this wait is bounded as well
-                if (!__all_sync(kFullMask, mbar_wait(stat_bar, (uint32_t)t & 1u, p.status, kToBwdStat))) {
+                if (!__all_sync(kFullMask, mbar_wait(stat_bar, (uint32_t)gt & 1u, p.status, kToBwdStat))) {
                     ok = false;
                     break;
                 }
             }
-            if (!__all_sync(kFullMask, mbar_wait(&t_full[buf], (uint32_t)(u >> 1) & 1u, p.status, kToBwdT))) {
+            if (!__all_sync(kFullMask, mbar_wait(&t_full[buf], (uint32_t)((g + u) >> 1) & 1u, p.status, kToBwdT))) {
                 ok = false;
                 break;
             }
             tc_fence_after();
             // Is any (own row, other index) pair of this step masked?  Only the diagonal tile of a causal
             // launch and the last tile of a ragged sequence are.
-            const bool diag = p.causal && (t_lo + t) == own;
+            const bool diag = p.causal && (step >> 1) == (it.own0 >> 7);
             const bool ragged = other0 + 64 > N;
             const uint32_t t1 = tT + buf * 128, t2 = t1 + 64;
             const float2 c2 = make_float2(c, c);
@@ -324,8 +390,8 @@ bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
                     // on the key side (an LSE of +inf makes the probability 0: absent queries, rows without a key)
                     float4 l4, d4;
                     if (kKeySide) {
-                        l4 = *reinterpret_cast<const float4*>(s_lse2 + buf * 64 + cbase + i);
-                        d4 = *reinterpret_cast<const float4*>(s_delta + buf * 64 + cbase + i);
+                        l4 = *reinterpret_cast<const float4*>(s_lse2 + sub * 64 + cbase + i);
+                        d4 = *reinterpret_cast<const float4*>(s_delta + sub * 64 + cbase + i);
                     } else {
                         l4 = make_float4(my_lse2, my_lse2, my_lse2, my_lse2);
                         d4 = make_float4(my_delta, my_delta, my_delta, my_delta);
@@ -364,31 +430,45 @@ bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
             tc_wait_st();
             tc_fence_before();
             mbar_arrive(&a_full[buf]);
+            if (kKeySide && (sub == 1 || u == n_u - 1)) ++gt;
         }
-        // ---- read-out: accumulators -> f32 global (scale folded into dQ and dK)
-        if (ok && __all_sync(kFullMask, mbar_wait(acc_done, 0, p.status, kToBwdAcc))) {
+        g += n_u;
+        // ---- read-out: accumulators -> f32 (scale folded into dQ and dK) -> 32 rows x 32 columns of this warp in shared
+        // memory, swizzled as the tensor map has it -> one TMA store, which clips the rows past N.  (Stored straight
+        // from registers, 16 bytes of 32 rows per instruction, the tile took 8192 store cycles.)
+        ok = ok && __all_sync(kFullMask, mbar_wait(acc_done, (uint32_t)k & 1u, p.status, kToBwdAcc));
+        if (ok) {
             tc_fence_after();
             constexpr int kOuts = kKeySide ? 2 : 1;
             constexpr int OC = D / 2;  // accumulator columns per thread
+            const int row0 = it.own0 + (warp & 3) * 32;
 #pragma unroll
             for (int o = 0; o < kOuts; ++o) {
-                float* dst = (o == 0 ? p.out1 : p.out2) + ((int64_t)bh * N + own_row) * D + half * OC;
                 const float mul = (kKeySide && o == 0) ? 1.f : p.scale;  // dV is not scaled
 #pragma unroll
                 for (int ch = 0; ch < OC / 32; ++ch) {
                     uint32_t a[32];
                     tmem_ld32(tAcc + o * D + half * OC + ch * 32, a);
                     tc_wait_ld();
-                    if (own_row < N) {
+                    if (lane == 0) tma_store_wait_read();  // the warp's previous store has read the staging rows
+                    __syncwarp();
 #pragma unroll
-                        for (int i = 0; i < 32; i += 4)
-                            *reinterpret_cast<float4*>(dst + ch * 32 + i) =
-                                make_float4(__uint_as_float(a[i]) * mul, __uint_as_float(a[i + 1]) * mul,
-                                            __uint_as_float(a[i + 2]) * mul, __uint_as_float(a[i + 3]) * mul);
+                    for (int i = 0; i < 32; i += 4)
+                        *reinterpret_cast<float4*>(stage + lane * 128 + (((i >> 2) ^ (lane & 7)) << 4)) =
+                            make_float4(__uint_as_float(a[i]) * mul, __uint_as_float(a[i + 1]) * mul,
+                                        __uint_as_float(a[i + 2]) * mul, __uint_as_float(a[i + 3]) * mul);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0 && row0 < N) {
+                        // the map counts in 2-byte elements
+                        tma_store_4d(o == 0 ? tm_o1 : tm_o2, stage, (half * OC + ch * 32) * 2, row0, it.h, it.b);
+                        tma_store_commit();
                     }
                 }
             }
         }
+        }
+        if (lane == 0) tma_store_wait_read();  // shared memory stays until the last store has read it
     }
 
     tc_fence_before();
@@ -399,16 +479,55 @@ bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     }
 }
 
-template <int D, bool kKeySide>
-cudaError_t launch_side(const CUtensorMap& x1, const CUtensorMap& x2, const CUtensorMap& y1, const CUtensorMap& y2,
-                        const Bwd5Params& p, int64_t bh, cudaStream_t stream) {
-    cudaError_t e = set_max_dynamic_smem_once<bwd_tcgen05_kernel<D, kKeySide>>(BwdCfg<D>::SMEM_BYTES);
+// CTAs [0, q_ctas) work through the query side's tiles, the others through the key side's.
+template <int D>
+__global__ void __launch_bounds__(320, 1)
+bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                   const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dk,
+                   const __grid_constant__ CUtensorMap tm_dv, const Bwd5Params p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const int warp = __shfl_sync(kFullMask, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    if (smem_u32(smem) & 1023u) {  // the swizzled tiles need it; all 227 KB are in use, so none is spent on rounding up
+        if (threadIdx.x == 0) atomicCAS(p.status, 0, (int)kToBwdAlign);
+        return;
+    }
+    const int cta = (int)blockIdx.x, nq = p.q_ctas;
+    if (cta < nq) bwd_side<D, false>(&tm_q, &tm_do, &tm_k, &tm_v, &tm_dq, &tm_dq, p, smem, warp, lane, cta, nq);
+    else bwd_side<D, true>(&tm_k, &tm_v, &tm_q, &tm_do, &tm_dv, &tm_dk, p, smem, warp, lane, cta - nq, (int)gridDim.x - nq);
+}
+
+template <int D>
+cudaError_t launch_sides(const CUtensorMap (&m)[7], Bwd5Params p, int64_t bh, cudaStream_t stream) {
+    cudaError_t e = set_max_dynamic_smem_once<bwd_tcgen05_kernel<D>>(BwdCfg<D>::SMEM_BYTES);
     if (e != cudaSuccess) return e;
-    const int64_t n_ctas = ((p.seq + 127) / 128) * bh;
-    if (n_ctas > 0x7fffffff) return cudaErrorInvalidValue;
-    dim3 grid((unsigned)n_ctas);
-    bwd_tcgen05_kernel<D, kKeySide><<<grid, 320, BwdCfg<D>::SMEM_BYTES, stream>>>(x1, x2, y1, y2, p);
-    return cudaGetLastError();
+    const int64_t n_tiles = (p.seq + 127) / 128, n_items = n_tiles * bh;
+    if (n_items > 0x3fffffff) return cudaErrorNotSupported;
+    const int64_t n_sm = sm_count();
+    // Both sides' tiles go out in one launch: small grids run side by side, and large ones have one tail instead of
+    // two.  Where the tiles exceed the SMs, the query side gets fewer of them: it has one accumulating product
+    // a step, the key side two.
+    int64_t nq = n_items, nk = n_items;
+    if (2 * n_items > n_sm) {
+        constexpr double share = D == 128 ? 0.44 : 0.40;  // measured best of 0.36 .. 0.48
+        nq = std::min(n_items, std::max<int64_t>(1, (int64_t)((double)n_sm * share + 0.5)));
+        nk = std::min(n_items, n_sm - nq);
+    }
+    p.q_ctas = (int)nq;
+    const bool paired = 8 * bh * p.seq * D > kLevelsBytes;
+    p.list[0] = make_level_schedule(bh, n_tiles, nq, paired);
+    p.list[1] = make_level_schedule(bh, n_tiles, nk, paired);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nq + nk));
+    cfg.blockDim = dim3(320);
+    cfg.dynamicSmemBytes = BwdCfg<D>::SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, bwd_tcgen05_kernel<D>, m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
 }
 
 }  // namespace
@@ -420,16 +539,15 @@ cudaError_t launch_backward_tcgen05(const void* q, const void* k, const void* v,
                                     int64_t seq, int dim, int causal, float scale, cudaStream_t stream) {
     const int64_t bh = batch * heads;
     if ((dim != 64 && dim != 128) || bh > 65535 || seq > (1 << 30)) return cudaErrorNotSupported;
-    // own-side tiles are 128-row boxes, other-side steps 64-row boxes of the same tensors
-    CUtensorMap mq, mk, mv, mdo, hq, hk, hv, hdo;
+    // inputs in boxes of 64 rows; outputs, f32 seen as pairs of 2-byte elements, in boxes of 32 rows x 32 columns
+    CUtensorMap m[7];
     const TensorStrides s = TensorStrides::contiguous(heads, seq, dim);
-    const void* ptrs[4] = {q, k, v, d_out};
-    CUtensorMap* full[4] = {&mq, &mk, &mv, &mdo};
-    CUtensorMap* half[4] = {&hq, &hk, &hv, &hdo};
-    for (int i = 0; i < 4; ++i)
-        if (!make_tensor_map_bf16_4d(full[i], ptrs[i], batch, heads, seq, dim, s.batch, s.head, s.row, 128) ||
-            !make_tensor_map_bf16_4d(half[i], ptrs[i], batch, heads, seq, dim, s.batch, s.head, s.row, 64))
+    const void* ptrs[7] = {q, k, v, d_out, dq, dk, dv};
+    for (int i = 0; i < 7; ++i) {
+        const int f = i < 4 ? 1 : 2;
+        if (!make_tensor_map_bf16_4d(&m[i], ptrs[i], batch, heads, seq, f * dim, f * s.batch, f * s.head, f * s.row, i < 4 ? 64 : 32))
             return cudaErrorNotSupported;
+    }
     Bwd5Params p;
     p.lse = lse;
     p.delta = delta;
@@ -440,23 +558,7 @@ cudaError_t launch_backward_tcgen05(const void* q, const void* k, const void* v,
     p.scale_log2 = scale * kLog2e;
     p.status = device_status_ptr();
     if (!p.status) return cudaErrorInvalidSymbol;
-    static const int env_group = [] {
-        const char* e = getenv("RT_ATTN_BACKWARD_HEAD_GROUP");
-        const int v = e ? atoi(e) : 0;
-        return v > 0 ? v : 4;  // measured: 2-4 about 1 % ahead of 1 (head-major), 16 level, 128 slower by 20 % (L2)
-    }();
-    p.head_group = env_group;
-    // query side: own (Q, dO), other (K, V) -> dQ
-    p.out1 = dq;
-    p.out2 = nullptr;
-    cudaError_t e = dim == 128 ? launch_side<128, false>(mq, mdo, hk, hv, p, bh, stream)
-                               : launch_side<64, false>(mq, mdo, hk, hv, p, bh, stream);
-    if (e != cudaSuccess) return e;
-    // key side: own (K, V), other (Q, dO) -> dV, dK
-    p.out1 = dv;
-    p.out2 = dk;
-    return dim == 128 ? launch_side<128, true>(mk, mv, hq, hdo, p, bh, stream)
-                      : launch_side<64, true>(mk, mv, hq, hdo, p, bh, stream);
+    return dim == 128 ? launch_sides<128>(m, p, bh, stream) : launch_sides<64>(m, p, bh, stream);
 }
 
 }  // namespace rt

@@ -37,6 +37,7 @@
 
 #include "kernels.h"
 #include "tc_ptx.cuh"
+#include "tile_schedule.cuh"
 #include "tensor_map.h"
 
 namespace rt {
@@ -79,7 +80,7 @@ struct TcParams {
     int n_qb;          // 256-row blocks per head
     int n_items, units;  // static schedule, see tc_item: items of the launch, (batch, query head) pairs
     int by_level;      // single-tile items: level after level instead of head after head
-    int rounds, tail_head, tail_skip, n_tail;  // paired rounds, and the blocks that they leave
+    LevelSchedule list;  // causal launches
     int sorted;        // length-sorted schedule (launches with per-batch kv_lens), see tc_item
     int keep_tab;      // sorted schedule with key_keep: index of the per-batch step bounds behind the order in the table, else 0
     int stagger_clocks;  // single-tile items: head start of tile 0 over tile 1, in SM clocks
@@ -231,44 +232,18 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
         if (p.keep_tab) keep_hi = 64 * sched[p.keep_tab + it.b];
     } else {
         const int G = (int)gridDim.x;
-        it.end = false;
-        if (kCausal && j < 2 * p.rounds) {
-            const int slot = (int)blockIdx.x + (j >> 1) * G, per_head = (p.n_qb + 1) >> 1, r = slot % per_head;
-            it.bh = slot / per_head;
-            qb = p.n_qb - 1 - r;
-            if (j & 1) {
-                if (r == qb) return it;  // the middle block of an odd count has no partner
-                qb = r;
-            }
+        if (kCausal) {
+            int rank;
+            if (!level_item(p.list, j, (int)blockIdx.x, G, it.bh, rank, it.end)) return it;
+            qb = p.n_qb - 1 - rank;
         } else {
-            const int jt = kCausal ? j - 2 * p.rounds : j;
-            it.end = jt * G >= p.n_tail;
-            if (it.end) return it;
-            const int pos = jt * G + ((jt & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x);
-            if (pos >= p.n_tail) return it;
-            if (kCausal) {
-                // level t: the t-th heaviest block of every head left; the head that the rounds end in is missing
-                // from the first and last tail_skip levels
-                const int full = p.units - p.tail_head - 1, mid = p.tail_skip * full,
-                          hi = mid + (p.n_qb - 2 * p.tail_skip) * (full + 1);
-                int t;
-                if (pos < mid) {
-                    t = pos / full;
-                    it.bh = p.tail_head + 1 + pos % full;
-                } else if (pos < hi) {
-                    t = p.tail_skip + (pos - mid) / (full + 1);
-                    it.bh = p.tail_head + (pos - mid) % (full + 1);
-                } else {
-                    t = p.n_qb - p.tail_skip + (pos - hi) / full;
-                    it.bh = p.tail_head + 1 + (pos - hi) % full;
-                }
-                qb = p.n_qb - 1 - t;
-            } else {
-                // head after head; the lighter ragged blocks last
-                const int whole = p.seq / 256, n_whole = p.units * whole;
-                it.bh = pos < n_whole ? pos / whole : pos - n_whole;
-                qb = pos < n_whole ? pos % whole : whole;
-            }
+            // head after head; the lighter ragged blocks last
+            it.end = j * G >= p.n_items;
+            const int pos = j * G + ((j & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x);
+            if (pos >= p.n_items) return it;
+            const int whole = p.seq / 256, n_whole = p.units * whole;
+            it.bh = pos < n_whole ? pos / whole : pos - n_whole;
+            qb = pos < n_whole ? pos % whole : whole;
         }
         it.b = it.bh / p.heads;
         it.h = it.bh % p.heads;
@@ -1401,18 +1376,8 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
     const int64_t n_ctas = (persistent && n_items > n_sm) ? n_sm : n_items;
     p.n_items = (int)n_items;
     p.units = (int)bh;
-    p.rounds = p.tail_head = p.tail_skip = 0;
-    p.n_tail = (int)n_items;
+    p.list = make_level_schedule(bh, n_qb, n_ctas, batch * heads_kv * seq_kv * dim * 4 > kLevelsKvBytes && n_ctas < n_items);
     p.by_level = n_items * p.split > n_sm ? 1 : 0;
-    if (causal && n_ctas < n_items && !p.sorted) {
-        const int64_t per_head = (n_qb + 1) / 2, all = bh * per_head / n_ctas;
-        const int64_t kv_bytes = batch * heads_kv * seq_kv * dim * 4;
-        p.rounds = (kv_bytes > kLevelsKvBytes && all > 1) ? (int)(all - 1) : 0;
-        const int64_t taken = p.rounds * n_ctas;
-        p.tail_head = (int)(taken / per_head);
-        p.tail_skip = (int)(taken % per_head);
-        p.n_tail = p.tail_head == bh ? 0 : (int)((bh - p.tail_head) * n_qb - 2 * p.tail_skip);
-    }
     p.direct_out = n_ctas == n_items ? 1 : 0;  // every CTA has exactly one item
     const bool keep = key_keep != nullptr;
     p.tighten = (keep && p.direct_out && seq_kv > 0) ? 1 : 0;

@@ -193,3 +193,31 @@ def test_prefill_clusters(B, Hq, Hkv, Nq, Nkv, D, causal, lens):
         ref = torch.softmax(s, -1) @ vb
         assert float((out[b].float() - ref).norm() / ref.norm()) < 1e-2
         assert torch.allclose(lse[b], torch.logsumexp(s, -1), rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("B,H,N,D,causal,part", [
+    (2, 37, 129, 64, True, 1),      # as many tiles of both sides as SMs, then twice that
+    (3, 64, 200, 64, False, 1),     # several tiles a CTA, an odd count of steps
+    (28, 20, 1100, 64, True, 7),    # operands beyond L2: paired rounds that end inside a head
+    (9, 16, 577, 128, True, 3),     # levels only, last tile with one row
+])
+def test_backward_schedules(B, H, N, D, causal, part):
+    """Every tile of either side is visited once whatever the schedule: bit for bit what launches over parts of the
+    batch give."""
+    import torch
+    import rustorch_b200 as rt
+    torch.manual_seed(8)
+    q, k, v, do = (torch.randn(B, H, N, D, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    out, lse = rt.prefill_bf16(q, k, v, causal=causal)
+    grads = rt.backward_bf16(q, k, v, out, do, lse, causal=causal)
+    for b in range(0, B, part):
+        s = slice(b, b + part)
+        for whole, piece in zip(grads, rt.backward_bf16(*(x[s].contiguous() for x in (q, k, v, out, do, lse)), causal=causal)):
+            assert torch.equal(whole[s], piece)
+    x = [t[-1].float().requires_grad_() for t in (q, k, v)]
+    w = x[0] @ x[1].transpose(1, 2) / D ** 0.5
+    if causal:
+        w = w.masked_fill(torch.ones(N, N, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    (torch.softmax(w, -1) @ x[2]).backward(do[-1].float())
+    for g, r in zip(grads, x):
+        assert float((g[-1] - r.grad).norm() / r.grad.norm()) < 2e-2
