@@ -62,6 +62,7 @@ struct DecodeSplit {
                    // kSplitShare: chunks of one size for all `batch` <= 32 sequences, about `target` of them in all,
     int batch;     //              dealt to a flat grid of `ctas` CTAs
     int ctas;
+    int slots;     //              CTAs resident at a time
     float target;
 };
 
@@ -95,14 +96,21 @@ __device__ __forceinline__ DecodeChunk find_chunk(const DecodeSplit& sp, int n_k
     float total = (float)visible;
 #pragma unroll
     for (int off = 16; off; off >>= 1) total += __shfl_xor_sync(kFullMask, total, off);
-    const int share = (int)ceilf(total * (float)n_kv / sp.target);
-    const int size = round_up_64(max(share, (visible + sp.n_chunks - 1) / sp.n_chunks));
-    const int n = max(1, (visible + size - 1) / size), mine = lane < sp.batch ? n * n_kv : 0;
-    int end = mine;
+    int share = (int)ceilf(total * (float)n_kv / sp.target);
+    int n, size, mine, end;
+    for (int tries = 0;; ++tries) {
+        const int most = round_up_64(max(share, (visible + sp.n_chunks - 1) / sp.n_chunks));
+        n = max(1, (visible + most - 1) / most);
+        size = round_up_64((visible + n - 1) / n);  // equal chunks: the last one would end early otherwise
+        end = mine = lane < sp.batch ? n * n_kv : 0;
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int y = __shfl_up_sync(kFullMask, end, off);
-        if (lane >= off) end += y;
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(kFullMask, end, off);
+            if (lane >= off) end += y;
+        }
+        // Lengths alike can all just miss one chunk less; a few CTAs more than fit at once cost a second wave.
+        if (tries == 3 || __shfl_sync(kFullMask, end, 31) <= sp.slots) break;
+        share += share >> 3;
     }
     const int want = blockIdx.x;
     const unsigned owner = __ballot_sync(kFullMask, want >= end - mine && want < end);

@@ -19,6 +19,8 @@
 //   * chunk results are written as normalised (O f32, LSE) partials and merged by
 //     merge_partials_kernel, the same kernel that merges per-GPU partials.
 #include "common.cuh"
+#include <algorithm>
+
 #include "kernels.h"
 
 namespace rt {
@@ -850,8 +852,12 @@ static DecodeSplit pick_split(int64_t batch, int n_kv, int head_dim, int64_t max
             if (groups * group_bytes >= (40 << 20)) {
                 const int64_t n = (span + 63) / 64;
                 sp.mode = kSplitShare;
-                sp.n_chunks = (int)(n < most ? n : most);
+                // no more of one sequence than if it held all tokens (the merge looks at every one: 35.1 -> 32.8 us at
+                // B=3 Hq=64 Hkv=8 D=128, 5000 to 20000 tokens, with 36 instead of 79)
+                const int64_t held = (slots - groups / 2) / n_kv + 1;
+                sp.n_chunks = (int)std::min(std::min(n, most), held);
                 sp.batch = (int)batch;
+                sp.slots = (int)slots;
                 // a sequence's last chunk is half empty on average; at most groups chunks are started beyond the target
                 sp.target = (float)(slots - groups / 2);
                 sp.ctas = (int)(slots + groups - groups / 2);
