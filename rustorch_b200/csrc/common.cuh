@@ -76,12 +76,12 @@ struct DecodeChunk {
 __device__ __forceinline__ int round_up_64(int x) { return max(64, (x + 63) & ~63); }
 
 // Called by all threads of a warp; every warp comes to the same answer on its own.  visible_of(b): tokens of sequence b.
-template <class VisibleOf>
+template <bool kShare, class VisibleOf>
 __device__ __forceinline__ DecodeChunk find_chunk(const DecodeSplit& sp, int n_kv, VisibleOf&& visible_of) {
     DecodeChunk c;
     c.none = false;
     c.rest = 0;
-    if (sp.mode != kSplitShare) {
+    if (!kShare) {
         c.idx = blockIdx.x, c.kvh = blockIdx.y, c.b = blockIdx.z;
         const int visible = visible_of(c.b);
         const int size = sp.mode == kSplitFixed ? sp.chunk : round_up_64((visible + sp.n_chunks - 1) / sp.n_chunks);

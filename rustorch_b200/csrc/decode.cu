@@ -73,12 +73,14 @@ __global__ void __launch_bounds__(128) gqa_decode_splitkv_kernel(const DecodePar
     const int lig = lane % LPT;  // lane within the group: owns dims [lig*8, lig*8+8)
     const bool direct = (p.split.n_chunks == 1);
 
-    const DecodeChunk ck = find_chunk(p.split, p.n_kv, [&](int seq) {  // tokens of a sequence inside the launch's range
+    auto visible_of = [&](int seq) {  // tokens of a sequence inside the launch's range
         int64_t len = p.kv_lens ? (int64_t)p.kv_lens[seq] : p.kv_len_uniform;
         if (len > p.max_seq) len = p.max_seq;
         if (p.kv_end >= 0 && p.kv_end < len) len = p.kv_end;
         return len > p.kv_begin ? (int)(len - p.kv_begin) : 0;
-    });
+    };
+    const DecodeChunk ck = p.split.mode == kSplitShare ? find_chunk<true>(p.split, p.n_kv, visible_of)
+                                                       : find_chunk<false>(p.split, p.n_kv, visible_of);
     if (ck.none) return;
     const int chunk_idx = ck.idx, kvh = ck.kvh, b = ck.b;
     const int64_t row0 = (int64_t)b * p.n_heads + (int64_t)kvh * G;  // first output row of the group

@@ -240,7 +240,7 @@ struct DecodeTcCfg {
 
 enum { kToDecFull = 301 };
 
-template <int D, int G>
+template <int D, int G, bool kShare>
 __global__ void __launch_bounds__(128, 2)
 gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                      const DecodeTcParams p) {
@@ -262,17 +262,17 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
     // Nothing is read from global memory before it.
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    const DecodeChunk ck = find_chunk(p.split, p.n_kv, [&](int seq) {  // tokens of a sequence inside the launch's range
+    const DecodeChunk ck = find_chunk<kShare>(p.split, p.n_kv, [&](int seq) {  // tokens of a sequence inside the launch's range
         int64_t len = p.kv_lens ? (int64_t)p.kv_lens[seq] : p.kv_len_uniform;
         if (len > p.max_seq) len = p.max_seq;
         if (p.kv_end >= 0 && p.kv_end < len) len = p.kv_end;
         return len > p.kv_begin ? (int)(len - p.kv_begin) : 0;
     });
-    if (ck.none) return;
+    if (kShare && ck.none) return;
     const int chunk_idx = ck.idx, kvh = ck.kvh, b = ck.b;
     const int64_t row0 = (int64_t)b * p.n_heads + (int64_t)kvh * G;  // first output row of the group
     const int64_t c0 = p.kv_begin + ck.lo, c1 = p.kv_begin + ck.hi;
-    for (int i = tid; i < ck.rest * G; i += 128)
+    for (int i = tid; kShare && i < ck.rest * G; i += 128)
         p.part_lse[(int64_t)(chunk_idx + 1 + i / G) * p.rows + row0 + i % G] = -INFINITY;
 
     if (c0 >= c1) {  // nothing visible in this chunk: identity partial
@@ -509,11 +509,11 @@ static bool make_cache_map(CUtensorMap* map, const void* base, int64_t rows, int
     return encode_bf16_map_cached(map, 2, base, dims, strides, box);
 }
 
-template <int D, int G>
-static cudaError_t launch_dg(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeTcParams& p, int64_t batch,
+template <int D, int G, bool kShare>
+static cudaError_t launch_dgs(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeTcParams& p, int64_t batch,
                              cudaStream_t stream) {
-    auto kern = gqa_decode_tc_kernel<D, G>;
-    cudaError_t e = set_max_dynamic_smem_once<gqa_decode_tc_kernel<D, G>>(DecodeTcCfg<D>::SMEM_BYTES);
+    auto kern = gqa_decode_tc_kernel<D, G, kShare>;
+    cudaError_t e = set_max_dynamic_smem_once<gqa_decode_tc_kernel<D, G, kShare>>(DecodeTcCfg<D>::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     // RT_ATTN_DECODE_PDL=0 launches without programmatic stream serialisation.
     static const bool pdl = [] {
@@ -533,6 +533,13 @@ static cudaError_t launch_dg(const CUtensorMap& mk, const CUtensorMap& mv, const
         cfg.numAttrs = 1;
     }
     return cudaLaunchKernelEx(&cfg, kern, mk, mv, p);
+}
+
+template <int D, int G>
+static cudaError_t launch_dg(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeTcParams& p, int64_t batch,
+                             cudaStream_t stream) {
+    return p.split.mode == kSplitShare ? launch_dgs<D, G, true>(mk, mv, p, batch, stream)
+                                       : launch_dgs<D, G, false>(mk, mv, p, batch, stream);
 }
 
 template <int D>
