@@ -1179,9 +1179,12 @@ static cudaError_t launch_tc_s(const CUtensorMap& mq, const CUtensorMap& mk, con
         const char* s = getenv("RT_ATTN_PREFILL_PDL");
         return s ? (s[0] == '0' ? 0 : 1) : -1;
     }();
-    // Measured: the overlap pays for short single-tile launches (up to 1 us of 9-16 us); for long ones the
-    // dependency wait costs as much as the launch gap it hides.
-    const bool pdl = !kSplit && (env_pdl >= 0 ? env_pdl == 1 : (kSingle && p.seq_kv <= 1024));
+    // The next launch's set-up, and its first CTAs on SMs that run out of work, overlap this one's tail: 3 to 11 % of
+    // launches of 15 to 120 us with uneven items, nothing or 1 us below.  Two kinds lose 1 to 4 % instead and go without:
+    // one wave of long equal chains on most SMs (a prompt chunk), and lists of many items, whose tail is short.
+    const int n_sm = sm_count();
+    const bool equal_wave = p.n_items * 4 > 3 * n_sm && p.n_items <= n_sm && p.seq_kv > 4096;
+    const bool pdl = !kSplit && (env_pdl >= 0 ? env_pdl == 1 : kSingle ? !equal_wave : p.n_items < 8 * n_sm);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_ctas);
     cfg.blockDim = dim3(384);
