@@ -1184,25 +1184,23 @@ static cudaError_t launch_tc_s(const CUtensorMap& mq, const CUtensorMap& mk, con
     // one wave of long equal chains on most SMs (a prompt chunk), and lists of many items, whose tail is short.
     const int n_sm = sm_count();
     const bool equal_wave = p.n_items * 4 > 3 * n_sm && p.n_items <= n_sm && p.seq_kv > 4096;
-    const bool pdl = !kSplit && (env_pdl >= 0 ? env_pdl == 1 : kSingle ? !equal_wave : p.n_items < 8 * n_sm);
+    const bool pdl = env_pdl >= 0 ? env_pdl == 1 : kSplit || (kSingle ? !equal_wave : p.n_items < 8 * n_sm);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_ctas);
     cfg.blockDim = dim3(384);
     cfg.dynamicSmemBytes = TcCfg<D>::SMEM_BYTES;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
     if (pdl) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
     if constexpr (kSplit) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)p.split;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = (unsigned)p.split;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
     }
     return cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, mo, p);
 }
