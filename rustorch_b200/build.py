@@ -50,12 +50,31 @@ def needs_build() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _built_for() -> str:
+    """What the extension is tied to besides its source: the interpreter, and the torch whose headers and libraries it uses."""
+    import torch
+    return f"{sys.implementation.cache_tag} {torch.__version__} abi{int(torch.compiled_with_cxx11_abi())}\n"
+
+
+def binding_is_current() -> bool:
+    """The extension is newer than its sources and was built for this interpreter and torch."""
+    header = os.path.join(PKG_DIR, "..", "include", "rustorch_attn.h")
+    stamp = BINDING_PATH + ".stamp"
+    if not (os.path.exists(BINDING_PATH) and os.path.exists(stamp)):
+        return False
+    if os.path.getmtime(BINDING_PATH) <= max(os.path.getmtime(BINDING_SOURCE), os.path.getmtime(header)):
+        return False
+    with open(stamp) as f:
+        return f.read() == _built_for()
+
+
 def build_binding(force: bool = False) -> str:
     """g++ over torch_binding.cpp against torch's headers; linked to the C-ABI library next to it."""
-    header = os.path.join(PKG_DIR, "..", "include", "rustorch_attn.h")
-    if not force and os.path.exists(BINDING_PATH) and os.path.getmtime(BINDING_PATH) > max(
-            os.path.getmtime(BINDING_SOURCE), os.path.getmtime(header)):
+    if not force and binding_is_current():
         return BINDING_PATH
+    stamp = BINDING_PATH + ".stamp"
+    if os.path.exists(stamp):  # a build that is cut short leaves no record
+        os.remove(stamp)
     import sysconfig
     import torch
     root = os.path.dirname(torch.__file__)
@@ -70,6 +89,8 @@ def build_binding(force: bool = False) -> str:
     if proc.returncode != 0:
         sys.stderr.write(proc.stdout + proc.stderr)
         raise RuntimeError("g++ failed building _torch_binding.so")
+    with open(stamp, "w") as f:
+        f.write(_built_for())
     return BINDING_PATH
 
 
