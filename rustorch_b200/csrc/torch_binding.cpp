@@ -71,6 +71,18 @@ inline bool scale_arg(PyObject* o, float& v) {
     return true;
 }
 
+// The truth of a flag; false for a value whose truth test raises (an array of several elements): the wrapper's own test
+// raises it then.
+inline bool flag_arg(PyObject* o, bool& v) {
+    const int truth = PyObject_IsTrue(o);
+    if (truth < 0) {
+        PyErr_Clear();
+        return false;
+    }
+    v = truth != 0;
+    return true;
+}
+
 inline Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Device& dev) {
     return at::detail::empty_cuda(sizes, type, dev, std::nullopt);
 }
@@ -123,9 +135,11 @@ PyObject* gqa_decode(PyObject*, PyObject* const* arg, Py_ssize_t n) {
         DecodeArgs a;
         int64_t kv_len, kv_begin, kv_end;
         float scale;
+        bool want_lse;
         if (!decode_args(q, k, v, a) || !optional_arg(arg[3], lens) || !int_arg(arg[4], kv_len, 0) ||
             !int_arg(arg[5], kv_begin, 0) || !int_arg(arg[6], kv_end, -1) || !scale_arg(arg[7], scale) ||
-            !optional_arg(arg[10], ws) || !optional_arg(arg[11], out) || !optional_arg(arg[12], lse))
+            !flag_arg(arg[9], want_lse) || !optional_arg(arg[10], ws) || !optional_arg(arg[11], out) ||
+            !optional_arg(arg[12], lse))
             Py_RETURN_NONE;
         if (lens && !(vector_of(*lens, a.B, a.dev) && lens->dim() == 1)) Py_RETURN_NONE;
         if (ws && !dense(*ws, at::kByte, a.dev)) Py_RETURN_NONE;
@@ -146,7 +160,7 @@ PyObject* gqa_decode(PyObject*, PyObject* const* arg, Py_ssize_t n) {
             new_out = empty(q->sizes(), out_type, a.dev);
             out = &new_out;
         }
-        if (!lse && PyObject_IsTrue(arg[9]) == 1) {
+        if (!lse && want_lse) {
             new_lse = empty({a.B, a.Hq}, kF32, a.dev);
             lse = &new_lse;
         }
@@ -223,8 +237,9 @@ PyObject* prefill_bf16(PyObject*, PyObject* const* arg, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         if (n != 11) Py_RETURN_NONE;
         const Tensor *q = tensor_arg(arg[0]), *k = tensor_arg(arg[1]), *v = tensor_arg(arg[2]), *out, *lse;
-        if (!q || !k || !v || !q->is_cuda() || q->dim() != 4 || k->dim() != 4 || !optional_arg(arg[7], out) ||
-            !optional_arg(arg[8], lse))
+        bool causal, want_lse;
+        if (!q || !k || !v || !q->is_cuda() || q->dim() != 4 || k->dim() != 4 || !flag_arg(arg[3], causal) ||
+            !optional_arg(arg[7], out) || !optional_arg(arg[8], lse) || !flag_arg(arg[9], want_lse))
             Py_RETURN_NONE;
         const at::Device dev = q->device();
         const int64_t B = q->size(0), H = q->size(1), N = q->size(2), D = q->size(3), Hkv = k->size(1), Nkv = k->size(2);
@@ -241,7 +256,7 @@ PyObject* prefill_bf16(PyObject*, PyObject* const* arg, Py_ssize_t n) {
                                                         : empty(q->sizes(), kBf16, dev);
             out = &new_out;
         }
-        if (!lse && PyObject_IsTrue(arg[9]) == 1) {
+        if (!lse && want_lse) {
             new_lse = empty({B, H, N}, kF32, dev);
             lse = &new_lse;
         }
@@ -255,7 +270,7 @@ PyObject* prefill_bf16(PyObject*, PyObject* const* arg, Py_ssize_t n) {
         if (strided)
             for (const Tensor* t : all)
                 if (t->numel() == 0 || t->stride(3) != 1) Py_RETURN_NONE;
-        const int flags = PyObject_IsTrue(arg[3]) == 1 ? RT_MASK_CAUSAL : RT_MASK_NONE;
+        const int flags = causal ? RT_MASK_CAUSAL : RT_MASK_NONE;
         void* stream = c10::cuda::getCurrentCUDAStream().stream();
         const int rc = unlocked([&] {
             if (strided)
@@ -281,8 +296,9 @@ PyObject* mha_prefill_bf16(PyObject*, PyObject* const* arg, Py_ssize_t n) {
         if (n != 11) Py_RETURN_NONE;
         const Tensor *q = tensor_arg(arg[0]), *k = tensor_arg(arg[1]), *v = tensor_arg(arg[2]);
         int64_t H, Hkv;
+        bool causal, want_lse;
         if (!q || !k || !v || !q->is_cuda() || q->dim() != 3 || k->dim() != 3 || !int_arg(arg[3], H, 0) ||
-            !int_arg(arg[4], Hkv, H) || H <= 0 || Hkv <= 0)
+            !int_arg(arg[4], Hkv, H) || H <= 0 || Hkv <= 0 || !flag_arg(arg[5], causal) || !flag_arg(arg[9], want_lse))
             Py_RETURN_NONE;
         const at::Device dev = q->device();
         const int64_t B = q->size(0), T = q->size(1), E = q->size(2), S = k->size(1), D = E / H;
@@ -293,10 +309,9 @@ PyObject* mha_prefill_bf16(PyObject*, PyObject* const* arg, Py_ssize_t n) {
             Py_RETURN_NONE;
         const Tensor out = empty({B, T, E}, kBf16, dev);
         Tensor lse;
-        const bool want_lse = PyObject_IsTrue(arg[9]) == 1;
         if (want_lse) lse = empty({B, H, T}, kF32, dev);
         const int64_t sq[3] = {T * E, D, E}, sk[3] = {S * Hkv * D, D, Hkv * D};
-        const int flags = PyObject_IsTrue(arg[5]) == 1 ? RT_MASK_CAUSAL : RT_MASK_NONE;
+        const int flags = causal ? RT_MASK_CAUSAL : RT_MASK_NONE;
         void* stream = c10::cuda::getCurrentCUDAStream().stream();
         const int rc = unlocked([&] {
             return rt_attn_prefill_strided_bf16(ptr(q), ptr(k), ptr(v), ptr(&out), want_lse ? ptr<float>(&lse) : nullptr, B, H,
@@ -313,7 +328,8 @@ PyObject* prefill_f32(PyObject*, PyObject* const* arg, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         if (n != 8) Py_RETURN_NONE;
         const Tensor *q = tensor_arg(arg[0]), *k = tensor_arg(arg[1]), *v = tensor_arg(arg[2]);
-        if (!q || !k || !v || !q->is_cuda() || q->dim() != 4 || k->dim() != 4) Py_RETURN_NONE;
+        bool causal;
+        if (!q || !k || !v || !q->is_cuda() || q->dim() != 4 || k->dim() != 4 || !flag_arg(arg[3], causal)) Py_RETURN_NONE;
         const at::Device dev = q->device();
         const int64_t B = q->size(0), H = q->size(1), N = q->size(2), D = q->size(3), Hkv = k->size(1), Nkv = k->size(2);
         MaskArgs m;
@@ -321,7 +337,7 @@ PyObject* prefill_f32(PyObject*, PyObject* const* arg, Py_ssize_t n) {
             v->sizes() != k->sizes() || !mask_args(arg[4], arg[5], arg[6], arg[7], B, Nkv, dev, m))
             Py_RETURN_NONE;
         const Tensor out = empty(q->sizes(), kF32, dev), lse = empty({B, H, N}, kF32, dev);
-        const int flags = PyObject_IsTrue(arg[3]) == 1 ? RT_MASK_CAUSAL : RT_MASK_NONE;
+        const int flags = causal ? RT_MASK_CAUSAL : RT_MASK_NONE;
         void* stream = c10::cuda::getCurrentCUDAStream().stream();
         const int rc = unlocked([&] {
             return rt_attn_prefill_f32(ptr<float>(q), ptr<float>(k), ptr<float>(v), ptr<float>(&out), ptr<float>(&lse), B, H,
@@ -345,17 +361,18 @@ PyObject* backward(PyObject*, PyObject* const* arg, Py_ssize_t n) {
         const at::Device dev = t[0]->device();
         const int64_t B = t[0]->size(0), H = t[0]->size(1), N = t[0]->size(2), D = t[0]->size(3);
         float scale;
+        bool causal;
         for (int i = 0; i < 5; ++i)
             if (!dense(*t[i], kIsBf16 ? kBf16 : kF32, dev) || t[i]->sizes() != t[0]->sizes()) Py_RETURN_NONE;
         const Tensor& lse = *t[5];
         if (!(dense(lse, kF32, dev) && lse.dim() == 3 && lse.size(0) == B && lse.size(1) == H && lse.size(2) == N) ||
-            !scale_arg(arg[7], scale))
+            !flag_arg(arg[6], causal) || !scale_arg(arg[7], scale))
             Py_RETURN_NONE;
         const Tensor dq = empty(t[0]->sizes(), kF32, dev), dk = empty(t[0]->sizes(), kF32, dev),
                      dv = empty(t[0]->sizes(), kF32, dev);
         const size_t need = rt_attn_backward_workspace_bytes(B, H, N);
         const Tensor ws = empty({(int64_t)(need > 4 ? need : 4)}, at::kByte, dev);
-        const int flags = PyObject_IsTrue(arg[6]) == 1 ? RT_MASK_CAUSAL : RT_MASK_NONE;
+        const int flags = causal ? RT_MASK_CAUSAL : RT_MASK_NONE;
         void* stream = c10::cuda::getCurrentCUDAStream().stream();
         const int rc = unlocked([&] {
             if constexpr (kIsBf16)

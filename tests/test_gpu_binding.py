@@ -64,3 +64,30 @@ def test_extension_and_ctypes_paths_agree(name, monkeypatch):
         if a is not None:
             assert a.shape == b.shape and a.stride() == b.stride() and a.dtype == b.dtype
             assert torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0))
+
+
+class _NoTruth:
+    def __bool__(self):
+        raise ValueError("truth is ambiguous")
+
+
+@pytest.mark.parametrize("name", ["decode", "prefill", "prefill_lse", "mha", "mha_lse", "f32", "backward_bf16", "backward_f32"])
+def test_flag_without_a_truth_value_raises_its_own_error(name):
+    """A flag whose truth test raises (as an array of several elements does): the caller sees that error."""
+    import torch
+    import rustorch_b200 as rt
+    x = torch.zeros(1, 2, 64, 64, device="cuda", dtype=torch.bfloat16)
+    f, act, qd = x.float(), x.view(1, 64, 128), x[:, :, 0].contiguous()
+    lse, bad = torch.zeros(1, 2, 64, device="cuda"), _NoTruth()
+    call = {
+        "decode": lambda: rt.gqa_decode(qd, x, x, kv_len=3, return_lse=bad),
+        "prefill": lambda: rt.prefill_bf16(x, x, x, causal=bad),
+        "prefill_lse": lambda: rt.prefill_bf16(x, x, x, return_lse=bad),
+        "mha": lambda: rt.mha_prefill_bf16(act, act, act, 2, causal=bad),
+        "mha_lse": lambda: rt.mha_prefill_bf16(act, act, act, 2, return_lse=bad),
+        "f32": lambda: rt.prefill_f32(f, f, f, causal=bad),
+        "backward_bf16": lambda: rt.backward_bf16(x, x, x, x, x, lse, causal=bad),
+        "backward_f32": lambda: rt.backward_f32(f, f, f, f, f, lse, causal=bad),
+    }[name]
+    with pytest.raises(ValueError, match="truth is ambiguous"):
+        call()
