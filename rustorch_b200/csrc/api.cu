@@ -289,7 +289,7 @@ static_assert(kMaxHostChunks <= rt::HostJob::Device::kMaxChunks, "one event per 
 // (the link alone takes 300), 1054 -> 291 us in bf16.
 int rt_flash_forward_f32_host(const float* q, size_t q_len, const float* k, size_t k_len, const float* v,
                               size_t v_len, float* out, size_t out_len, int64_t batch, int64_t heads, int64_t seq,
-                              int64_t dim, int mask_kind, const uint8_t* keep, size_t keep_len, int precision) {
+                              int64_t dim, int mask_kind, const uint8_t* keep, size_t keep_len, int precision) try {
     // validate(): cpu_forward.rs:142-169
     if (dim == 0) return RT_ERR_ZERO_DIM;
     if (batch < 0 || heads < 0 || seq < 0 || dim < 0) return RT_ERR_BAD_LENGTH;
@@ -334,7 +334,6 @@ int rt_flash_forward_f32_host(const float* q, size_t q_len, const float* k, size
     const uint8_t* keep_dev = nullptr;
     if (mask_kind == RT_MASKKIND_PADDING) {
         RT_CUDA(dkeep.alloc(keep_len));
-        RT_CUDA(cudaMemcpyAsync(dkeep.p, keep, keep_len, cudaMemcpyHostToDevice, hd.in));
         keep_dev = dkeep.as<uint8_t>();
     }
     const int flags = (mask_kind == RT_MASKKIND_CAUSAL) ? RT_MASK_CAUSAL : RT_MASK_NONE;
@@ -352,6 +351,8 @@ int rt_flash_forward_f32_host(const float* q, size_t q_len, const float* k, size
         job.upload(c, (host_convert ? bv : dv).as<char>() + off * size, v + off, cnt, size, in_mode, stage_v);
         job.download(c, out + off, (host_convert ? bo : dout).as<char>() + off * size, cnt, size, out_mode, stage_out);
     }
+    // from here on nothing returns without waiting for what is under way
+    if (keep_dev) RT_CUDA(cudaMemcpyAsync(dkeep.p, keep, keep_len, cudaMemcpyHostToDevice, hd.in));
     return job.run(n_chunks, [&](int c, cudaStream_t s) -> int {
         const int64_t units = plan[c].h1 - plan[c].h0;
         const size_t off = (size_t)plan[c].h0 * slab, cnt = (size_t)units * slab;
@@ -371,12 +372,14 @@ int rt_flash_forward_f32_host(const float* q, size_t q_len, const float* k, size
             RT_CUDA(rt::launch_bf16_to_f32(bo.as<char>() + off * 2, dout.as<float>() + off, (int64_t)cnt, s));
         return rc;
     });
+} catch (...) {
+    return rt::exception_status();
 }
 
 // The same pipeline for bf16 host data; per-batch kv_lens keep a chunk inside one batch element, or make it whole ones.
 int rt_attn_prefill_bf16_host(const void* q, const void* k, const void* v, void* out, float* lse, int64_t batch,
                               int64_t heads, int64_t seq, int dim, int mask_flags, const int32_t* kv_lens,
-                              float scale) {
+                              float scale) try {
     if (dim == 0) return RT_ERR_ZERO_DIM;
     if (batch < 0 || heads < 0 || seq < 0 || dim < 0) return RT_ERR_BAD_LENGTH;
     const size_t n = (size_t)batch * heads * seq * dim;
@@ -397,10 +400,7 @@ int rt_attn_prefill_bf16_host(const void* q, const void* k, const void* v, void*
     RT_CUDA(dout.alloc(n * 2));
     const size_t rows = (size_t)batch * heads * seq;
     if (lse) RT_CUDA(dlse.alloc(rows * 4));
-    if (kv_lens) {
-        RT_CUDA(dlens.alloc((size_t)batch * 4));
-        RT_CUDA(cudaMemcpyAsync(dlens.p, kv_lens, (size_t)batch * 4, cudaMemcpyHostToDevice, hd.in));
-    }
+    if (kv_lens) RT_CUDA(dlens.alloc((size_t)batch * 4));
     const size_t slab = (size_t)seq * dim;  // elements of one (b,h)
     HostChunk plan[kMaxHostChunks];
     const int n_chunks = plan_host_chunks(batch, heads, 3 * slab * 2, plan);
@@ -417,6 +417,7 @@ int rt_attn_prefill_bf16_host(const void* q, const void* k, const void* v, void*
         if (lse)
             job.download(c, lse + at * seq, dlse.as<float>() + at * seq, units * seq, 4, rt::HostMode::kCopy, stage_lse);
     }
+    if (kv_lens) RT_CUDA(cudaMemcpyAsync(dlens.p, kv_lens, (size_t)batch * 4, cudaMemcpyHostToDevice, hd.in));
     return job.run(n_chunks, [&](int c, cudaStream_t s) -> int {
         const size_t at = (size_t)plan[c].b0 * heads + plan[c].h0, off = at * slab * 2;
         return rt_attn_prefill_bf16(dq.as<char>() + off, dk.as<char>() + off, dv.as<char>() + off, dout.as<char>() + off,
@@ -424,6 +425,8 @@ int rt_attn_prefill_bf16_host(const void* q, const void* k, const void* v, void*
                                     dim, mask_flags, kv_lens ? dlens.as<int32_t>() + plan[c].b0 : nullptr, nullptr, 0,
                                     scale, s);
     });
+} catch (...) {
+    return rt::exception_status();
 }
 
 // ------------------------------------------------------------------------------ backward
@@ -469,7 +472,7 @@ int rt_attn_backward_bf16(const void* q, const void* k, const void* v, const voi
 int rt_flash_backward_f32_host(const float* q, size_t q_len, const float* k, size_t k_len, const float* v,
                                size_t v_len, const float* d_out, size_t d_out_len, float* dq, size_t dq_len, float* dk,
                                size_t dk_len, float* dv, size_t dv_len, int64_t batch, int64_t heads, int64_t seq,
-                               int64_t dim, int mask_kind) {
+                               int64_t dim, int mask_kind) try {
     // flash_backward has no dim check of its own: with dim = 0 every length is 0 and the call is a no-op
     if (batch < 0 || heads < 0 || seq < 0 || dim < 0) return RT_ERR_BAD_LENGTH;
     const size_t expected = (size_t)batch * (size_t)heads * (size_t)seq * (size_t)dim;
@@ -517,6 +520,8 @@ int rt_flash_backward_f32_host(const float* q, size_t q_len, const float* k, siz
                                     blse.as<float>(), bdq.as<float>(), bdk.as<float>(), bdv.as<float>(), batch, heads, seq,
                                     (int)dim, flags, -1.f, bdelta.p, stat_bytes, s);
     });
+} catch (...) {
+    return rt::exception_status();
 }
 
 // ------------------------------------------------------------------------------ decode
@@ -771,7 +776,7 @@ int rt_attn_merge_records_after_rows(const float* records, const uint32_t* row_f
 
 int rt_gqa_forward_f32_host(const float* q, size_t q_len, const float* k, size_t k_len, const float* v, size_t v_len,
                             float* out, size_t out_len, int64_t batch, int64_t n_heads, int64_t n_kv_heads,
-                            int64_t seq_q, int64_t seq_kv, int64_t head_dim) {
+                            int64_t seq_q, int64_t seq_kv, int64_t head_dim) try {
     // gqa.rs:106-141
     if (n_kv_heads <= 0 || n_heads < 0 || n_heads % n_kv_heads != 0) return RT_ERR_HEAD_COUNT;
     if (batch < 0 || seq_q < 0 || seq_kv < 0 || head_dim < 0) return RT_ERR_BAD_LENGTH;
@@ -808,6 +813,8 @@ int rt_gqa_forward_f32_host(const float* q, size_t q_len, const float* k, size_t
                                    n_kv_heads, seq_q, seq_kv, (int)head_dim, RT_MASK_NONE, nullptr, nullptr, nullptr, 0,
                                    -1.f, s);
     });
+} catch (...) {
+    return rt::exception_status();
 }
 
 int rt_kv_append_bf16(void* k_cache, void* v_cache, const void* k_in, const void* v_in, int64_t batch, int n_kv,

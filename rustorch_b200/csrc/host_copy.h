@@ -22,8 +22,10 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <functional>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -149,6 +151,18 @@ class HostQueue {
     std::atomic<size_t> next_{0}, limit_{0};
 };
 
+// The status for the exception being handled.  The C entry points catch all (memory, a thread or a lock that the system
+// refuses): none may reach a caller whose frames need not be C++.
+inline int exception_status() noexcept {
+    try {
+        throw;
+    } catch (const std::bad_alloc&) {
+        return (int)cudaErrorMemoryAllocation;
+    } catch (...) {
+        return (int)cudaErrorUnknown;
+    }
+}
+
 // The worker threads and the pinned ring of the process.
 class HostWorkers {
   public:
@@ -160,14 +174,20 @@ class HostWorkers {
     uint8_t* down_slot(size_t i) { return ring + (kUp + i % kDown) * kPiece; }
 
     cudaError_t init() {
-        if (ring) return cudaSuccess;
-        void* p = nullptr;
-        const cudaError_t e = cudaHostAlloc(&p, (kUp + kDown) * kPiece, cudaHostAllocPortable);
-        if (e != cudaSuccess) return e;
-        ring = static_cast<uint8_t*>(p);
-        const int cores = (int)std::thread::hardware_concurrency();
-        const int n = cores > 15 ? 7 : cores > 2 ? cores / 2 - 1 : 0;
-        for (int i = 0; i < n; ++i) threads_.emplace_back([this] { work(); });
+        if (!ring) {
+            void* p = nullptr;
+            const cudaError_t e = cudaHostAlloc(&p, (kUp + kDown) * kPiece, cudaHostAllocPortable);
+            if (e != cudaSuccess) return e;
+            ring = static_cast<uint8_t*>(p);
+        }
+        const size_t cores = std::thread::hardware_concurrency(), n = cores > 15 ? 7 : cores > 2 ? cores / 2 - 1 : 0;
+        // A process that gets no more threads works with the ones it has, none at worst: the calling thread copies as
+        // well.  The next call asks again.
+        try {
+            threads_.reserve(n);
+            while (threads_.size() < n) threads_.emplace_back([this] { work(); });
+        } catch (const std::exception&) {
+        }
         return cudaSuccess;
     }
     // Between begin and end the workers take tasks from both queues; end returns once none of them looks at them.
@@ -276,20 +296,27 @@ class HostJob {
         size_t n_up = 0, n_down = 0;
         for (const Piece& p : up_) n_up += p.staged;
         for (const Piece& p : down_) n_down += p.staged;
-        const bool workers = n_up + n_down > 0;
-        if (workers) {
-            const cudaError_t e = w_.init();
-            if (e != cudaSuccess) return (int)e;
-            w_.up.reset(n_up);
-            w_.down.reset(n_down);
-            size_t k = 0;
-            for (const Piece& p : up_)
-                if (p.staged) w_.up.tasks[k] = HostTask{w_.up_slot(k), p.host, p.n, p.mode, true}, ++k;
-            w_.up.release(n_up < HostWorkers::kUp ? n_up : HostWorkers::kUp);
-            w_.begin();
+        bool working = false;
+        int rc = 0;
+        try {
+            if (n_up + n_down > 0) {
+                rc = (int)w_.init();
+                if (rc == 0) {
+                    w_.up.reset(n_up);
+                    w_.down.reset(n_down);
+                    size_t k = 0;
+                    for (const Piece& p : up_)
+                        if (p.staged) w_.up.tasks[k] = HostTask{w_.up_slot(k), p.host, p.n, p.mode, true}, ++k;
+                    w_.up.release(n_up < HostWorkers::kUp ? n_up : HostWorkers::kUp);
+                    w_.begin();
+                    working = true;
+                }
+            }
+            if (rc == 0) rc = drive(n_chunks, n_up, launch);
+        } catch (...) {
+            rc = exception_status();
         }
-        int rc = drive(n_chunks, n_up, launch);
-        if (workers) w_.end();
+        if (working) w_.end();
         // nothing may still use the ring or the caller's memory when the call returns
         for (cudaStream_t s : {d_.in, d_.comp[0], d_.comp[1], d_.comp[2], d_.comp[3], d_.out}) {
             const cudaError_t e = cudaStreamSynchronize(s);
