@@ -19,6 +19,7 @@
 #endif
 
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
@@ -135,6 +136,7 @@ class HostQueue {
     }
     std::vector<HostTask> tasks;
     void release(size_t upto) { limit_.store(upto, std::memory_order_release); }  // tasks below `upto` are filled in
+    bool waiting() const { return next_.load() < limit_.load(); }                 // a released task that nobody has taken
     bool done(size_t i) const { return done_[i].load(std::memory_order_acquire) != 0; }
     bool run_one() {
         size_t i = next_.load(std::memory_order_relaxed);
@@ -190,6 +192,15 @@ class HostWorkers {
         }
         return cudaSuccess;
     }
+    // Tasks of q below `upto` may be taken from now on.
+    void release(HostQueue& q, size_t upto) {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            q.release(upto);
+            if (asleep_ == 0) return;
+        }
+        cv_.notify_all();
+    }
     // Between begin and end the workers take tasks from both queues; end returns once none of them looks at them.
     void begin() {
         active_.store(true);
@@ -204,6 +215,7 @@ class HostWorkers {
             std::lock_guard<std::mutex> lock(mu_);  // a worker enters under this lock, or sees active_ false
             active_.store(false);
         }
+        cv_.notify_all();
         while (inside_.load() != 0) std::this_thread::yield();
     }
     ~HostWorkers() {
@@ -229,17 +241,33 @@ class HostWorkers {
                 inside_.fetch_add(1);
             }
             int idle = 0;
+            std::chrono::steady_clock::time_point idle_since;
             while (active_.load(std::memory_order_relaxed)) {
-                if (down.run_one() || up.run_one()) idle = 0;
-                else if (++idle > 256) std::this_thread::yield();
+                if (down.run_one() || up.run_one()) {
+                    idle = 0;
+                    continue;
+                }
+                if (++idle <= 256) continue;
+                std::this_thread::yield();
+                if (idle == 257) idle_since = std::chrono::steady_clock::now();
+                if (idle % 16 != 0 || std::chrono::steady_clock::now() - idle_since < kSpin) continue;
+                std::unique_lock<std::mutex> lock(mu_);  // tasks are released under this lock
+                ++asleep_;
+                cv_.wait(lock, [&] { return !active_.load() || down.waiting() || up.waiting(); });
+                --asleep_;
+                idle = 0;
             }
             inside_.fetch_sub(1);
         }
     }
+    // A worker without a task looks for one this long and then sleeps until one is released.  To be woken takes some 50 us,
+    // which would come on top of a short kernel; while a longer one runs, or only pinned data moves, the cores stay free.
+    static constexpr std::chrono::microseconds kSpin{200};
     std::vector<std::thread> threads_;
     std::mutex mu_;
     std::condition_variable cv_;
     uint64_t generation_ = 0;
+    int asleep_ = 0;  // in the middle of a call
     bool stop_ = false;
     std::atomic<bool> active_{false};
     std::atomic<int> inside_{0};
@@ -307,7 +335,7 @@ class HostJob {
                     size_t k = 0;
                     for (const Piece& p : up_)
                         if (p.staged) w_.up.tasks[k] = HostTask{w_.up_slot(k), p.host, p.n, p.mode, true}, ++k;
-                    w_.up.release(n_up < HostWorkers::kUp ? n_up : HostWorkers::kUp);
+                    w_.release(w_.up, n_up < HostWorkers::kUp ? n_up : HostWorkers::kUp);
                     w_.begin();
                     working = true;
                 }
@@ -391,8 +419,8 @@ class HostJob {
                     if (e == cudaErrorNotReady) break;
                     RT_TRY(e);
                     const size_t upto = t.end[t.tail++ % Device::kTransfers];
-                    if (is_up) w_.up.release(upto + HostWorkers::kUp < n_up ? upto + HostWorkers::kUp : n_up);
-                    else w_.down.release(upto);
+                    if (is_up) w_.release(w_.up, upto + HostWorkers::kUp < n_up ? upto + HostWorkers::kUp : n_up);
+                    else w_.release(w_.down, upto);
                     moved = true;
                 }
             }

@@ -1,11 +1,14 @@
 // Drives csrc/host_copy.h against a stand-in for the CUDA runtime in which every copy is done at once, so that what the
 // staging threads do can be tested without a GPU and with a system that refuses threads or memory.
-//   host_copy_check threads | memory
+//   host_copy_check threads | memory | idle
 #include "../rustorch_b200/csrc/host_copy.h"
 
 #include <dlfcn.h>
 #include <pthread.h>
+#include <sys/resource.h>
+#include <time.h>
 
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 
@@ -49,7 +52,7 @@ static rt::HostJob::Device device;
 // entry point would; -1 for a wrong result.
 constexpr size_t n = 6 << 20;
 static std::vector<float> host(n), dev(n), back(n);
-static int call() {
+static int call(int sleep_ms = 0) {
     for (size_t i = 0; i < n; ++i) host[i] = (float)i, back[i] = 0.f;
     int rc;
     try {
@@ -58,11 +61,20 @@ static int call() {
             job.upload(c, dev.data() + c * n / 2, host.data() + c * n / 2, n / 2, 4, rt::HostMode::kCopy, true);
             job.download(c, back.data() + c * n / 2, dev.data() + c * n / 2, n / 2, 4, rt::HostMode::kCopy, true);
         }
-        rc = job.run(2, [](int, cudaStream_t) { return 0; });
+        rc = job.run(2, [&](int, cudaStream_t) {
+            if (sleep_ms) std::this_thread::sleep_for(std::chrono::milliseconds(sleep_ms));
+            return 0;
+        });
     } catch (...) {
         rc = rt::exception_status();
     }
     return rc != 0 ? rc : back == host ? 0 : -1;
+}
+
+static double cpu_ms(clockid_t c) {
+    timespec t;
+    clock_gettime(c, &t);
+    return t.tv_sec * 1e3 + t.tv_nsec * 1e-6;
 }
 
 #define CHECK(x)                                                     \
@@ -99,6 +111,14 @@ int main(int argc, char** argv) {
             if (!short_of) break;
         }
         CHECK(refused > 3);
+    } else if (what == 'i') {  // while a kernel runs and there is nothing to copy, the staging threads sleep
+        CHECK(call() == 0);
+        const double all = cpu_ms(CLOCK_PROCESS_CPUTIME_ID), own = cpu_ms(CLOCK_THREAD_CPUTIME_ID);
+        CHECK(call(300) == 0);  // 0.6 s of waiting
+        const double others = cpu_ms(CLOCK_PROCESS_CPUTIME_ID) - all - (cpu_ms(CLOCK_THREAD_CPUTIME_ID) - own);
+        printf("%.1f ms by the staging threads\n", others);
+        CHECK(others < 100);
+        for (int i = 0; i < 200; ++i) CHECK(call(i % 3) == 0);  // to sleep and back, often
     } else {
         return 2;
     }

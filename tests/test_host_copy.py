@@ -1,4 +1,4 @@
-"""The staging threads of the host entries, on a system that refuses threads or memory.
+"""The staging threads of the host entries, on a system that refuses threads or memory, and while there is nothing to copy.
 
 ``host_copy_check.cpp`` compiles ``csrc/host_copy.h`` against a stand-in for the CUDA runtime."""
 import os
@@ -19,7 +19,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["threads", "memory"])
+@pytest.mark.parametrize("what", ["threads", "memory", "idle"])
 def test_staging(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.endswith("ok\n"), (r.returncode, r.stdout, r.stderr)
