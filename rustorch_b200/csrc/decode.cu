@@ -745,15 +745,18 @@ cudaError_t launch_rope_kv_append(void* q, const void* k_in, const void* v_in, v
 // down from 1024 until the grid both covers the SMs x 2 resident CTAs and fills its last wave
 // to at least 95 % (a long single sequence otherwise loses up to a quarter of a wave).  It depends
 // only on (batch, n_kv, max_seq) so that rt_gqa_decode_workspace_bytes can size the scratch.
-// RT_ATTN_DECODE_CHUNK=<multiple of 64> overrides it.
-static int pick_chunk_tokens(int64_t batch, int n_kv, int64_t max_seq, int64_t slots);
-int decode_chunk_tokens(int64_t batch, int n_kv, int64_t max_seq) {
-    static int forced = [] {
+// RT_ATTN_DECODE_CHUNK=<multiple of 64> is the chunk of every launch instead, here and in pick_split.
+static int forced_chunk() {
+    static const int forced = [] {
         const char* e = getenv("RT_ATTN_DECODE_CHUNK");
         int c = e ? atoi(e) : 0;
         return (c >= 64 && c % 64 == 0) ? c : 0;
     }();
-    if (forced) return forced;
+    return forced;
+}
+static int pick_chunk_tokens(int64_t batch, int n_kv, int64_t max_seq, int64_t slots);
+int decode_chunk_tokens(int64_t batch, int n_kv, int64_t max_seq) {
+    if (const int forced = forced_chunk()) return forced;
     // A decode call asks half a dozen times for the same shape, and the walk below is up to 15 rounds of 64-bit
     // divisions (0.4 us): the last answer is kept per thread.
     struct Last {
@@ -836,7 +839,9 @@ static DecodeSplit pick_split(int64_t batch, int n_kv, int head_dim, int64_t max
     sp.chunk = decode_chunk_tokens(batch, n_kv, max_seq);
     const int64_t groups = batch * (int64_t)n_kv, slots = (int64_t)sm_count() * (head_dim == 64 ? 4 : head_dim == 128 ? 2 : 1);
     const int64_t whole = (span + 63) / 64 * 64, group_bytes = span * head_dim * 4;
-    if (groups >= slots || (groups >= 2 * (int64_t)sm_count() && span > 4096)) {
+    if (forced_chunk()) {
+        // cut at fixed places, sp.chunk apart
+    } else if (groups >= slots || (groups >= 2 * (int64_t)sm_count() && span > 4096)) {
         if (span <= 4096) sp.chunk = (int)whole;
     } else if (groups >= 64 && group_bytes <= (256 << 10)) {
         sp.chunk = (int)whole;

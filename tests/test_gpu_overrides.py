@@ -5,6 +5,7 @@ The library reads its overrides once per process (a launch costs no getenv), so 
 monkeypatch: every override here gets a child pytest process that runs an existing GPU test file with the variable
 set.  What runs under each override:
   RT_ATTN_DECODE_IMPL=simt           the CUDA-core decode kernel for every shape        (csrc/decode.cu)
+  RT_ATTN_DECODE_CHUNK=128           every sequence cut at that length                   (csrc/decode.cu)
   RT_ATTN_DECODE_FUSED_MERGE=0       the separate chunk-merge kernel everywhere          (csrc/decode.cu)
   RT_ATTN_DECODE_PUSH_IN_KERNEL=1    record delivery from inside the decode kernel       (csrc/decode_tc.cu)
   RT_ATTN_EXCHANGE_PDL=0             the row-exchange kernel under a plain launch        (csrc/decode.cu)
@@ -37,6 +38,7 @@ def run_tests_with(var, value, target, select=None, timeout=900):
 
 @pytest.mark.parametrize("var,value,target,select", [
     ("RT_ATTN_DECODE_IMPL", "simt", "test_gpu_decode.py", None),
+    ("RT_ATTN_DECODE_CHUNK", "128", "decode_chunk_cases.py", None),
     ("RT_ATTN_DECODE_FUSED_MERGE", "0", "test_gpu_decode.py", None),
     ("RT_ATTN_DECODE_PUSH_IN_KERNEL", "1", "test_gpu_decode.py", "exchange or push or peer or record"),
     ("RT_ATTN_EXCHANGE_PDL", "0", "test_gpu_decode.py", "exchange"),
