@@ -81,7 +81,7 @@ struct TcParams {
     int n_items, units;  // static schedule, see tc_item: items of the launch, (batch, query head) pairs
     int by_level;      // single-tile items: level after level instead of head after head
     LevelSchedule list;  // causal launches
-    int sorted;        // length-sorted schedule (launches with per-batch kv_lens), see tc_item
+    int sorted;        // length-sorted order (launches with per-batch kv_lens), see tc_item
     int keep_tab;      // sorted schedule with key_keep: index of the per-batch step bounds behind the order in the table, else 0
     int stagger_clocks;  // single-tile items: head start of tile 0 over tile 1, in SM clocks
     int direct_out;    // one item per CTA: the epilogue stores its rows straight from registers (no staged tile, no TMA store)
@@ -179,6 +179,7 @@ struct TcItem {
 // no queue, no atomics and no scratch memory are needed), the item list is that order with all heads of a
 // pair side by side, and it is dealt to the CTAs boustrophedon (0..G-1, G-1..0, ...), heaviest first: the
 // persistent kernel's overlap of one item's set-up with the previous item's tail, and a balanced finish.
+// 128-row items start in that order too where choose_items finds that it pays.
 template <bool kCausal, bool kSingle>
 __device__ __forceinline__ void tc_steps(const TcParams& p, int b, int q0, int& kv_hi, int& q_off, int& U0, int& U1,
                                          int keep_hi = 0x7fffffff, int* t0 = nullptr) {
@@ -204,7 +205,7 @@ __device__ __forceinline__ void tc_steps(const TcParams& p, int b, int q0, int& 
     }
 }
 
-template <bool kCausal, bool kSingle>
+template <bool kCausal, bool kSingle, bool kByLength>
 __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16_t* sched, int keep_hi = 0x7fffffff) {
     TcItem it;
     it.valid = false;
@@ -213,11 +214,19 @@ __device__ __forceinline__ TcItem tc_item(int j, const TcParams& p, const uint16
     if (kSingle) {  // the CTA's only item
         it.end = j > 0;
         if (it.end) return it;
-        const int n = p.by_level ? p.units : p.n_qb, item = (int)blockIdx.x / p.split, a = item / n, r = item % n;
-        it.bh = p.by_level ? r : a;
-        qb = p.n_qb - 1 - (p.by_level ? a : r);
-        it.b = it.bh / p.heads;
-        it.h = it.bh % p.heads;
+        if (kByLength) {
+            const int pair = sched[(int)blockIdx.x / p.heads];
+            qb = pair % p.n_qb;
+            it.b = pair / p.n_qb;
+            it.h = (int)blockIdx.x % p.heads;
+            it.bh = it.b * p.heads + it.h;
+        } else {
+            const int n = p.by_level ? p.units : p.n_qb, item = (int)blockIdx.x / p.split, a = item / n, r = item % n;
+            it.bh = p.by_level ? r : a;
+            qb = p.n_qb - 1 - (p.by_level ? a : r);
+            it.b = it.bh / p.heads;
+            it.h = it.bh % p.heads;
+        }
     } else if (p.sorted) {
         const int G = (int)gridDim.x;
         it.end = (int64_t)j * G >= (int64_t)p.n_items;
@@ -313,7 +322,7 @@ __device__ __forceinline__ void merge_cluster(const TcParams& p, const TcItem& i
 // (o_free: the next item's first PV may overwrite it), stages it in the Q buffer (stage_full),
 // one thread stores it (q_empty: the next item's Q may land).  A tile that sees no key in an
 // item takes no part in these (its rows are written as NaN directly).
-template <int D, bool kCausal, bool kKeep, bool kSingle, bool kSplit>
+template <int D, bool kCausal, bool kKeep, bool kSingle, bool kSplit, bool kByLength>
 __global__ void __launch_bounds__(384, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -384,7 +393,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
             int kv_hi, q_off, U0, U1;
             const int keep_hi = (kKeep && p.keep_tab) ? 64 * sched[p.keep_tab + i / p.n_qb] : 0x7fffffff;
-            tc_steps<kCausal, kSingle>(p, i / p.n_qb, (i % p.n_qb) * 256, kv_hi, q_off, U0, U1, keep_hi);
+            tc_steps<kCausal, kSingle>(p, i / p.n_qb, kByLength ? (i % p.n_qb) * 128 - 128 : (i % p.n_qb) * 256, kv_hi,
+                                       q_off, U0, U1, keep_hi);
             cost[i] = (uint16_t)min(U0 + U1, 65535);
         }
         __syncthreads();
@@ -426,7 +436,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         grid_dep_wait();
         // Q and the first K tile of the first item are requested right away, so their latency
         // overlaps the TMEM allocation and the CTA-wide barrier below.
-        const TcItem it = tc_item<kCausal, kSingle>(0, p, sched);
+        const TcItem it = tc_item<kCausal, kSingle, kByLength>(0, p, sched);
         if (!it.end && it.valid && it.n_tiles > 0) {
             first_preloaded = true;
             if constexpr (kSingle) {
@@ -465,7 +475,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // the bound (the preload above relies on that); a row that sees no kept key is recognised as before.
         grid_dep_wait();
         if (warp < 8) {
-            const uint8_t* keep = p.key_keep + (int64_t)tc_item<kCausal, kSingle>(0, p, sched).b * p.keep_batch_stride;
+            const uint8_t* keep = p.key_keep + (int64_t)tc_item<kCausal, kSingle, kByLength>(0, p, sched).b * p.keep_batch_stride;
             int hi = 1;
             for (int i = threadIdx.x; i < Nkv; i += 256)
                 if (__ldg(keep + i)) hi = i + 1;
@@ -498,7 +508,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             // A single-tile item is its CTA's only item; Q and K tile 0 were requested during setup.  Each
             // issuer reads every tile once and asks for K tile u + 2 right after the PV of step u, so K runs
             // two tiles ahead of V in the request order: K1 | K2 V0 | K3 V1 | ...
-            const TcItem it = tc_item<kCausal, kSingle>(0, p, sched, keep_hi);
+            const TcItem it = tc_item<kCausal, kSingle, kByLength>(0, p, sched, keep_hi);
             if (first_preloaded) {
                 bool ok = true;
                 int kg = 1, vg = 0;
@@ -541,7 +551,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             int na0 = 0, na1 = 0;  // items so far in which tile w took part (phase of its per-item barriers)
             bool ok = true;
             for (int j = 0; ok; ++j) {
-                const TcItem it = tc_item<kCausal, kSingle>(j, p, sched, keep_hi);
+                const TcItem it = tc_item<kCausal, kSingle, kByLength>(j, p, sched, keep_hi);
                 if (it.end) break;
                 if (!it.valid || it.n_tiles == 0) continue;  // nothing to load
                 auto load_q = [&](int w, int na) {
@@ -630,7 +640,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             };
             bool ok = true;
             for (int j = 0; ok; ++j) {
-                const TcItem it = tc_item<kCausal, kSingle>(j, p, sched, keep_hi);
+                const TcItem it = tc_item<kCausal, kSingle, kByLength>(j, p, sched, keep_hi);
                 if (it.end) break;
                 if (!it.valid || it.n_tiles == 0) continue;
                 const int n_u = it.steps(w);
@@ -746,7 +756,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         bool ok = true;
 
         for (int j = 0; ok; ++j) {
-            const TcItem it = tc_item<kCausal, kSingle>(j, p, sched, keep_hi);
+            const TcItem it = tc_item<kCausal, kSingle, kByLength>(j, p, sched, keep_hi);
             if (it.end) break;
             if (!it.valid) continue;
             const int n_iter = it.steps(w);
@@ -1051,7 +1061,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             // ---- the cluster's partial rows: CTA r reads its 128 / split rows from every CTA's shared memory, merges them
             // as above and stores them.  (A CTA that gave up on a wait still meets the barriers.)
             cluster_sync_all();
-            const TcItem it = tc_item<kCausal, kSingle>(0, p, sched, keep_hi);
+            const TcItem it = tc_item<kCausal, kSingle, kByLength>(0, p, sched, keep_hi);
             if (ok) {
                 if (p.split == 2) merge_cluster<D, 2>(p, it, smem_u32(sK), smem_u32(sV));
                 else if (p.split == 4) merge_cluster<D, 4>(p, it, smem_u32(sK), smem_u32(sV));
@@ -1168,11 +1178,11 @@ bool make_tensor_map_bf16_3d(CUtensorMap* map, const void* base, int64_t bh, int
     return encode_bf16_map_cached(map, 3, base, dims, strides, box);
 }
 
-template <int D, bool kCausal, bool kKeep, bool kSingle, bool kSplit>
+template <int D, bool kCausal, bool kKeep, bool kSingle, bool kSplit, bool kByLength = false>
 static cudaError_t launch_tc_s(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                              const TcParams& p, int64_t n_ctas, cudaStream_t stream) {
-    auto kern = prefill_tc_kernel<D, kCausal, kKeep, kSingle, kSplit>;
-    cudaError_t e = set_max_dynamic_smem_once<prefill_tc_kernel<D, kCausal, kKeep, kSingle, kSplit>>(TcCfg<D>::SMEM_BYTES);
+    auto kern = prefill_tc_kernel<D, kCausal, kKeep, kSingle, kSplit, kByLength>;
+    cudaError_t e = set_max_dynamic_smem_once<prefill_tc_kernel<D, kCausal, kKeep, kSingle, kSplit, kByLength>>(TcCfg<D>::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     // RT_ATTN_PREFILL_PDL=0|1 forces programmatic stream serialization off or on.
     static const int env_pdl = [] {
@@ -1208,8 +1218,10 @@ static cudaError_t launch_tc_s(const CUtensorMap& mq, const CUtensorMap& mk, con
 template <int D, bool kCausal, bool kKeep>
 static cudaError_t launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                              const TcParams& p, int64_t n_ctas, cudaStream_t stream) {
-    if constexpr (!kKeep)
+    if constexpr (!kKeep) {
         if (p.split > 1) return launch_tc_s<D, kCausal, false, true, true>(mq, mk, mv, mo, p, n_ctas * p.split, stream);
+        if (p.single_tile && p.sorted) return launch_tc_s<D, kCausal, false, true, false, true>(mq, mk, mv, mo, p, n_ctas, stream);
+    }
     return p.single_tile ? launch_tc_s<D, kCausal, kKeep, true, false>(mq, mk, mv, mo, p, n_ctas, stream)
                          : launch_tc_s<D, kCausal, kKeep, false, false>(mq, mk, mv, mo, p, n_ctas, stream);
 }
@@ -1223,8 +1235,8 @@ static int cluster_slots(int split) {
     std::atomic<int>& slot = known[dev][split == 2 ? 0 : split == 4 ? 1 : 2];
     int n = slot.load(std::memory_order_relaxed);
     if (n > 0) return n - 1;
-    auto kern = prefill_tc_kernel<128, true, false, true, true>;
-    if (set_max_dynamic_smem_once<prefill_tc_kernel<128, true, false, true, true>>(TcCfg<128>::SMEM_BYTES) != cudaSuccess) return 0;
+    auto kern = prefill_tc_kernel<128, true, false, true, true, false>;
+    if (set_max_dynamic_smem_once<prefill_tc_kernel<128, true, false, true, true, false>>(TcCfg<128>::SMEM_BYTES) != cudaSuccess) return 0;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)split;
@@ -1253,17 +1265,28 @@ static int cluster_slots(int split) {
 // 100 rows against 20000 keys D=64 130 -> 24.)  (Between the first two they picked the faster kind
 // or one within 10 % of it on 57 of 57 shapes, within 3 % on 54; the block-count rule that this replaces took
 // 33 us instead of 23 on H=16 N=1795 D=128, 49 / 27 on H=8 N=3500 D=64.)  Lengths that only the
-// device knows are taken at their largest.
-static int choose_items(int64_t bh, int64_t seq, int64_t seq_kv, int64_t dim, bool causal, bool offsets, bool may_split, int n_sm) {
+// device knows (`uneven`) are taken at their largest, but not as equal: without a mask, whole waves of the longest took
+// 256-row items for B=5 H=8 400 rows against 6000 keys D=64 (79 us, 50 with 128 rows) and 128-row items for B=24 H=16
+// D=128 (440 us, 324 with 256 rows by length).
+// *by_length: whether 128-row items are better started in the order of their lengths, where all items of a sequence are
+// about as long (`sortable`: no mask, or a chunk's offsets).  That costs every item about 2 us before its first load
+// (the lengths, the ranking).  Without it a longest item may start last, with nothing to hide behind: over 360 shapes of
+// 2 to 24 sequences, lengths an eighth to all of the cache, that cost between a tenth and a half of its time.  B=6 H=8
+// 700 rows against 8192 keys D=128 106 us in batch order, 79 by length; B=3 H=32 1000 against 3000 D=64 80 and 88.
+static int choose_items(int64_t bh, int64_t seq, int64_t seq_kv, int64_t dim, bool causal, bool offsets, bool uneven, bool sortable,
+                        bool may_split, int n_sm, bool* by_length) {
+    *by_length = false;
     const int64_t n1 = (seq + 127) / 128, n2 = (seq + 255) / 256;
     if (bh * n2 >= 8 * (int64_t)n_sm) return 0;  // many items: the lower total wins, and no loop over long heads
     const double key1 = dim == 128 ? 1.0 : 0.84, item1 = dim == 128 ? 4.8 : 4.2, merge = 4.0;  // 128-row items
     const double key2 = dim == 128 ? 2.0 : 1.7, key2_one = 1.1, item2 = 3.0, first2 = 2.5;     // 256-row items
     const int64_t all = (seq_kv + 127) / 128, off = (causal && offsets && seq_kv > seq) ? seq_kv - seq : 0;
     auto tiles = [&](int64_t row_end) { return causal ? std::min(all, (off + std::min(row_end, seq) + 127) / 128) : all; };
-    // equal CTAs come in whole waves; a causal list is dealt out to within about 8 %
-    auto span = [&](double sum, double mx, int64_t n, int slots) {
-        return causal ? std::max(mx, 1.08 * sum * (double)bh / slots) : mx * (double)((bh * n + slots - 1) / slots);
+    // equal CTAs come in whole waves; a list of unequal ones is dealt out to within about 8 % (of 256-row items that only
+    // the lengths make unequal, 12 %: over 240 shapes the faster kind or within 0.4 % of it on average, 1.2 % with 8 and
+    // 2.5 % with 16)
+    auto span = [&](double sum, double mx, int64_t n, int slots, double over = 1.08) {
+        return causal || uneven ? std::max(mx, over * sum * (double)bh / slots) : mx * (double)((bh * n + slots - 1) / slots);
     };
     double sum = 0, mx = 0;
     for (int64_t i = 0; i < n2; ++i) {
@@ -1271,7 +1294,7 @@ static int choose_items(int64_t bh, int64_t seq, int64_t seq_kv, int64_t dim, bo
         sum += c;
         mx = std::max(mx, c);
     }
-    double best = span(sum, mx, n2, n_sm) + first2;
+    double best = span(sum, mx, n2, n_sm, uneven && !causal ? 1.12 : 1.08) + first2;
     int kind = 0;
     for (int split = 1; split <= (may_split ? 8 : 1); split *= 2) {
         sum = mx = 0;
@@ -1283,6 +1306,7 @@ static int choose_items(int64_t bh, int64_t seq, int64_t seq_kv, int64_t dim, bo
         // a second wave of clusters starts only when whole clusters end (10 us and more a wave)
         if (split > 1 && (bh * n1 * split > n_sm || bh * n1 * split > cluster_slots(split))) break;
         const double t = span(sum, mx, n1 * split, n_sm);
+        if (split == 1 && sortable && bh * n1 > n_sm) *by_length = span(sum + 2.0 * n1, mx + 2.0, n1, n_sm) < t + 0.12 * mx;
         if (t < best) {
             best = t;
             kind = split;
@@ -1345,7 +1369,12 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
         const char* s = getenv("RT_ATTN_PREFILL_SCHED");
         return (s && !strcmp(s, "persistent")) ? 1 : (s && !strcmp(s, "percta")) ? 2 : 0;
     }();
-    const int kind = choose_items(bh, seq, seq_kv, dim, causal, q_offsets != nullptr, key_keep == nullptr && env_tiles == 0, n_sm);
+    const bool uneven = kv_lens != nullptr && batch > 1;
+    // (the ranking of 128-row items: one pass of the CTA's first 128 threads)
+    const bool sortable = uneven && (q_offsets != nullptr || !causal) && key_keep == nullptr && batch * ((seq + 127) / 128) <= 128;
+    bool by_length;
+    const int kind = choose_items(bh, seq, seq_kv, dim, causal, q_offsets != nullptr, uneven, sortable,
+                                  key_keep == nullptr && env_tiles == 0, n_sm, &by_length);
     p.single_tile = kind > 0 ? 1 : 0;
     p.split = kind > 1 ? kind : 1;
     static const int env_stagger = [] {
@@ -1374,6 +1403,7 @@ cudaError_t launch_prefill_tc(const void* q, const void* k, const void* v, void*
         p.keep_tab = keep_sorted ? (int)n_pairs : 0;
         persistent = true;
     }
+    if (p.single_tile && p.split == 1 && by_length && env_sched != 2) p.sorted = 1;
     const int64_t n_ctas = (persistent && n_items > n_sm) ? n_sm : n_items;
     p.n_items = (int)n_items;
     p.units = (int)bh;

@@ -195,6 +195,29 @@ def test_prefill_clusters(B, Hq, Hkv, Nq, Nkv, D, causal, lens):
         assert torch.allclose(lse[b], torch.logsumexp(s, -1), rtol=1e-4, atol=1e-3)
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nkv,D,causal,lens", [
+    (4, 16, 2, 300, 2500, 64, True, (300, 2500, 0, 2499)),   # one sequence empty, two alike
+    (5, 8, 8, 513, 2600, 128, True, (640, 2600, 700, 513, 200)),  # fewer keys than queries: rows without a key
+    (2, 40, 8, 200, 3000, 128, False, (129, 2999)),          # no mask: the length alone
+    (32, 2, 1, 500, 4000, 64, True, (500, 4000)),            # as many pairs as are ranked
+    (33, 2, 1, 500, 4000, 64, True, (500, 4000)),            # more: the order of the batch
+])
+def test_prefill_chunks_by_length(oracle, B, Hq, Hkv, Nq, Nkv, D, causal, lens):
+    """More 128-row items than SMs, of sequences whose lengths only the device knows."""
+    import rustorch_b200 as rt
+    n = np.linspace(min(lens), max(lens), B).astype(np.int32) if len(lens) != B else np.array(lens, dtype=np.int32)
+    if len(lens) != B:
+        np.random.default_rng(2).shuffle(n)
+    off = (n - Nq).astype(np.int32)
+    q = util.normal_bf16(oracle, (B, Hq, Nq, D), util.SEED_Q)
+    k, v = (util.normal_bf16(oracle, (B, Hkv, Nkv, D), s) for s in (util.SEED_K, util.SEED_V))
+    out, lse = rt.prefill_bf16(*(util.to_cuda_bf16(x) for x in (q, k, v)), causal=causal, kv_lens=util.to_cuda(n),
+                               q_offsets=util.to_cuda(off) if causal else None)
+    _, ref, ref_lse = oracle.attention_general(q, k, v, causal=causal, kv_lens=n, q_offsets=off if causal else None)
+    util.check_output(util.to_np(out), ref, label=f"B{B} {Nq}/{Nkv} D{D}")
+    util.check_lse(util.to_np(lse), ref_lse)
+
+
 @pytest.mark.parametrize("B,H,N,D,causal,part", [
     (2, 37, 129, 64, True, 1),      # as many tiles of both sides as SMs, then twice that
     (3, 64, 200, 64, False, 1),     # several tiles a CTA, an odd count of steps
