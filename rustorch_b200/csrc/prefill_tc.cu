@@ -1271,8 +1271,8 @@ static int cluster_slots(int split) {
 // *by_length: whether 128-row items are better started in the order of their lengths, where all items of a sequence are
 // about as long (`sortable`: no mask, or a chunk's offsets).  That costs every item about 2 us before its first load
 // (the lengths, the ranking).  Without it a longest item may start last, with nothing to hide behind: over 360 shapes of
-// 2 to 24 sequences, lengths an eighth to all of the cache, that cost between a tenth and a half of its time.  B=6 H=8
-// 700 rows against 8192 keys D=128 106 us in batch order, 79 by length; B=3 H=32 1000 against 3000 D=64 80 and 88.
+// 2 to 24 sequences, lengths an eighth to all of the cache, that cost between a tenth and a half of its time.  B=4 H=8
+// 700 rows against 8192 keys D=128 78 us in batch order, 59 by length; B=3 H=32 1000 against 3000 D=64 80 and 88.
 static int choose_items(int64_t bh, int64_t seq, int64_t seq_kv, int64_t dim, bool causal, bool offsets, bool uneven, bool sortable,
                         bool may_split, int n_sm, bool* by_length) {
     *by_length = false;
