@@ -1189,12 +1189,16 @@ static cudaError_t launch_tc_s(const CUtensorMap& mq, const CUtensorMap& mk, con
         const char* s = getenv("RT_ATTN_PREFILL_PDL");
         return s ? (s[0] == '0' ? 0 : 1) : -1;
     }();
-    // The next launch's set-up, and its first CTAs on SMs that run out of work, overlap this one's tail: 3 to 11 % of
-    // launches of 15 to 120 us with uneven items, nothing or 1 us below.  Two kinds lose 1 to 4 % instead and go without:
-    // one wave of long equal chains on most SMs (a prompt chunk), and lists of many items, whose tail is short.
-    const int n_sm = sm_count();
-    const bool equal_wave = p.n_items * 4 > 3 * n_sm && p.n_items <= n_sm && p.seq_kv > 4096;
-    const bool pdl = env_pdl >= 0 ? env_pdl == 1 : kSplit || (kSingle ? !equal_wave : p.n_items < 8 * n_sm);
+    // The next launch's set-up, and its first CTAs on SMs that run out of work, overlap this one's tail: 2 to 25 % of
+    // launches below 50 us, 0.5 to 2 % of ones up to 1 ms, over 1100 shapes of all kinds and 1 to 30 items per SM.  One
+    // kind is faster without: a wave of 128-row items at D = 128 of which many walk one long K/V in step (CTAs that start
+    // where SMs fall free lose the step).  16 and more on one K/V: N=4352 H=3 without a mask 35.1 against 38.5 us, causal
+    // 34.2 / 36.3, N=8192 H=2 59.7 / 64.0; level at 2000 keys, 0 to 5 % either way at 3000.  4 to 15 on one: 1 to 2.5 %
+    // from 7000 keys on, below them the overlap gains 1 to 5 %, as it does at D = 64 everywhere.
+    const int share = p.n_qb * (p.heads / p.heads_kv);
+    const bool in_step = D == 128 && kSingle && !kSplit && p.n_items <= sm_count() &&
+                         p.seq_kv >= (share >= 16 ? 3500 : share >= 4 ? 7000 : INT32_MAX);
+    const bool pdl = env_pdl >= 0 ? env_pdl == 1 : !in_step;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_ctas);
     cfg.blockDim = dim3(384);
