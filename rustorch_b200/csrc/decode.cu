@@ -830,10 +830,13 @@ static cudaError_t launch_decode_d(const DecodeParams& p, int group, int64_t bat
 //    after the others.
 //  * 64 groups and more of at most 256 KB of K and V: also whole.  That is 5 us for one CTA, less than a merge costs.
 //  * Fewer groups: one wave, about slots / groups chunks per sequence.  Per-sequence lengths are only known on the
-//    device.  From 40 MB on (6 us at the HBM rate) and up to 32 sequences, chunks of one size for all of them, so that
-//    every CTA streams equally long (D = 64, 112 groups of 1000 to 4096 tokens: 27 -> 13 us; 8 sequences of 500 to 4000
-//    over 8 KV heads, D = 128: 17.6 -> 14.0 us); the scan of the lengths costs 0.4 us, so smaller launches cut every
-//    sequence into equal parts of its own, or, up to 2048 tokens and for larger batches, at fixed places.
+//    device.  From 40 MB on (6 us at the HBM rate) and up to 32 sequences (a lane each), chunks of one size for all of them,
+//    so that every CTA streams equally long (D = 64, 112 groups of 1000 to 4096 tokens: 27 -> 13 us; 8 sequences of 500 to
+//    4000 over 8 KV heads, D = 128: 17.6 -> 14.0 us); the scan of the lengths costs 0.4 us, so smaller launches, and larger
+//    batches, cut every sequence into equal parts of its own: at fixed places a sequence shorter than the first
+//    leaves all but one CTA idle (33 sequences of 2048 tokens in a cache of 32768, one KV head, D = 128: 30 -> 12 us, of
+//    655 to 9830 at D = 256 128 -> 47; over 1500 shapes of 33 to 128 sequences 0.88 of the time, at worst 1.16 where the
+//    lengths fill the cache).  Up to 2048 tokens at fixed places.
 static DecodeSplit pick_split(int64_t batch, int n_kv, int head_dim, int64_t max_seq, int64_t span, bool ragged) {
     DecodeSplit sp{};
     sp.chunk = decode_chunk_tokens(batch, n_kv, max_seq);
@@ -855,8 +858,8 @@ static DecodeSplit pick_split(int64_t batch, int n_kv, int head_dim, int64_t max
         if (parts > most) parts = most;
         const int64_t want = ((span + parts - 1) / parts + 63) / 64 * 64;
         if (want <= (1 << 20)) sp.chunk = (int)want;
-        if (ragged && batch <= 32 && parts > 1 && !twice && span < (1 << 30)) {
-            if (groups * group_bytes >= (40 << 20)) {
+        if (ragged && parts > 1 && !twice && span < (1 << 30)) {
+            if (batch <= 32 && groups * group_bytes >= (40 << 20)) {
                 const int64_t n = (span + 63) / 64;
                 sp.mode = kSplitShare;
                 // no more of one sequence than if it held all tokens (the merge looks at every one: 35.1 -> 32.8 us at

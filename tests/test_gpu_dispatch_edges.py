@@ -81,6 +81,8 @@ def test_host_entry_staged_equals_pinned(precision, B, H, N):
     (3, 16, 8, 128, 4096, (0, 4096)),     # shares of all tokens, one sequence empty
     (32, 4, 2, 64, 2600, (5, 2600)),      # the same with a full warp of sequences
     (2, 8, 1, 256, 2100, (2050, 2099)),   # equal parts of every sequence
+    (33, 8, 2, 128, 2300, (0, 2300)),     # the same with more sequences than a warp has lanes
+    (37, 4, 4, 64, 2400, (0, 2400)),      # and merged by the CTA that completes a group
     (5, 4, 2, 128, 1000, (63, 65)),       # fixed parts, most of them empty
     (90, 1, 1, 256, 1100, (900, 1100)),   # D = 256: two waves
 ])
