@@ -84,6 +84,7 @@ def test_host_entry_staged_equals_pinned(precision, B, H, N):
     (33, 8, 2, 128, 2300, (0, 2300)),     # the same with more sequences than a warp has lanes
     (37, 4, 4, 64, 2400, (0, 2400)),      # and merged by the CTA that completes a group
     (5, 4, 2, 128, 1000, (63, 65)),       # fixed parts, most of them empty
+    (1, 4, 1, 64, 40000, (39999, 39999)),  # one group: as many parts as its merge is worth
     (90, 1, 1, 256, 1100, (900, 1100)),   # D = 256: two waves
 ])
 def test_decode_splits(oracle, B, Hq, Hkv, D, S, lens):
