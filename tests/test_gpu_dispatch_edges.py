@@ -1,4 +1,5 @@
-"""Sizes at which a branch of a kernel or of a launch rule changes, each against the CPU oracle."""
+"""Sizes at which a branch of a kernel or of a launch rule changes, each against the CPU oracle or, where that would take
+minutes (schedules, sorted keep flags, clusters), against torch in f32 to the same limits."""
 import numpy as np
 import pytest
 
@@ -135,7 +136,7 @@ def test_prefill_schedules(B, H, N, D, causal, part):
     if causal:
         s = s.masked_fill(torch.ones(N, N, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
     ref = torch.softmax(s, -1) @ v[-1].float()
-    assert float((out[-1].float() - ref).norm() / ref.norm()) < 1e-2
+    assert float((out[-1].float() - ref).norm() / ref.norm()) <= util.TOL_REL_L2
     assert torch.allclose(lse[-1], torch.logsumexp(s, -1), rtol=1e-4, atol=1e-3)
 
 
@@ -163,7 +164,7 @@ def test_keep_flags_sorted(B, H, N, Nkv, D, causal):
         dead = torch.isinf(s).all(-1)
         assert torch.equal(torch.isnan(out[b]).all(-1), dead) and torch.equal(lse[b] == float("-inf"), dead)
         x, y = out[b].float()[~dead], ref[~dead]
-        assert float((x - y).norm()) <= 1e-2 * float(y.norm())
+        assert float((x - y).norm()) <= util.TOL_REL_L2 * float(y.norm())
         assert torch.allclose(lse[b][~dead], torch.logsumexp(s, -1)[~dead], rtol=1e-4, atol=1e-3)
 
 
@@ -194,7 +195,7 @@ def test_prefill_clusters(B, Hq, Hkv, Nq, Nkv, D, causal, lens):
         if causal:
             s = s.masked_fill(torch.ones(Nq, lens[b], dtype=torch.bool, device="cuda").triu(int(off[b]) + 1), float("-inf"))
         ref = torch.softmax(s, -1) @ vb
-        assert float((out[b].float() - ref).norm() / ref.norm()) < 1e-2
+        assert float((out[b].float() - ref).norm() / ref.norm()) <= util.TOL_REL_L2
         assert torch.allclose(lse[b], torch.logsumexp(s, -1), rtol=1e-4, atol=1e-3)
 
 
@@ -246,4 +247,4 @@ def test_backward_schedules(B, H, N, D, causal, part):
         w = w.masked_fill(torch.ones(N, N, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
     (torch.softmax(w, -1) @ x[2]).backward(do[-1].float())
     for g, r in zip(grads, x):
-        assert float((g[-1] - r.grad).norm() / r.grad.norm()) < 2e-2
+        assert float((g[-1] - r.grad).norm() / r.grad.norm()) <= 1e-2

@@ -38,6 +38,7 @@ def run_tests_with(var, value, target, select=None, timeout=900):
 
 @pytest.mark.parametrize("var,value,target,select", [
     ("RT_ATTN_DECODE_IMPL", "simt", "test_gpu_decode.py", None),
+    ("RT_ATTN_DECODE_IMPL", "simt", "test_gpu_dispatch_edges.py", "decode_splits"),
     ("RT_ATTN_DECODE_CHUNK", "128", "decode_chunk_cases.py", None),
     ("RT_ATTN_DECODE_FUSED_MERGE", "0", "test_gpu_decode.py", None),
     ("RT_ATTN_DECODE_PUSH_IN_KERNEL", "1", "test_gpu_decode.py", "exchange or push or peer or record"),
