@@ -86,7 +86,7 @@ const char* rt_attn_error_string(int status);
 
 /*
  * Reads (and clears) the device-side status word of the current device: 0 = clean,
- * otherwise a code identifying which bounded wait inside a kernel gave up (101-113: a barrier of
+ * otherwise a code identifying which bounded wait inside a kernel gave up (101-114: a barrier of
  * the prefill kernel, 301: a TMA stage of the decode kernel, 401: a peer's record in
  * rt_attn_merge_records_after).  Synchronises the device.  Returns RT_OK, a cudaError_t, or RT_ERR_DEVICE_TIMEOUT when *status != 0.
  */

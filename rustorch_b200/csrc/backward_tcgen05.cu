@@ -377,8 +377,7 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
             const uint32_t t1 = tT + buf * 128, t2 = t1 + 64;
             const float2 c2 = make_float2(c, c);
             {
-                constexpr int ch = 0;  // this thread's single chunk: score columns [32 half, 32 half + 32) of the step
-                const int cbase = half * 32;
+                const int cbase = half * 32;  // this thread's score columns of the step: [32 half, 32 half + 32)
                 uint32_t a1[32], a2[32];
                 tmem_ld32(t1 + cbase, a1);
                 tmem_ld32(t2 + cbase, a2);
@@ -423,7 +422,6 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
                     pk_ds[i / 2 + 1] = float2_to_bf16x2(db.x, db.y);
                 }
                 // the 32 bf16 values go into the first 16 of this thread's own 32 columns (in registers by now)
-                (void)ch;
                 if (kKeySide) tmem_st16(t1 + cbase, pk_p);
                 tmem_st16(t2 + cbase, pk_ds);
             }

@@ -1,12 +1,14 @@
 // f32 flash-attention forward on CUDA cores, plus the f32 <-> bf16 conversion kernels.
 //
-// This is the exact-arithmetic companion of the tensor-core kernel: f32 inputs, f32
-// accumulation, accurate expf, any head dim up to 256, seq_q != seq_kv and grouped KV heads.
-// It backs the host mirrors of flash_forward_masked (crates/rustorch-attention/src/cpu_forward.rs:193-242)
+// The exact-arithmetic companions of the tensor-core kernel: f32 inputs, f32
+// accumulation, CUDA's exponentials, any head dim up to 256, seq_q != seq_kv and grouped KV heads.
+// They back the host mirrors of flash_forward_masked (crates/rustorch-attention/src/cpu_forward.rs:193-242)
 // and gqa_forward_f32 (crates/rustorch-nn/src/gqa.rs:94-210) at the reference's own 1e-4
-// tolerance.  One warp owns one query row and walks the keys in tiles of 32 staged in shared
-// memory; the online-softmax recurrence is the reference's (cpu_forward.rs:355-386) with the
+// tolerance.  The online-softmax recurrence is the reference's (cpu_forward.rs:355-386) with the
 // leading-masked-tile case resolved to the finite answer.
+//   prefill_f32_tiled_kernel  16 query rows and more: 64 rows per CTA, register tiles, exp2f (simt_tile.cuh)
+//   prefill_f32_kernel        fewer rows: one warp owns one query row and walks the keys in tiles of 32 staged in
+//                             shared memory, expf
 #include <cstdlib>
 
 #include "common.cuh"

@@ -116,7 +116,6 @@ __device__ __forceinline__ float2 exp2_poly2(float2 x) {
     y.y = __int_as_float(__float_as_int(y.y) + (__float_as_int(t.y) << 23));
     return y;
 }
-// Which of the 16 element pairs of a 32-column chunk take the polynomial path.
 // Which of the 16 element pairs of a 32-column chunk take the polynomial path (a quarter: more
 // than that costs more issue slots on the FMA pipe than it frees on the MUFU pipe).
 __host__ __device__ constexpr bool poly_pair(int q) { return (q & 3) == 3; }
