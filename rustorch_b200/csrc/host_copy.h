@@ -11,7 +11,8 @@
 // workers convert as they copy, which halves what crosses the link.  Pinned host memory skips the ring.
 //
 // The workers and the ring (16 MB up, 8 MB down) are made by the first call that needs them, serve one call at a time
-// (the entry points hold a lock) and are given back when the library is unloaded.
+// (the entry points hold a lock) and are given back when the library is unloaded.  The workers sleep while there is
+// nothing to copy; the calling thread polls until the call ends, as in any blocking CUDA call.
 #pragma once
 #include <cuda_runtime.h>
 #if defined(__x86_64__)
