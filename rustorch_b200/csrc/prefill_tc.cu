@@ -343,7 +343,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     uint64_t* v_empty = v_full + VS;      // [2 tiles][VS]
     uint64_t* s_full = v_empty + 2 * VS;  // [2 tiles][2 buffers]
     uint64_t* p_full = s_full + 4;        // [2 tiles][2 buffers]
-    uint64_t* o_full = p_full + 4;        // [2]  one phase per PV step (O at rest for a rescale)
+    uint64_t* o_full = p_full + 4;        // [2]  one phase per item of two steps or more: its last PV but one has retired
     uint64_t* o_done = o_full + 2;        // [2]  one phase per item: the last PV of the tile has retired
     uint64_t* o_free = o_done + 2;        // [2]  one phase per item: the epilogue has read O out of TMEM
     uint64_t* stage_full = o_free + 2;    // [2]  one phase per item: the O tile is staged in shared memory
@@ -628,110 +628,155 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             const uint32_t tS = tmem_base + C::COL_S + w * 128, tO = tmem_base + C::COL_O + w * D;
             uint64_t* const ke = k_empty + w * KS;
             uint64_t* const ve = v_empty + w * VS;
-            int kg = 0, vg = 0;    // ring index of the item's first K / V tile
-            int na = 0;            // items so far in which this tile took part
-            int cp0 = 0, cp1 = 0;  // p_full phases of each S buffer consumed before the item
-            auto commit = [&](uint64_t* bar) {
-                if (leader) mma_commit(bar);
-            };
+            uint64_t* const sf = s_full + w * 2;
+            uint64_t* const pf = p_full + w * 2;
+            // Ring slots and phases are carried along: every instruction between a P that has arrived and the score MMA
+            // behind its PV is on the critical path of the softmax warps, and so is whatever this loop does instead of
+            // looking for the next P.
+            uint32_t ks = 0, kph = 0, vs = 0, vph = 0;  // slot and phase of the next K / V tile
+            uint32_t p0 = 0, p1 = 0;                    // phase of the next P in each score buffer
+            uint32_t na = 0;                            // items so far in which this tile took part
             auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
                 return __all_sync(kFullMask, mbar_wait(bar, parity, p.status, code));
             };
+            auto next_k = [&] {
+                if (++ks == KS) ks = 0, kph ^= 1;
+            };
+            auto next_v = [&] {
+                if (++vs == VS) vs = 0, vph ^= 1;
+            };
+            // (called by the elected lane)
+            auto issue_S = [&](int b, uint64_t bk) {
+#pragma unroll
+                for (int kk = 0; kk < D / 16; ++kk) {
+                    const uint32_t off = (uint32_t)(((kk / 4) * SUB + (kk % 4) * 32) >> 4);
+                    mma_ss(tS + b * 64, dq + off, bk + off, idesc_s, kk > 0);
+                }
+                mma_commit(&sf[b]);
+            };
+            auto issue_PV = [&](int b, uint64_t bv, uint32_t acc) {  // P (bf16) sits in the first 32 columns of the score buffer
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    mma_ts(tO, tS + b * 64 + kk * 8, bv + (uint64_t)((kk * 2048) >> 4), idesc_o, kk > 0 ? 1u : acc);
+            };
+            constexpr uint32_t kTileEnc = TILE >> 4, kHalfEnc = HALF >> 4;
             bool ok = true;
             for (int j = 0; ok; ++j) {
                 const TcItem it = tc_item<kCausal, kSingle, kByLength>(j, p, sched, keep_hi);
                 if (it.end) break;
                 if (!it.valid || it.n_tiles == 0) continue;
                 const int n_u = it.steps(w);
-                // Step u of this tile reads half half_of(u) (64 rows) of the item's K/V tile tile_of(u): the
-                // tile's own steps are consecutive 64-key steps, or (single-tile items) every second one.
-                constexpr bool il = kSingle;
-                auto tile_of = [&](int u) { return il ? u : (u >> 1); };
-                auto half_of = [&](int u) { return il ? w : (u & 1); };
-                auto issue_S = [&](int u) {
-                    const uint64_t bk = dk + (uint64_t)((((kg + tile_of(u)) % KS) * TILE + half_of(u) * HALF) >> 4);
-                    const uint32_t d = tS + (u & 1) * 64;
-#pragma unroll
-                    for (int kk = 0; kk < D / 16; ++kk) {
-                        const uint32_t off = (uint32_t)(((kk / 4) * SUB + (kk % 4) * 32) >> 4);
-                        if (leader) mma_ss(d, dq + off, bk + off, idesc_s, kk > 0);
-                    }
-                };
-                // O_w += P V(u): P (bf16) sits in the first 32 columns of S[w][u&1]
-                auto issue_PV = [&](int u) {
-                    const uint64_t bv = dv + (uint64_t)((((vg + tile_of(u)) % VS) * TILE + half_of(u) * HALF) >> 4);
-                    const uint32_t a = tS + (u & 1) * 64;
-                    const uint32_t acc0 = u > 0 ? 1u : 0u;
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        if (leader)
-                            mma_ts(tO, a + kk * 8, bv + (uint64_t)((kk * 2048) >> 4), idesc_o, kk > 0 ? 1u : acc0);
-                };
-                auto last_use = [&](int u) { return il || (u & 1) || u == n_u - 1; };  // of a 128-key tile, by this Q tile
-
-                if (n_u > 0) {
-                    ok = wait(&k_full[kg % KS], (uint32_t)(kg / KS) & 1u, kToKFull) &&
-                         wait(&q_full[il ? 1 : w], (uint32_t)na & 1u, kToQ);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_S(0);
-                    commit(&s_full[w * 2]);
-                    int k_waited = 0, v_waited = -1;  // item-local tile indices already waited for
-                    if (il) commit(&ke[kg % KS]);
-                    if (n_u > 1) {
-                        if (il) {  // the second step reads the next K tile
-                            if (!wait(&k_full[(kg + 1) % KS], (uint32_t)((kg + 1) / KS) & 1u, kToKFull)) { ok = false; break; }
-                            k_waited = 1;
-                            tc_fence_after();
-                        }
-                        issue_S(1);
-                        commit(&s_full[w * 2 + 1]);
-                        if (il) commit(&ke[(kg + 1) % KS]);
-                    }
-                    if (!il) commit(&ke[kg % KS]);
-                    for (int u = 0; u < n_u && ok; ++u) {
-                        const int vt = tile_of(u);
-                        if (vt > v_waited) {
-                            if (!wait(&v_full[(vg + vt) % VS], (uint32_t)((vg + vt) / VS) & 1u, kToVFull)) { ok = false; break; }
-                            v_waited = vt;
-                        }
-                        if (!wait(&p_full[w * 2 + (u & 1)], (uint32_t)(((u & 1) ? cp1 : cp0) + (u >> 1)) & 1u, kToPFull)) { ok = false; break; }
-                        // the previous item's epilogue must have read O_w before it is overwritten
-                        if (u == 0 && na > 0 && !wait(&o_free[w], (uint32_t)(na - 1) & 1u, kToOFree)) { ok = false; break; }
+                if (kSingle) {
+                    // ---- the tile's steps are every second 64-key step: half w of every K/V tile
+                    const uint64_t bk0 = dk + w * kHalfEnc, bv0 = dv + w * kHalfEnc;
+                    if (n_u > 0) {
+                        ok = wait(&k_full[ks], kph, kToKFull) && wait(&q_full[1], na & 1u, kToQ);
+                        if (!ok) break;
                         tc_fence_after();
-                        issue_PV(u);
-                        commit(&o_full[w]);
-                        if (u == n_u - 1) commit(&o_done[w]);
-                        if (last_use(u)) commit(&ve[(vg + vt) % VS]);
-                        if (u + 2 < n_u) {
-                            const int kt = tile_of(u + 2);
-                            if (kt > k_waited) {
-                                if (!wait(&k_full[(kg + kt) % KS], (uint32_t)((kg + kt) / KS) & 1u, kToKFull)) { ok = false; break; }
-                                k_waited = kt;
-                                tc_fence_after();
-                            }
-                            issue_S(u + 2);
-                            commit(&s_full[w * 2 + (u & 1)]);
-                            if (last_use(u + 2)) commit(&ke[(kg + kt) % KS]);
+                        if (leader) {
+                            issue_S(0, bk0 + ks * kTileEnc);
+                            mma_commit(&ke[ks]);
                         }
+                        next_k();
+                        if (n_u > 1) {
+                            if (!wait(&k_full[ks], kph, kToKFull)) { ok = false; break; }
+                            tc_fence_after();
+                            if (leader) {
+                                issue_S(1, bk0 + ks * kTileEnc);
+                                mma_commit(&ke[ks]);
+                            }
+                            next_k();
+                        }
+                        for (int u = 0; u < n_u && ok; u += 2) {
+#pragma unroll
+                            for (int b = 0; b < 2; ++b) {
+                                if (b == 1 && u + 1 >= n_u) break;
+                                const bool more = u + b + 2 < n_u;
+                                ok = wait(&v_full[vs], vph, kToVFull) && (!more || wait(&k_full[ks], kph, kToKFull)) &&
+                                     wait(&pf[b], b ? p1 : p0, kToPFull);
+                                if (!ok) break;
+                                (b ? p1 : p0) ^= 1;
+                                tc_fence_after();
+                                if (leader) {
+                                    issue_PV(b, bv0 + vs * kTileEnc, (u + b > 0) ? 1u : 0u);
+                                    if (more) {
+                                        issue_S(b, bk0 + ks * kTileEnc);
+                                        mma_commit(&ke[ks]);
+                                    }
+                                    mma_commit(&ve[vs]);
+                                    if (u + b == n_u - 2) mma_commit(&o_full[w]);
+                                    if (u + b == n_u - 1) mma_commit(&o_done[w]);
+                                }
+                                next_v();
+                                if (more) next_k();
+                            }
+                        }
+                        ++na;
                     }
-                    ++na;
-                    cp0 += (n_u + 1) / 2;
-                    cp1 += n_u / 2;
+                } else {
+                    // ---- steps 2t and 2t + 1 read the halves of K/V tile t and use score buffers 0 and 1
+                    if (n_u > 0) {
+                        ok = wait(&k_full[ks], kph, kToKFull) && wait(&q_full[w], na & 1u, kToQ);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (leader) {
+                            const uint64_t bk = dk + ks * kTileEnc;
+                            issue_S(0, bk);
+                            if (n_u > 1) issue_S(1, bk + kHalfEnc);
+                            mma_commit(&ke[ks]);
+                        }
+                        next_k();
+                    }
+                    for (int u = 0; u < n_u; u += 2) {
+                        const bool more = u + 2 < n_u;
+                        ok = wait(&v_full[vs], vph, kToVFull) && (!more || wait(&k_full[ks], kph, kToKFull)) &&
+                             // the previous item's epilogue must have read O_w before it is overwritten
+                             (u > 0 || na == 0 || wait(&o_free[w], (na - 1) & 1u, kToOFree)) && wait(&pf[0], p0, kToPFull);
+                        if (!ok) break;
+                        p0 ^= 1;
+                        const uint64_t bk = dk + ks * kTileEnc, bv = dv + vs * kTileEnc;
+                        tc_fence_after();
+                        if (leader) {
+                            issue_PV(0, bv, u > 0 ? 1u : 0u);
+                            if (more) issue_S(0, bk);
+                            if (u + 2 == n_u) mma_commit(&o_full[w]);
+                        }
+                        if (u + 1 < n_u) {
+                            ok = wait(&pf[1], p1, kToPFull);
+                            if (!ok) break;
+                            p1 ^= 1;
+                            tc_fence_after();
+                            if (leader) {
+                                issue_PV(1, bv + kHalfEnc, 1u);
+                                if (u + 3 < n_u) issue_S(1, bk + kHalfEnc);
+                                if (u + 3 == n_u) mma_commit(&o_full[w]);
+                            }
+                        }
+                        if (leader) {
+                            if (more) mma_commit(&ke[ks]);
+                            else mma_commit(&o_done[w]);
+                            mma_commit(&ve[vs]);
+                        }
+                        next_v();
+                        if (more) next_k();
+                    }
+                    if (n_u > 0) ++na;
                 }
+                if (!ok) break;
                 // Tiles this Q tile does not read (it sees fewer keys than the other one) are passed on
                 // once they have landed, which keeps this issuer inside the ring window.
-                for (int t = il ? n_u : (n_u + 1) / 2; t < it.n_tiles && ok; ++t) {
-                    ok = wait(&k_full[(kg + t) % KS], (uint32_t)((kg + t) / KS) & 1u, kToKFull);
-                    if (ok) commit(&ke[(kg + t) % KS]);
-                    ok = ok && wait(&v_full[(vg + t) % VS], (uint32_t)((vg + t) / VS) & 1u, kToVFull);
-                    if (ok) commit(&ve[(vg + t) % VS]);
+                for (int t = kSingle ? n_u : (n_u + 1) / 2; t < it.n_tiles && ok; ++t) {
+                    ok = wait(&k_full[ks], kph, kToKFull) && wait(&v_full[vs], vph, kToVFull);
+                    if (ok && leader) {
+                        mma_commit(&ke[ks]);
+                        mma_commit(&ve[vs]);
+                    }
+                    next_k();
+                    next_v();
                 }
-                kg += it.n_tiles;
-                vg += it.n_tiles;
             }
             // All MMAs of both issuers must retire before TMEM is freed.
-            commit(done_bar);
+            if (leader) mma_commit(done_bar);
             wait(done_bar, 0, kToDone);
         }
       }  // warp 11 idle: it only completes the warpgroup for setmaxnreg
@@ -751,7 +796,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         const float c = p.scale_log2;
         int na = 0;            // items so far in which this tile took part
         int cs0 = 0, cs1 = 0;  // s_full phases of each S buffer consumed before the item
-        int co = 0;            // PV steps of this tile before the item (phase of o_full)
+        int co = 0;            // items of two steps or more before this one (phase of o_full)
         bool ok = true;
 
         for (int j = 0; ok; ++j) {
@@ -851,10 +896,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 } else {
                     const bool need = (mx > m_ref) && ((mx - m_ref) * c > 8.0f || m_ref == -INFINITY);
                     if (__any_sync(kFullMask, need)) {
-                        // O must be at rest: the PV of the previous step has to be complete.  (The score
-                        // MMA just waited for was issued after the PV before that one, so the barrier is
-                        // at most one phase behind and the parity wait is unambiguous.)
-                        if (!__all_sync(kFullMask, mbar_wait(&o_full[w], (uint32_t)(co + u - 1) & 1u, p.status, kToOFull))) {
+                        // O must be at rest: the PV of step u - 1 has to be complete.  The scores of step u + 1 were
+                        // requested right behind it; the last step has a barrier of its own for this.
+                        const bool at_rest = u + 1 < n_iter
+                            ? mbar_wait(&s_full[w * 2 + 1 - buf], (uint32_t)((buf ? cs0 : cs1) + ((u + 1) >> 1)) & 1u, p.status, kToOFull)
+                            : mbar_wait(&o_full[w], (uint32_t)co & 1u, p.status, kToOFull);
+                        if (!__all_sync(kFullMask, at_rest)) {
                             ok = false;
                             break;
                         }
@@ -1054,7 +1101,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             ++na;
             cs0 += (n_iter + 1) / 2;
             cs1 += n_iter / 2;
-            co += n_iter;
+            co += n_iter > 1 ? 1 : 0;
         }
         if constexpr (kSplit) {
             // ---- the cluster's partial rows: CTA r reads its 128 / split rows from every CTA's shared memory, merges them
