@@ -794,6 +794,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         const uint32_t tS = tmem_base + lane_sel + C::COL_S + w * 128;
         const uint32_t tO = tmem_base + lane_sel + C::COL_O + w * D;
         const float c = p.scale_log2;
+        const float grow = c > 0.f ? fminf(8.f / c, 3.0e38f) : 3.0e38f;  // raw scores that a factor of 2^8 stands for
         int na = 0;            // items so far in which this tile took part
         int cs0 = 0, cs1 = 0;  // s_full phases of each S buffer consumed before the item
         int co = 0;            // items of two steps or more before this one (phase of o_full)
@@ -822,9 +823,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 continue;
             }
 
-            float m_ref = -INFINITY;  // reference max (raw score units) the running sums are relative to
+            float m_ref = -INFINITY;  // reference max (raw score units) the running sums are relative to; -inf: no score was visible yet
             float l = 0.f;
-            bool seen = false;  // the row has met a score that no mask hides
             for (int u = 0; u < n_iter; ++u) {
                 const int buf = u & 1;
                 const int col0 = (il ? 2 * (it.t0 + u) + w : u) * 64;
@@ -838,11 +838,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     keep0 = __ballot_sync(kFullMask, f0);
                     keep1 = __ballot_sync(kFullMask, f1);
                 }
-                if (!__all_sync(kFullMask, mbar_wait(&s_full[w * 2 + buf], (uint32_t)((buf ? cs1 : cs0) + (u >> 1)) & 1u,
-                                                     p.status, kToSFull))) {
-                    ok = false;
-                    break;
-                }
+                // (No vote on the outcome: a wait that gives up clears the thread's `ok`, which the vote below sees.)
+                ok &= mbar_wait(&s_full[w * 2 + buf], (uint32_t)((buf ? cs1 : cs0) + (u >> 1)) & 1u, p.status, kToSFull);
                 tc_fence_after();
                 if (il && w == 1 && u == 0 && p.stagger_clocks > 0) {
                     // The two tiles of a single-tile item start together and would stay in step: both
@@ -888,28 +885,24 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     mx3 = max3(mx3, __uint_as_float(s[i + 6]), __uint_as_float(s[i + 7]));
                 }
                 const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-                seen = seen || (mx > -INFINITY);
 
                 // ---- lazy rescale: move the reference max only when it would grow by > 2^8
-                if (u == 0) {
-                    m_ref = mx;
-                } else {
-                    const bool need = (mx > m_ref) && ((mx - m_ref) * c > 8.0f || m_ref == -INFINITY);
-                    if (__any_sync(kFullMask, need)) {
+                if (__any_sync(kFullMask, mx > m_ref + grow || !ok)) {
+                    if (u > 0) {
                         // O must be at rest: the PV of step u - 1 has to be complete.  The scores of step u + 1 were
                         // requested right behind it; the last step has a barrier of its own for this.
-                        const bool at_rest = u + 1 < n_iter
+                        ok &= u + 1 < n_iter
                             ? mbar_wait(&s_full[w * 2 + 1 - buf], (uint32_t)((buf ? cs0 : cs1) + ((u + 1) >> 1)) & 1u, p.status, kToOFull)
                             : mbar_wait(&o_full[w], (uint32_t)co & 1u, p.status, kToOFull);
-                        if (!__all_sync(kFullMask, at_rest)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const float m_new = fmaxf(m_ref, mx);
-                        const float alpha = (m_new == -INFINITY) ? 1.f : fast_exp2((m_ref - m_new) * c);
-                        l *= alpha;
-                        m_ref = m_new;
+                    }
+                    ok = __all_sync(kFullMask, ok);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const float m_new = fmaxf(m_ref, mx);
+                    const float alpha = (m_new == -INFINITY) ? 1.f : fast_exp2((m_ref - m_new) * c);
+                    l *= alpha;
+                    m_ref = m_new;
+                    if (u > 0) {
 #pragma unroll
                         for (int ch = 0; ch < D / 32; ++ch) {
                             uint32_t o[32];
@@ -953,7 +946,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 tc_fence_before();
                 mbar_arrive(&p_full[w * 2 + buf]);
             }
+            ok = __all_sync(kFullMask, ok);
             if (!ok) break;
+            const bool seen = m_ref > -INFINITY;  // the row has met a score that no mask hides
 
             // ---- epilogue: O / l -> bf16 into the (now idle) shared-memory tile of Q_w in the swizzled
             // layout of the output tensor map, then one TMA store per 64-column half: 16-byte shared
