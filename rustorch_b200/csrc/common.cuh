@@ -54,11 +54,12 @@ __device__ __forceinline__ float fast_log2(float x) {
 }
 
 // How a decode launch cuts its sequences into chunks, one CTA each; see pick_split for the rule.
-enum { kSplitFixed = 0, kSplitEven, kSplitShare };
+enum { kSplitFixed = 0, kSplitEven, kSplitShare, kSplitCluster };
 struct DecodeSplit {
     int n_chunks;  // chunks of a sequence at most
     int chunk;     // kSplitFixed: tokens per chunk (grid: chunk, KV head, sequence)
     int mode;      // kSplitEven: n_chunks equal parts of every sequence's own length (same grid)
+                   // kSplitCluster: the same parts, merged by the cluster of n_chunks CTAs that streams them (no partials)
                    // kSplitShare: chunks of one size for all `batch` <= 32 sequences, about `target` of them in all,
     int batch;     //              dealt to a flat grid of `ctas` CTAs
     int ctas;

@@ -839,6 +839,7 @@ static cudaError_t launch_decode_d(const DecodeParams& p, int group, int64_t bat
 //    lengths fill the cache).  Up to 2048 tokens at fixed places.
 static DecodeSplit pick_split(int64_t batch, int n_kv, int head_dim, int64_t max_seq, int64_t span, bool ragged) {
     DecodeSplit sp{};
+
     sp.chunk = decode_chunk_tokens(batch, n_kv, max_seq);
     const int64_t groups = batch * (int64_t)n_kv, slots = (int64_t)sm_count() * (head_dim == 64 ? 4 : head_dim == 128 ? 2 : 1);
     const int64_t whole = (span + 63) / 64 * 64, group_bytes = span * head_dim * 4;
@@ -882,6 +883,42 @@ static DecodeSplit pick_split(int64_t batch, int n_kv, int head_dim, int64_t max
     return sp;
 }
 
+// kSplitCluster: a cluster of 2, 4, 8 or 16 CTAs streams a sequence and merges its parts through distributed shared memory, in
+// one launch without partials in global memory.  It saves the merge launch, 2.2 us on the device and 2.5 us of the host,
+// but its CTAs are fewer: all clusters must be resident at once, and a GPC holds whole ones only.  Estimates in us of what
+// sets the forms apart decide: a CTA streams its part at 35, 53 or 68 GB/s by head dim, a cluster launch takes longer to
+// start the more CTAs it has, a single CTA per sequence needs no merge at all, shares of all tokens balance unequal
+// lengths.  Lengths that only the device knows are taken as two thirds of the cache.
+// (Graph replays, caches out of HBM, 664 shapes of 2 to 128 groups and 130 to 9500 tokens, lengths an eighth to all of the
+// longest: 0.83 of the time of the other forms, at worst 1.07; the estimates miss the fastest form by 2 % on average.
+// 8 groups of 1000 tokens D = 64 6.2 -> 4.0 us, D = 128 6.1 -> 4.4, D = 256 8.5 -> 6.7; 64 groups of up to 1000 tokens D = 64
+// 11.9 -> 6.8; one sequence of 9500 tokens, 2 KV heads, D = 256 12.8 -> 14.9 and left alone.)
+static void pick_cluster(DecodeSplit& sp, int64_t groups, int head_dim, int64_t span, bool ragged, int64_t parts) {
+    // RT_ATTN_DECODE_CLUSTER=0 never takes clusters, nor do the overrides that choose how partials are merged;
+    // =2|4|8|16 takes that size wherever it fits (read once per process).
+    static const int env = [] {
+        const char* e = getenv("RT_ATTN_DECODE_CLUSTER");
+        if (e) return atoi(e);
+        auto is = [](const char* name, char c) {
+            const char* v = getenv(name);
+            return v && v[0] == c;
+        };
+        return is("RT_ATTN_DECODE_FUSED_MERGE", '0') || is("RT_ATTN_DECODE_PUSH_IN_KERNEL", '1') || is("RT_ATTN_MERGE_PDL", '0') ? 0 : -1;
+    }();
+    if (env == 0 || forced_chunk() || span <= 64 || span > (1 << 20)) return;
+    const double stream = (head_dim == 64 ? 0.0072 : head_dim == 128 ? 0.0096 : 0.015) * (ragged ? 0.67 : 1.0) * (double)span;
+    double best = sp.n_chunks <= 1 ? 1.15 * stream - 1.5 : stream / ((double)parts * (sp.mode == kSplitShare ? 1.25 : 1.0)) + 3.4;
+    for (int size = 2; size <= 16; size *= 2) {
+        if (env > 0 && size != env) continue;
+        const double t = stream / size + 0.004 * (double)(groups * size);
+        if ((t < best || env > 0) && groups * size <= decode_cluster_slots(head_dim, size)) {
+            best = t;
+            sp.mode = kSplitCluster;
+            sp.n_chunks = size;
+        }
+    }
+}
+
 cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void* out_bf16, float* out_f32,
                               float* lse, int64_t batch, int n_heads, int n_kv, int head_dim,
                               int64_t max_seq, const int32_t* kv_lens, int64_t kv_len_uniform,
@@ -908,7 +945,12 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
     if (!kv_lens && kv_len_uniform - kv_begin < span) span = kv_len_uniform - kv_begin;
     if (kv_end >= 0 && kv_end - kv_begin < span) span = kv_end - kv_begin;
     if (span < 1) span = 1;
+    const bool tc = decode_use_tensor_cores() && batch * n_kv * max_seq < (1ll << 31) - 64;
     p.split = pick_split(batch, n_kv, head_dim, max_seq, span, kv_lens != nullptr);
+    if (tc) {
+        const int64_t groups = batch * n_kv, slots = (int64_t)sm_count() * (head_dim == 64 ? 4 : head_dim == 128 ? 2 : 1);
+        pick_cluster(p.split, groups, head_dim, span, kv_lens != nullptr && batch > 1, std::max<int64_t>(1, slots / groups));
+    }
     p.rows = batch * n_heads;
     p.of_stride = of_stride > 0 ? of_stride : head_dim;
     p.lse_stride = lse_stride > 0 ? lse_stride : 1;
@@ -922,7 +964,7 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
     bool merged = false;
     if (tail) {  // the caller merges the chunk partials itself (split-KV row exchange)
         counters = nullptr;
-        tail->n_chunks = p.split.n_chunks;
+        tail->n_chunks = p.split.mode == kSplitCluster ? 1 : p.split.n_chunks;  // (a cluster writes the merged rows)
         tail->part_o = p.part_o;
         tail->part_lse = p.part_lse;
     }
@@ -940,7 +982,7 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
         }
     }
     if (e != cudaSuccess) return e;
-    if (merged && push && push->world > 0 && pushed) *pushed = true;  // delivered by the decode kernel itself
+    if (merged && p.split.mode != kSplitCluster && push && push->world > 0 && pushed) *pushed = true;  // delivered by the decode kernel itself
     if (p.split.n_chunks > 1 && !merged && !tail) {
         e = launch_merge_partials(p.part_o, p.part_lse, p.split.n_chunks, p.rows, head_dim, head_dim, 1, p.out_bf16, p.out_f32, lse,
                                   stream, nullptr, push, p.of_stride, p.lse_stride);

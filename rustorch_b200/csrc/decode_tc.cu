@@ -14,10 +14,13 @@
 //     (warp-uniformly) when no row maximum moved.
 // One CTA = 4 independent warps = one (sequence, KV head, chunk); warp states are merged through
 // shared memory and written as a normalised (O f32, LSE) partial, or as the final output when
-// the launch has a single chunk.  Rows past the visible range are masked in the scores and
+// the launch has a single chunk.  With kCluster > 0 the sequence's CTAs are a cluster that merges its partial rows
+// through distributed shared memory (merge_decode_cluster; which launches: pick_cluster in decode.cu).  Rows past the visible range are masked in the scores and
 // zeroed in V (uninitialised cache memory may hold NaN bit patterns).  Waits are bounded.
+#include <atomic>
 #include <cuda.h>
 #include <cstdlib>
+#include <type_traits>
 
 #include "kernels.h"
 #include "mma_sync.cuh"
@@ -240,7 +243,58 @@ struct DecodeTcCfg {
 
 enum { kToDecFull = 301 };
 
-template <int D, int G, bool kShare>
+__device__ __forceinline__ void decode_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t decode_map_cluster(uint32_t a, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+
+// The end of a sequence that a cluster of C CTAs has streamed: CTA r merges the rows' float4 columns
+// [r, r + 1) * G * D / (4 C) out of the partial rows (`part`, [G][D], relative to its maximum) and (max, sum) pairs (`ml`,
+// [G]) in all C shared memories.  All of a thread's remote loads are in flight together.
+template <int D, int G, int C>
+__device__ __forceinline__ void merge_decode_cluster(const DecodeTcParams& p, int64_t row0, uint32_t part, uint32_t ml, int rank) {
+    constexpr int kVec = G * D / (4 * C);
+    static_assert(kVec >= 1, "a float4 column per CTA at least");
+    decode_cluster_sync();
+    for (int i = threadIdx.x; i < kVec; i += 128) {
+        const int f = rank * kVec + i, gg = f / (D / 4), d = f % (D / 4) * 4;
+        float2 s[C];
+        float4 v[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(s[c].x), "=f"(s[c].y) : "r"(decode_map_cluster(ml + gg * 8, c)) : "memory");
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[c].x), "=f"(v[c].y), "=f"(v[c].z), "=f"(v[c].w) : "r"(decode_map_cluster(part + f * 16, c)) : "memory");
+        }
+        float m = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int c = 0; c < C; ++c) m = fmaxf(m, s[c].x);
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (s[c].x > -INFINITY) {  // (an empty part's rows were never written)
+                const float w = fast_exp2(s[c].x - m);
+                l += w * s[c].y;
+                o = make_float4(fmaf(w, v[c].x, o.x), fmaf(w, v[c].y, o.y), fmaf(w, v[c].z, o.z), fmaf(w, v[c].w, o.w));
+            }
+        const bool any = l > 0.f;
+        o = any ? make_float4(o.x / l, o.y / l, o.z / l, o.w / l) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int64_t row = row0 + gg;
+        if (p.out_bf16) *reinterpret_cast<uint2*>(p.out_bf16 + row * D + d) = make_uint2(float2_to_bf16x2(o.x, o.y), float2_to_bf16x2(o.z, o.w));
+        if (p.out_f32) {
+            float* dst = p.out_f32 + row * p.of_stride + d;  // (records: rows of D + 1 floats)
+            dst[0] = o.x, dst[1] = o.y, dst[2] = o.z, dst[3] = o.w;
+        }
+        if (d == 0 && p.lse) p.lse[row * p.lse_stride] = any ? (m + fast_log2(l)) * kLn2 : -INFINITY;
+    }
+    decode_cluster_sync();  // no CTA leaves while its partial rows are being read
+}
+
+template <int D, int G, bool kShare, int kCluster>
 __global__ void __launch_bounds__(128, 2)
 gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                      const DecodeTcParams p) {
@@ -277,6 +331,12 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
 
     if (c0 >= c1) {  // nothing visible in this chunk: identity partial
         launch_dependents();
+        if constexpr (kCluster > 0) {
+            float* ml = reinterpret_cast<float*>(smem) + NW * G * D + 2 * NW * G + G * D;
+            if (tid < G) ml[2 * tid] = -INFINITY, ml[2 * tid + 1] = 0.f;
+            merge_decode_cluster<D, G, kCluster>(p, row0, smem_u32(reinterpret_cast<float*>(smem) + NW * G * D + 2 * NW * G), smem_u32(ml), chunk_idx);
+            return;
+        }
         if (direct) {
             for (int i = tid; i < G * D; i += 128) {
                 const int64_t o = (row0 + i / D) * D + i % D;
@@ -483,6 +543,11 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
                 acc += w * sm_o[(x * G + gg) * D + d];
             }
         }
+        if constexpr (kCluster > 0) {
+            sm_l[NW * G + i] = acc;
+            if (d == 0) sm_l[NW * G + G * D + 2 * gg] = m, sm_l[NW * G + G * D + 2 * gg + 1] = l;
+            continue;
+        }
         const float outv = (l > 0.f) ? acc / l : 0.f;
         const float lse = (l > 0.f) ? (m + fast_log2(l)) * kLn2 : -INFINITY;
         const int64_t row = row0 + gg;
@@ -494,6 +559,10 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
             p.part_o[((int64_t)chunk_idx * p.rows + row) * D + d] = outv;
             if (d == 0) p.part_lse[(int64_t)chunk_idx * p.rows + row] = lse;
         }
+    }
+    if constexpr (kCluster > 0) {
+        merge_decode_cluster<D, G, kCluster>(p, row0, smem_u32(sm_l + NW * G), smem_u32(sm_l + NW * G + G * D), chunk_idx);
+        return;
     }
     if (!direct && p.counters) {
         __syncthreads();  // the warp-merge scratch at the start of the ring is free again
@@ -509,12 +578,16 @@ static bool make_cache_map(CUtensorMap* map, const void* base, int64_t rows, int
     return encode_bf16_map_cached(map, 2, base, dims, strides, box);
 }
 
-template <int D, int G, bool kShare>
+template <int D, int G, bool kShare, int kCluster>
 static cudaError_t launch_dgs(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeTcParams& p, int64_t batch,
                              cudaStream_t stream) {
-    auto kern = gqa_decode_tc_kernel<D, G, kShare>;
-    cudaError_t e = set_max_dynamic_smem_once<gqa_decode_tc_kernel<D, G, kShare>>(DecodeTcCfg<D>::SMEM_BYTES);
+    auto kern = gqa_decode_tc_kernel<D, G, kShare, kCluster>;
+    cudaError_t e = set_max_dynamic_smem_once<gqa_decode_tc_kernel<D, G, kShare, kCluster>>(DecodeTcCfg<D>::SMEM_BYTES);
     if (e != cudaSuccess) return e;
+    if constexpr (kCluster > 8) {  // beyond the portable size
+        e = allow_large_cluster_once<gqa_decode_tc_kernel<D, G, kShare, kCluster>>();
+        if (e != cudaSuccess) return e;
+    }
     // RT_ATTN_DECODE_PDL=0 launches without programmatic stream serialisation.
     static const bool pdl = [] {
         const char* e = getenv("RT_ATTN_DECODE_PDL");
@@ -525,12 +598,17 @@ static cudaError_t launch_dgs(const CUtensorMap& mk, const CUtensorMap& mv, cons
     cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = DecodeTcCfg<D>::SMEM_BYTES;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
     if (pdl) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if constexpr (kCluster > 0) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = kCluster;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
     }
     return cudaLaunchKernelEx(&cfg, kern, mk, mv, p);
 }
@@ -538,8 +616,13 @@ static cudaError_t launch_dgs(const CUtensorMap& mk, const CUtensorMap& mv, cons
 template <int D, int G>
 static cudaError_t launch_dg(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeTcParams& p, int64_t batch,
                              cudaStream_t stream) {
-    return p.split.mode == kSplitShare ? launch_dgs<D, G, true>(mk, mv, p, batch, stream)
-                                       : launch_dgs<D, G, false>(mk, mv, p, batch, stream);
+    if (p.split.mode == kSplitCluster)
+        return p.split.n_chunks == 16  ? launch_dgs<D, G, false, 16>(mk, mv, p, batch, stream)
+               : p.split.n_chunks == 8 ? launch_dgs<D, G, false, 8>(mk, mv, p, batch, stream)
+               : p.split.n_chunks == 4 ? launch_dgs<D, G, false, 4>(mk, mv, p, batch, stream)
+                                       : launch_dgs<D, G, false, 2>(mk, mv, p, batch, stream);
+    return p.split.mode == kSplitShare ? launch_dgs<D, G, true, 0>(mk, mv, p, batch, stream)
+                                       : launch_dgs<D, G, false, 0>(mk, mv, p, batch, stream);
 }
 
 template <int D>
@@ -554,6 +637,50 @@ static cudaError_t launch_d(const CUtensorMap& mk, const CUtensorMap& mv, const 
     return cudaErrorInvalidValue;
 }
 
+// CTAs that clusters of `size` CTAs of this kernel can have resident on the current device at a time (GPCs hold whole clusters
+// only, and how many depends on the part).  Asked once per device, head dim and size; 0 where such clusters do not run.
+template <int D, int C>
+static int decode_cluster_query() {
+    auto kern = gqa_decode_tc_kernel<D, 4, false, C>;
+    if (set_max_dynamic_smem_once<gqa_decode_tc_kernel<D, 4, false, C>>(DecodeTcCfg<D>::SMEM_BYTES) != cudaSuccess) return 0;
+    if (C > 8 && allow_large_cluster_once<gqa_decode_tc_kernel<D, 4, false, C>>() != cudaSuccess) return 0;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C * 256);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = DecodeTcCfg<D>::SMEM_BYTES;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n * C;
+}
+int decode_cluster_slots(int head_dim, int size) {
+    static std::atomic<int> known[64][3][4];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::atomic<int>& slot = known[dev][head_dim == 64 ? 0 : head_dim == 128 ? 1 : 2][size == 2 ? 0 : size == 4 ? 1 : size == 8 ? 2 : 3];
+    const int have = slot.load(std::memory_order_relaxed);
+    if (have > 0) return have - 1;
+    auto ask = [&](auto dim) {
+        constexpr int D = decltype(dim)::value;
+        return size == 2   ? decode_cluster_query<D, 2>()
+               : size == 4 ? decode_cluster_query<D, 4>()
+               : size == 8 ? decode_cluster_query<D, 8>() : decode_cluster_query<D, 16>();
+    };
+    const int n = head_dim == 64    ? ask(std::integral_constant<int, 64>{})
+                  : head_dim == 128 ? ask(std::integral_constant<int, 128>{})
+                                    : ask(std::integral_constant<int, 256>{});
+    slot.store(n + 1, std::memory_order_relaxed);
+    return n;
+}
+
 // Returns cudaErrorNotSupported when this kernel does not cover the shape (the caller then
 // uses the CUDA-core kernel).
 cudaError_t launch_gqa_decode_tc(const void* q, const void* k, const void* v, void* out_bf16, float* out_f32,
@@ -562,7 +689,7 @@ cudaError_t launch_gqa_decode_tc(const void* q, const void* k, const void* v, vo
                                  float scale, float* part_o, float* part_lse, int* counters, const DecodeSplit& split,
                                  int64_t of_stride, int64_t lse_stride, bool* merged, const MergePush* push,
                                  cudaStream_t stream) {
-    *merged = false;
+    *merged = split.mode == kSplitCluster;
     const int64_t cache_rows = batch * n_kv * max_seq;
     if ((head_dim != 64 && head_dim != 128 && head_dim != 256) || cache_rows >= (1ll << 31) - 64)
         return cudaErrorNotSupported;
@@ -619,7 +746,7 @@ cudaError_t launch_gqa_decode_tc(const void* q, const void* k, const void* v, vo
     const bool many_ctas = batch * n_kv * (int64_t)n_chunks >= 4 * (int64_t)sm_count();
     const bool batched = n_chunks <= kMaxFusedChunks && many_ctas && !pushing;
     // (kSplitShare: no fixed number of chunks per group to count to)
-    p.counters = (n_chunks > 1 && split.mode != kSplitShare && fits && (batched || push_ok) && !fused_off) ? counters : nullptr;
+    p.counters = (n_chunks > 1 && split.mode != kSplitShare && split.mode != kSplitCluster && fits && (batched || push_ok) && !fused_off) ? counters : nullptr;
     p.push = MergePush{};
     if (p.counters) {
         cudaError_t e = cudaMemsetAsync(p.counters, 0, sizeof(int) * (size_t)batch * n_kv, stream);

@@ -84,6 +84,8 @@ cudaError_t launch_rope_kv_append(void* q, const void* k_in, const void* v_in, v
                                   cudaStream_t stream);
 
 // ---- decode_tc.cu: TMA + mma.sync decode for head dim 64/128; cudaErrorNotSupported = shape not covered
+// CTAs that clusters of 2, 4, 8 or 16 CTAs of the decode kernel can have resident at a time (kSplitCluster).
+int decode_cluster_slots(int head_dim, int size);
 cudaError_t launch_gqa_decode_tc(const void* q, const void* k, const void* v, void* out_bf16, float* out_f32,
                                  float* lse, int64_t batch, int n_heads, int n_kv, int head_dim, int64_t max_seq,
                                  const int32_t* kv_lens, int64_t kv_len_uniform, int64_t kv_begin, int64_t kv_end,
@@ -110,6 +112,19 @@ inline cudaError_t set_max_dynamic_smem_once(int bytes) {
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
     e = cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
+    return e;
+}
+
+// The same for clusters of more than the 8 CTAs that every part can run.
+template <auto Kern>
+inline cudaError_t allow_large_cluster_once() {
+    static bool done[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+    e = cudaFuncSetAttribute(Kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
     return e;
 }
