@@ -24,21 +24,25 @@
 // MMAs of step u+2 occupy the tensor pipe (the forward kernel pipelines S and P the same way).
 // TMEM (512 columns): buffer b of step u (b = u & 1) holds T1 at [128 b, 128 b + 64) and T2 at
 // [128 b + 64, 128 b + 128); accumulators from 256 (dQ, or dV then dK), D columns each; P^T / dS (bf16)
-// overwrite 32 of the columns of T1 / T2.
+// overwrite 32 of the columns of T1 / T2 (query side at D = 128: 32 columns of their own per buffer, see kApart).
 // From one tile to the next the pipeline does not drain: the next own rows load once the last score MMAs have read the
 // present ones, and the next tile's first score MMAs run while the accumulators are read out (through shared memory
 // and TMA stores).  One CTA per tile, with its set-up, first loads and read-out exposed each time, took 651 us on
-// B=4 H=32 N=2048 D=128 causal (498 now), 45 on B=1 H=32 N=658 D=64 (24), 46 on B=4 H=8 N=625 D=128 (25).
-//  320 threads: warps 0-7 element-wise work and the final read-out,
+// B=4 H=32 N=2048 D=128 causal (498 with one issuing warp, 456 with two and what follows), 45 on B=1 H=32 N=658 D=64 (23).
+//  384 threads: warps 0-7 element-wise work and the final read-out,
 // two threads per own row (warp w owns rows 32 (w % 4).. and the 32 score columns of half w / 4; its bf16
 // results go back into the first 16 of its OWN columns, so the two threads of a row never touch each other's
 // inputs, and the accumulating MMAs take K elements 0-31 from columns [0,16) and 32-63 from [32,48));
-// warp 8 TMA producer, warp 9 TMEM allocation and MMA issue.
+// warp 8 TMA producer, warp 9 TMEM allocation and the accumulating MMAs, warp 10 the score MMAs, warp 11 the columns' statistics.
+// What bounds a step: the MMAs on the key side at D = 128 (1270 clocks of 1280), MMAs and their hand-over on its query side (1140 of
+// 1024), the element-wise chain at D = 64 (1030 and 980 for 640 and 512 of MMA); between two items the read-out, 4000 clocks of f32
+// stores at D = 128, and the refill.
 // Every mbarrier wait is bounded; on expiry the kernel records a code in the device status word and
 // leaves through the common teardown.
 #include <cuda.h>
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "kernels.h"
 #include "tc_ptx.cuh"
@@ -60,6 +64,8 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 // Q, K, V and dO up to this size are taken to stay in L2 (126 MB) with their gradients passing through.
 constexpr int64_t kLevelsBytes = 96ll << 20;
 
+constexpr int kBwdThreads = 384;
+
 template <int D>
 struct BwdCfg {
     static constexpr int TILE_BYTES = 128 * D * 2;
@@ -69,8 +75,8 @@ struct BwdCfg {
     static constexpr int HSUB_BYTES = 64 * 64 * 2;
     static constexpr int STAGES = 4;                // ring slots, each (Y1 | Y2) of one 64-row step
     static constexpr int STAGE_OUT = 8 * 32 * 128;  // per element-wise warp: 32 rows x 32 f32 columns on their way out
-    static constexpr int NBARS = 2 + 2 * STAGES + 6;
-    static constexpr int STAT_BYTES = 2 * 2 * 128 * 4;  // two slots of LSE * log2(e) and delta of a 128-row other tile
+    static constexpr int NBARS = 2 + 2 * STAGES + 13;
+    static constexpr int STAT_BYTES = 2 * 2 * 128 * 4;  // two slots of -LSE * log2(e) and -delta of a 128-row other tile
     static constexpr int SMEM_BYTES = 2 * TILE_BYTES + STAGES * 2 * HALF_BYTES + STAGE_OUT + STAT_BYTES + NBARS * 8 + 16;
     static constexpr uint32_t COL_T = 0, COL_ACC = 256;  // T1 of buffer b at COL_T + 128 b, T2 64 columns further
     static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB of shared memory a CTA can opt into");
@@ -101,6 +107,11 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
                                          const Bwd5Params& p, uint8_t* smem, int warp, int lane, int cta, int n_ctas) {
     using C = BwdCfg<D>;
     constexpr int TILE = C::TILE_BYTES, SUB = C::SUB_BYTES, STAGES = C::STAGES, HALFT = C::HALF_BYTES, HSUB = C::HSUB_BYTES;
+    // Where TMEM has room behind the accumulators, the A operands have columns of their own (per buffer P^T and dS^T, or
+    // dS, 32 each): the score MMAs of step u + 2 then follow the reading of T(u), not the accumulating MMAs of step u.
+    constexpr bool kApart = !kKeySide && D == 128;
+    constexpr uint32_t COL_A = C::COL_ACC + (kKeySide ? 2 : 1) * D, A_BUF = kKeySide ? 64 : 32;
+    static_assert(!kApart || COL_A + 2 * A_BUF <= 512, "TMEM columns");
     uint8_t* sX1 = smem;
     uint8_t* sX2 = sX1 + TILE;
     uint8_t* sY = sX2 + TILE;  // [STAGES][Y1 | Y2], 64 rows each
@@ -114,8 +125,11 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
     uint64_t* t_full = y_empty + STAGES;    // [2] per buffer, one phase per use: T1, T2 are in TMEM
     uint64_t* a_full = t_full + 2;          // [2] per buffer, one phase per use: the bf16 A operands are in TMEM
     uint64_t* acc_done = a_full + 2;        // [1] one phase per item: its last accumulating MMA has retired
-    uint64_t* stat_bar = acc_done + 1;      // [1] one phase per other tile: the column statistics are in shared memory
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stat_bar + 1);
+    uint64_t* stat_bar = acc_done + 1;      // [2] key side, per slot, one phase per other tile: the column statistics are in shared memory
+    uint64_t* acc_step = stat_bar + 2;      // [2] per buffer, one phase per use: the MMAs that read the A operands have retired
+    uint64_t* t_read = acc_step + 2;        // [2] per buffer, one phase per use: T1, T2 are in registers (kApart)
+    uint64_t* acc_half = t_read + 2;        // [2] key side, as acc_step: the MMAs that read P^T have
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_half + 2);
 
     const int N = p.seq;
     const LevelSchedule& list = p.list[kKeySide ? 1 : 0];
@@ -163,9 +177,13 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
         for (int i = 0; i < 2; ++i) {
             mbar_init(&t_full[i], 1);
             mbar_init(&a_full[i], 256);
+            mbar_init(&acc_step[i], 1);
+            mbar_init(&t_read[i], 256);
+            mbar_init(&acc_half[i], 1);
         }
         mbar_init(acc_done, 1);
-        mbar_init(stat_bar, 256);
+        mbar_init(&stat_bar[0], 32);
+        mbar_init(&stat_bar[1], 32);
         fence_barrier_init();
         fence_proxy_async();
     }
@@ -217,103 +235,134 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
             for (int u = max(0, g - STAGES); u < g; ++u)
                 mbar_wait(&y_full[u % STAGES], (uint32_t)(u / STAGES) & 1u, p.status, kToBwdDrain);
         }
-    } else if (warp == 9) {
-        // ============================================================== MMA issuer
+    } else if (warp == 11) {
+        // ============================================================== key side: the columns' statistics
+        // -LSE (as log2; -inf, which makes every probability 0, for absent queries and rows without a visible key) and -delta
+        // of the 128 queries of each other tile, negated here once rather than per score, into the slot that was last
+        // read two tiles ago (its last step's rows are free: every thread has handed that step's operands over).
+        if (kKeySide) {
+            int g = 0, gt = 0, before = 0, before2 = 0;  // steps and tiles so far, last step of the tile before and of the one before that
+            bool ok = true;
+            BwdItem it;
+            for (int j = 0; ok && fetch(j, it); g += it.n_u) {
+                const float* lse = p.lse + (int64_t)it.bh * N;
+                const float* delta = p.delta + (int64_t)it.bh * N;
+                for (int u = 0; u < it.n_u && ok; u += 2, ++gt) {
+                    float l[4], d[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int qi = (it.s_lo + u) * 64 + i * 32 + lane;
+                        const float raw = qi < N ? __ldg(lse + qi) : INFINITY;
+                        l[i] = (raw > -INFINITY && raw < INFINITY) ? raw * -kLog2e : -INFINITY;
+                        d[i] = qi < N ? -__ldg(delta + qi) : 0.f;
+                    }
+                    if (gt >= 2)
+                        ok = __all_sync(kFullMask, mbar_wait(&y_empty[before2 % STAGES], (uint32_t)(before2 / STAGES) & 1u, p.status, kToBwdStat));
+                    float* to = stat + (gt & 1) * 256;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        to[i * 32 + lane] = l[i];
+                        to[128 + i * 32 + lane] = d[i];
+                    }
+                    mbar_arrive(&stat_bar[gt & 1]);
+                    before2 = before;
+                    before = g + min(u + 1, it.n_u - 1);
+                }
+            }
+        }
+    } else if (warp >= 9) {
+        // ============================================================== MMA issuers
+        // One warp for the score MMAs, one for the accumulating ones: an issuing warp is held until the pipe takes its MMA, so
+        // what a single one did between two steps (two waits that were already over, commits: 345 clocks of 1625 a key-side
+        // step at D=128) left the pipe idle.
         const bool leader = elect_one();
-        constexpr uint32_t idesc_t = make_idesc_bf16(128, 64, 0, 0);
-        constexpr uint32_t idesc_a = make_idesc_bf16(128, D, 0, 1);
-        const uint64_t dx1 = make_smem_desc_sw128(smem_u32(sX1), 16, 1024);
-        const uint64_t dx2 = make_smem_desc_sw128(smem_u32(sX2), 16, 1024);
-        const uint64_t dy_k = make_smem_desc_sw128(smem_u32(sY), 16, 1024);    // other tile as a K-major operand
-        const uint64_t dy_mn = make_smem_desc_sw128(smem_u32(sY), HSUB, 1024);  // the same rows as an MN-major operand
         const uint32_t tT = tmem_base + C::COL_T, tAcc = tmem_base + C::COL_ACC;
-        auto commit = [&](uint64_t* bar) {
-            if (leader) mma_commit(bar);
-        };
-        auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+        auto wait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
             return __all_sync(kFullMask, mbar_wait(bar, parity, p.status, code));
         };
-        // T1 = X1 Y1^T, T2 = X2 Y2^T over the 64 other-side rows of step u (counted over all items), into buffer u & 1
-        // (they overwrite the A operands of step u - 2: the pipe runs this thread's MMAs in issue order, after the accumulating
-        // MMAs of that step)
-        auto issue_T = [&](int u) {
-            const int st = u % STAGES;
-            const uint64_t y1 = dy_k + (uint64_t)((st * 2 * HALFT) >> 4), y2 = y1 + (uint64_t)(HALFT >> 4);
-            const uint32_t t1 = tT + (u & 1) * 128, t2 = t1 + 64;
-#pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-                const uint32_t offx = (uint32_t)(((kk / 4) * SUB + (kk % 4) * 32) >> 4);
-                const uint32_t offy = (uint32_t)(((kk / 4) * HSUB + (kk % 4) * 32) >> 4);
-                if (leader) mma_ss(t1, dx1 + offx, y1 + offy, idesc_t, kk > 0);
-            }
-#pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-                const uint32_t offx = (uint32_t)(((kk / 4) * SUB + (kk % 4) * 32) >> 4);
-                const uint32_t offy = (uint32_t)(((kk / 4) * HSUB + (kk % 4) * 32) >> 4);
-                if (leader) mma_ss(t2, dx2 + offx, y2 + offy, idesc_t, kk > 0);
-            }
-        };
-        auto wait_rows = [&](int u) {  // the rows of step u have landed
-            const bool got = wait(&y_full[u % STAGES], (uint32_t)(u / STAGES) & 1u, kToBwdYFull);
-            tc_fence_after();
-            return got;
-        };
-        int g = 0;  // the item's first step
         bool ok = true;
         BwdItem it;
-        for (int j = 0, k = 0; ok && fetch(j, it); ++k) {
-            // The item's first score MMAs follow the previous item's last accumulating ones and run while the element-wise
-            // warps read those accumulators out; their next results, which the first accumulating MMAs here
-            // wait for, come after that.
-            const int n_u = it.n_u;
-            ok = wait(x_full, (uint32_t)k & 1u, kToBwdX);
-            for (int u = 0; u < min(2, n_u) && ok; ++u) {
-                ok = wait_rows(g + u);
-                if (!ok) break;
-                issue_T(g + u);
-                commit(&t_full[(g + u) & 1]);
-                if (u == n_u - 1) commit(x_empty);
-            }
-            for (int u = 0; u < n_u && ok; ++u) {
-                const int gu = g + u, st = gu % STAGES;
-                if (!wait(&a_full[gu & 1], (uint32_t)(gu >> 1) & 1u, kToBwdA)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint64_t y1 = dy_mn + (uint64_t)((st * 2 * HALFT) >> 4), y2 = y1 + (uint64_t)(HALFT >> 4);
-                const uint32_t t1 = tT + (gu & 1) * 128, t2 = t1 + 64;
-                const uint32_t acc0 = u > 0 ? 1u : 0u;
-                if (kKeySide) {
-                    // dV += P^T dO (A = P^T in the first 32 columns of T1, B = Y2 = dO), dK += dS^T Q (A in T2, B = Y1 = Q)
+        if (warp == 10) {
+            // T1 = X1 Y1^T, T2 = X2 Y2^T over the 64 other-side rows of every step, two steps ahead of the accumulating MMAs.  The
+            // first ones of an item run while the element-wise warps read the accumulators of the one before out.
+            constexpr uint32_t idesc_t = make_idesc_bf16(128, 64, 0, 0);
+            const uint64_t dx1 = make_smem_desc_sw128(smem_u32(sX1), 16, 1024);
+            const uint64_t dx2 = make_smem_desc_sw128(smem_u32(sX2), 16, 1024);
+            const uint64_t dy = make_smem_desc_sw128(smem_u32(sY), 16, 1024);  // other tile as a K-major operand
+            int st = 0;                       // ring slot of the step
+            uint32_t ph = 0, b = 0, pb = 3;   // its phase; the step's buffer; bit b: phase in which the buffer is free
+            for (int j = 0, k = 0; ok && fetch(j, it); ++k) {
+                ok = wait(x_full, (uint32_t)k & 1u, kToBwdX);
+                for (int u = 0; u < it.n_u && ok; ++u) {
+                    ok = wait(&y_full[st], ph, kToBwdYFull) && wait(kApart ? &t_read[b] : kKeySide ? &acc_half[b] : &acc_step[b], (pb >> b) & 1u, kToBwdAcc);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t y1 = dy + (uint64_t)((st * 2 * HALFT) >> 4), y2 = y1 + (uint64_t)(HALFT >> 4);
+                    const uint32_t t1 = tT + b * 128, t2 = t1 + 64;
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        if (leader)
-                            mma_ts(tAcc, t1 + kk * 8 + (kk >= 2 ? 16 : 0), y2 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        if (leader)
-                            mma_ts(tAcc + D, t2 + kk * 8 + (kk >= 2 ? 16 : 0), y1 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
-                } else {
-                    // dQ += dS K (A = dS in the first 32 columns of T2, B = Y1 = K)
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        if (leader)
-                            mma_ts(tAcc, t2 + kk * 8 + (kk >= 2 ? 16 : 0), y1 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
-                }
-                commit(&y_empty[st]);  // the step's rows are free once these MMAs (and the score MMAs before them) retire
-                if (u == n_u - 1) commit(acc_done);
-                if (u + 2 < n_u) {
-                    if (!wait_rows(gu + 2)) {
-                        ok = false;
-                        break;
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        const uint32_t offx = (uint32_t)(((kk / 4) * SUB + (kk % 4) * 32) >> 4);
+                        const uint32_t offy = (uint32_t)(((kk / 4) * HSUB + (kk % 4) * 32) >> 4);
+                        if (leader) mma_ss(t1, dx1 + offx, y1 + offy, idesc_t, kk > 0);
                     }
-                    issue_T(gu + 2);
-                    commit(&t_full[gu & 1]);
-                    if (u + 2 == n_u - 1) commit(x_empty);
+                    if (kKeySide) {  // T1 overwrites P^T while the MMAs that read dS^T, in T2, still run
+                        ok = wait(&acc_step[b], (pb >> b) & 1u, kToBwdAcc);
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
+#pragma unroll
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        const uint32_t offx = (uint32_t)(((kk / 4) * SUB + (kk % 4) * 32) >> 4);
+                        const uint32_t offy = (uint32_t)(((kk / 4) * HSUB + (kk % 4) * 32) >> 4);
+                        if (leader) mma_ss(t2, dx2 + offx, y2 + offy, idesc_t, kk > 0);
+                    }
+                    if (leader) mma_commit(&t_full[b]);
+                    if (leader && u == it.n_u - 1) mma_commit(x_empty);
+                    pb ^= 1u << b;
+                    b ^= 1;
+                    if (++st == STAGES) st = 0, ph ^= 1;
                 }
             }
-            g += n_u;
+        } else {
+            constexpr uint32_t idesc_a = make_idesc_bf16(128, D, 0, 1);
+            const uint64_t dy = make_smem_desc_sw128(smem_u32(sY), HSUB, 1024);  // the other tile's rows as an MN-major operand
+            int st = 0;                      // ring slot of the step
+            uint32_t b = 0, pa = 0;          // the step's buffer; bit b: phase of its A operands
+            for (int j = 0; ok && fetch(j, it);) {
+                // (The first A operands of an item come after the element-wise warps have read the accumulators out.)
+                for (int u = 0; u < it.n_u; ++u) {
+                    ok = wait(&a_full[b], (pa >> b) & 1u, kToBwdA);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t y1 = dy + (uint64_t)((st * 2 * HALFT) >> 4), y2 = y1 + (uint64_t)(HALFT >> 4);
+                    // P^T, dS^T (or dS): contiguous, or the first 16 of every 32 columns of T1 and T2
+                    const uint32_t a1 = kApart ? tmem_base + COL_A + b * A_BUF : tT + b * 128;
+                    const uint32_t a2 = kApart ? (kKeySide ? a1 + 32 : a1) : a1 + 64;
+                    auto k16 = [](int kk) { return (uint32_t)(kk * 8 + (!kApart && kk >= 2 ? 16 : 0)); };
+                    const uint32_t acc0 = u > 0 ? 1u : 0u;
+                    if (kKeySide) {
+                        // dV += P^T dO (B = Y2 = dO), dK += dS^T Q (B = Y1 = Q)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            if (leader) mma_ts(tAcc, a1 + k16(kk), y2 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
+                        if (leader) mma_commit(&acc_half[b]);
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            if (leader) mma_ts(tAcc + D, a2 + k16(kk), y1 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
+                    } else {
+                        // dQ += dS K (B = Y1 = K)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            if (leader) mma_ts(tAcc, a2 + k16(kk), y1 + (uint64_t)((kk * 2048) >> 4), idesc_a, kk > 0 ? 1u : acc0);
+                    }
+                    if (leader) mma_commit(&acc_step[b]);
+                    if (leader) mma_commit(&y_empty[st]);  // the step's rows: its score MMAs have retired before
+                    if (leader && u == it.n_u - 1) mma_commit(acc_done);
+                    pa ^= 1u << b;
+                    b ^= 1;
+                    if (++st == STAGES) st = 0;
+                }
+            }
         }
     } else {
         // ============================================================== element-wise warps (two threads per own row)
@@ -324,48 +373,36 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
         const uint32_t tAcc = tmem_base + lane_sel + C::COL_ACC;
         uint8_t* const stage = sOut + warp * 4096;
         const float c = p.scale_log2;
-        // LSE (as log2; +inf, which makes every probability 0, for absent queries and rows without a visible key) and
-        // delta of one query.  Requested a tile (key side) or an item (query side) ahead.
+        // Query side: the row's own statistics (see warp 11 for the key side's), requested an item ahead.
         float raw_lse = 0.f, raw_delta = 0.f;
-        auto request = [&](const BwdItem& it, int qi) {
+        auto request = [&](const BwdItem& it) {
+            const int qi = it.own0 + r;
             raw_lse = qi < N ? __ldg(p.lse + (int64_t)it.bh * N + qi) : INFINITY;
-            raw_delta = qi < N ? __ldg(p.delta + (int64_t)it.bh * N + qi) : 0.f;
+            raw_delta = qi < N ? -__ldg(p.delta + (int64_t)it.bh * N + qi) : 0.f;
         };
-        auto lse2 = [&] { return (raw_lse > -INFINITY && raw_lse < INFINITY) ? raw_lse * kLog2e : INFINITY; };
         int j = 0, g = 0, gt = 0;  // list entry, first step of the item, other tiles so far (key side)
         BwdItem it, nx;
         bool ok = true, more = fetch(j, it);
-        if (more) request(it, kKeySide ? it.s_lo * 64 + r : it.own0 + r);
+        if (!kKeySide && more) request(it);
         for (int k = 0; more && ok; ++k, it = nx) {
         more = fetch(j, nx);
         const int own_row = it.own0 + r, n_u = it.n_u;
         float my_lse2 = 0.f, my_delta = 0.f;  // query side: this row's statistics
         if (!kKeySide) {
-            my_lse2 = lse2();
+            my_lse2 = (raw_lse > -INFINITY && raw_lse < INFINITY) ? raw_lse * -kLog2e : -INFINITY;
             my_delta = raw_delta;
-            if (more) request(nx, nx.own0 + r);
+            if (more) request(nx);
         }
         for (int u = 0; u < n_u && ok; ++u) {
             const int step = it.s_lo + u, buf = (g + u) & 1, sub = step & 1;
             const int other0 = step * 64;  // first other-side row of this step
-            float* s_lse2 = stat + (gt & 1) * 256;
-            float* s_delta = s_lse2 + 128;
-            if (kKeySide && sub == 0) {
-                // the statistics of this tile's 128 queries (columns); the slot was last read two tiles ago, and
-                // every thread has passed the a_full arrivals of that tile's successor by now
-                if (half == 0) {
-                    s_lse2[r] = lse2();
-                    s_delta[r] = raw_delta;
-                    if (u + 2 < n_u) request(it, other0 + 128 + r);
-                    else if (more) request(nx, nx.s_lo * 64 + r);
-                }
-                mbar_arrive(stat_bar);  // an mbarrier rather than bar.sync, so that this wait is bounded as well
-                if (!__all_sync(kFullMask, mbar_wait(stat_bar, (uint32_t)gt & 1u, p.status, kToBwdStat))) {
-                    ok = false;
-                    break;
-                }
-            }
-            if (!__all_sync(kFullMask, mbar_wait(&t_full[buf], (uint32_t)((g + u) >> 1) & 1u, p.status, kToBwdT))) {
+            const float* s_lse2 = stat + (gt & 1) * 256;
+            const float* s_delta = s_lse2 + 128;
+            if (kKeySide && sub == 0) ok &= mbar_wait(&stat_bar[gt & 1], (uint32_t)(gt >> 1) & 1u, p.status, kToBwdStat);
+            ok &= mbar_wait(&t_full[buf], (uint32_t)((g + u) >> 1) & 1u, p.status, kToBwdT);
+            // its A operands: the MMAs of two steps ago have read them
+            if (kApart && g + u >= 2) ok &= mbar_wait(&acc_step[buf], (uint32_t)(((g + u) >> 1) - 1) & 1u, p.status, kToBwdAcc);
+            if (!__all_sync(kFullMask, ok)) {  // (one vote for the waits of the step)
                 ok = false;
                 break;
             }
@@ -382,11 +419,17 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
                 tmem_ld32(t1 + cbase, a1);
                 tmem_ld32(t2 + cbase, a2);
                 tc_wait_ld();
+                if (kApart) {
+                    tc_fence_before();
+                    mbar_arrive(&t_read[buf]);
+                }
                 uint32_t pk_p[16], pk_ds[16];
+                // (Compiled twice: a test per four columns cuts the step into eight pieces whose exponentials cannot overlap.)
+                auto columns = [&](auto masked) {
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
                     // statistics of four columns: the row's own on the query side, one 16-byte broadcast read each
-                    // on the key side (an LSE of +inf makes the probability 0: absent queries, rows without a key)
+                    // on the key side (a negated LSE of -inf makes the probability 0: absent queries, rows without a key)
                     float4 l4, d4;
                     if (kKeySide) {
                         l4 = *reinterpret_cast<const float4*>(s_lse2 + sub * 64 + cbase + i);
@@ -396,12 +439,12 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
                         d4 = make_float4(my_delta, my_delta, my_delta, my_delta);
                     }
                     const float2 xa = __ffma2_rn(make_float2(__uint_as_float(a1[i]), __uint_as_float(a1[i + 1])), c2,
-                                                 make_float2(-l4.x, -l4.y));
+                                                 make_float2(l4.x, l4.y));
                     const float2 xb = __ffma2_rn(make_float2(__uint_as_float(a1[i + 2]), __uint_as_float(a1[i + 3])), c2,
-                                                 make_float2(-l4.z, -l4.w));
+                                                 make_float2(l4.z, l4.w));
                     float2 pa = make_float2(fast_exp2(xa.x), fast_exp2(xa.y));
                     float2 pb = make_float2(fast_exp2(xb.x), fast_exp2(xb.y));
-                    if (diag || ragged) {
+                    if constexpr (decltype(masked)::value) {
                         const int o0 = other0 + cbase + i;
                         auto hidden = [&](int other) {
                             return other >= N || (p.causal && (kKeySide ? own_row > other : other > own_row));
@@ -412,18 +455,26 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
                         if (hidden(o0 + 3)) pb.y = 0.f;
                     }
                     const float2 ta = __fadd2_rn(make_float2(__uint_as_float(a2[i]), __uint_as_float(a2[i + 1])),
-                                                 make_float2(-d4.x, -d4.y));
+                                                 make_float2(d4.x, d4.y));
                     const float2 tb = __fadd2_rn(make_float2(__uint_as_float(a2[i + 2]), __uint_as_float(a2[i + 3])),
-                                                 make_float2(-d4.z, -d4.w));
+                                                 make_float2(d4.z, d4.w));
                     const float2 da = __fmul2_rn(pa, ta), db = __fmul2_rn(pb, tb);
                     pk_p[i / 2] = float2_to_bf16x2(pa.x, pa.y);
                     pk_p[i / 2 + 1] = float2_to_bf16x2(pb.x, pb.y);
                     pk_ds[i / 2] = float2_to_bf16x2(da.x, da.y);
                     pk_ds[i / 2 + 1] = float2_to_bf16x2(db.x, db.y);
                 }
-                // the 32 bf16 values go into the first 16 of this thread's own 32 columns (in registers by now)
-                if (kKeySide) tmem_st16(t1 + cbase, pk_p);
-                tmem_st16(t2 + cbase, pk_ds);
+                };
+                if (diag || ragged) columns(std::true_type{});
+                else columns(std::false_type{});
+                if constexpr (kApart) {
+                    const uint32_t to = tmem_base + lane_sel + COL_A + buf * A_BUF + half * 16;
+                    if (kKeySide) tmem_st16(to, pk_p);
+                    tmem_st16(to + (kKeySide ? 32 : 0), pk_ds);
+                } else {  // into the first 16 of this thread's own 32 columns (in registers by now)
+                    tmem_st16(t1 + cbase, pk_p);
+                    tmem_st16(t2 + cbase, pk_ds);
+                }
             }
             tc_wait_st();
             tc_fence_before();
@@ -479,7 +530,7 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
 
 // CTAs [0, q_ctas) work through the query side's tiles, the others through the key side's.
 template <int D>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                    const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dk,
@@ -504,11 +555,11 @@ cudaError_t launch_sides(const CUtensorMap (&m)[7], Bwd5Params p, int64_t bh, cu
     const int64_t n_sm = sm_count();
     // Both sides' tiles go out in one launch: small grids run side by side, and large ones have one tail instead of
     // two.  Where the tiles exceed the SMs, the query side gets fewer of them: it has one accumulating product
-    // a step, the key side two (share: measured best of 0.34 .. 0.46 on 8 causal shapes; equal tiles come in whole
+    // a step, the key side two (share: measured best of 0.39 .. 0.50 on 16 shapes; equal tiles come in whole
     // waves, so without a mask the split with the shortest longer side is taken, 77 -> 72 us at B=2 H=16 N=1024 D=128).
     int64_t nq = n_items, nk = n_items;
     if (2 * n_items > n_sm) {
-        constexpr double share = D == 128 ? 0.43 : 0.41;
+        constexpr double share = D == 128 ? 0.45 : 0.46;
         nq = std::max<int64_t>(1, (int64_t)((double)n_sm * share + 0.5));
         if (!p.causal) {
             double best = 1e30;
@@ -527,7 +578,7 @@ cudaError_t launch_sides(const CUtensorMap (&m)[7], Bwd5Params p, int64_t bh, cu
     p.list[1] = make_level_schedule(bh, n_tiles, nk, paired);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(nq + nk));
-    cfg.blockDim = dim3(320);
+    cfg.blockDim = dim3(kBwdThreads);
     cfg.dynamicSmemBytes = BwdCfg<D>::SMEM_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
