@@ -59,7 +59,8 @@ struct TcCfg {
     // (batch, query block) pairs the length-sorted schedule can hold (two uint16 per pair); what is left of
     // the 227 KB of shared memory at D = 128 bounds it there
     static constexpr int SCHED_CAP = (D == 128) ? 384 : 2048;
-    static constexpr int SMEM_BYTES = (2 + KS + VS) * TILE_BYTES + NBARS * 8 + 48 + 4 * SCHED_CAP + 1024;
+    static constexpr bool OWN_STAGE = (D == 64);        // the O tiles on their way out have shared memory of their own
+    static constexpr int SMEM_BYTES = (2 + KS + VS + (OWN_STAGE ? 2 : 0)) * TILE_BYTES + NBARS * 8 + 48 + 4 * SCHED_CAP + 1024;
     static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB of shared memory a CTA can opt into");
     static constexpr uint32_t TMEM_COLS = 512;
     static constexpr uint32_t COL_S = 0, COL_O = 256;   // S: tile w, buffer b at COL_S + w*128 + b*64
@@ -334,9 +335,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     uint8_t* sQ = smem;
     uint8_t* sK = sQ + 2 * TILE;
     uint8_t* sV = sK + KS * TILE;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + VS * TILE);
+    uint8_t* sO = C::OWN_STAGE ? sV + VS * TILE : sQ;  // [2] staged O tiles
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + (VS + (C::OWN_STAGE ? 2 : 0)) * TILE);
     uint64_t* q_full = bars;              // [2]
-    uint64_t* q_empty = q_full + 2;       // [2]  the O tile staged in the Q buffer has been read out
+    uint64_t* q_empty = q_full + 2;       // [2]  the next Q may land (see early_q)
     uint64_t* k_full = q_empty + 2;       // [KS]
     uint64_t* k_empty = k_full + KS;      // [2 tiles][KS]: the issuer of tile w is done with the slot
     uint64_t* v_full = k_empty + 2 * KS;  // [VS]
@@ -660,6 +662,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                     mma_ts(tO, tS + b * 64 + kk * 8, bv + (uint64_t)((kk * 2048) >> 4), idesc_o, kk > 0 ? 1u : acc);
             };
             constexpr uint32_t kTileEnc = TILE >> 4, kHalfEnc = HALF >> 4;
+            constexpr bool early_q = C::OWN_STAGE;  // nothing is staged in the Q buffer: it is free behind the item's last scores
             bool ok = true;
             for (int j = 0; ok; ++j) {
                 const TcItem it = tc_item<kCausal, kSingle, kByLength>(j, p, sched, keep_hi);
@@ -724,6 +727,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                             issue_S(0, bk);
                             if (n_u > 1) issue_S(1, bk + kHalfEnc);
                             mma_commit(&ke[ks]);
+                            if (early_q && n_u <= 2) mma_commit(&q_empty[w]);
                         }
                         next_k();
                     }
@@ -739,6 +743,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         if (leader) {
                             issue_PV(0, bv, u > 0 ? 1u : 0u);
                             if (more) issue_S(0, bk);
+                            if (early_q && u + 3 == n_u) mma_commit(&q_empty[w]);
                             if (u + 2 == n_u) mma_commit(&o_full[w]);
                         }
                         if (u + 1 < n_u) {
@@ -749,6 +754,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                             if (leader) {
                                 issue_PV(1, bv + kHalfEnc, 1u);
                                 if (u + 3 < n_u) issue_S(1, bk + kHalfEnc);
+                                if (early_q && u + 4 == n_u) mma_commit(&q_empty[w]);
                                 if (u + 3 == n_u) mma_commit(&o_full[w]);
                             }
                         }
@@ -823,6 +829,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 continue;
             }
 
+            // The tile's last O has been read out of its staging buffer; the other threads learn it through o_done, below.
+            if (C::OWN_STAGE && !il && row_in_tile == 0) tma_store_wait_read();
             float m_ref = -INFINITY;  // reference max (raw score units) the running sums are relative to; -inf: no score was visible yet
             float l = 0.f;
             for (int u = 0; u < n_iter; ++u) {
@@ -1044,7 +1052,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 // empty when it never saw a visible score, not when its sum is exactly 0.
                 const bool valid = seen && (l > 0.f);
                 const float inv = valid ? 1.f / l : 0.f;
-                uint8_t* stage = sQ + w * TILE + row_in_tile * 128;  // every score MMA that read Q_w has retired
+                uint8_t* stage = sO + w * TILE + row_in_tile * 128;  // (in the Q buffer: every score MMA that read Q_w has retired)
                 __nv_bfloat16* dst = p.out + it.b * p.o_stride_b + it.h * p.o_stride_h + (int64_t)row * p.o_stride_row;
 #pragma unroll
                 for (int ch = 0; ch < D / 32; ++ch) {
@@ -1087,9 +1095,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 } else {
 #pragma unroll
                     for (int s = 0; s < C::NSUB; ++s)
-                        tma_store_4d(&tm_o, sQ + w * TILE + s * SUB, s * 64, it.qrow(w, il), it.h, it.b);
-                    tma_store_commit_and_wait_read();  // the staged tile has been read: the next Q may land
-                    mbar_arrive(&q_empty[w]);
+                        tma_store_4d(&tm_o, sO + w * TILE + s * SUB, s * 64, it.qrow(w, il), it.h, it.b);
+                    tma_store_commit();
+                    if (!C::OWN_STAGE) {
+                        tma_store_wait_read();  // the staged tile has been read: the next Q may land
+                        mbar_arrive(&q_empty[w]);
+                    }
                 }
             }
             ok = __all_sync(kFullMask, ok);
@@ -1098,6 +1109,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             cs1 += n_iter / 2;
             co += n_iter > 1 ? 1 : 0;
         }
+        if (C::OWN_STAGE && !kSingle && row_in_tile == 0) tma_store_wait_read();  // shared memory stays until the last store has read it
         if constexpr (kSplit) {
             // ---- the cluster's partial rows: CTA r reads its 128 / split rows from every CTA's shared memory, merges them
             // as above and stores them.  (A CTA that gave up on a wait still meets the barriers.)
