@@ -9,6 +9,8 @@
 //   prefill_f32_tiled_kernel  16 query rows and more: 64 rows per CTA, register tiles, exp2f (simt_tile.cuh)
 //   prefill_f32_kernel        fewer rows: one warp owns one query row and walks the keys in tiles of 32 staged in
 //                             shared memory, expf
+#include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -30,6 +32,7 @@ struct SimtParams {
     const uint8_t* key_keep;
     int64_t keep_batch_stride;
     float scale;
+    int split;  // CTAs (one cluster) that share the keys of a row block
 };
 
 __global__ void __launch_bounds__(kSimtRows * 32) prefill_f32_kernel(const SimtParams p) {
@@ -144,7 +147,21 @@ __global__ void __launch_bounds__(kSimtRows * 32) prefill_f32_kernel(const SimtP
 // Against the 256-thread kernel with 4 x 4 scores a thread that this replaces (scalar loads transposed into shared
 // memory with 16-way conflicts): B=1 H=8 N=2048 D=64 causal 371 -> 120 us (36 TFLOP/s), B=2 H=16 N=1000 D=128 causal
 // 520 -> 232 us, B=4 H=16 N=1024 D=64 656 -> 435 us (40 TFLOP/s of the FP32 pipe's 74).
-template <int NC, int G>
+// Launches of few row blocks leave SMs idle while each block walks its keys alone; there a cluster of 2, 4 or 8 CTAs shares
+// them (kSplit): each takes every split-th pair of tiles, leaves its partial rows in shared memory, and merges 64 / split rows out
+// of all of them.  (N=2048 D=64 causal, H=1 121 -> 40 us, H=2 122 -> 71; B=1 H=4 N=600 D=80 56 -> 44; the merge costs about half a step.)
+__device__ __forceinline__ void f32_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float f32_remote(const float* a, int rank) {
+    uint32_t r;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(a)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+    return v;
+}
+
+template <int NC, int G, bool kSplit>
 __global__ void __launch_bounds__(simt::kGroup * G, 1)
 prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, const int64_t row_blocks) {
     using namespace simt;
@@ -159,7 +176,8 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
     const Share share = Share::of<kGroup>(tid, D, vec), q_share = Share::of<kGroup * G>((int)threadIdx.x, D, vec);
 
     // CTA order: under a causal mask the longest row blocks of all heads first
-    const int64_t n_bh = (int64_t)gridDim.x / row_blocks, x = blockIdx.x;
+    const int rank = kSplit ? (int)blockIdx.x % p.split : 0, split = kSplit ? p.split : 1;
+    const int64_t n_bh = (int64_t)gridDim.x / split / row_blocks, x = blockIdx.x / split;
     const int64_t bh = p.causal ? x % n_bh : x / row_blocks;
     const int64_t row0 = (p.causal ? row_blocks - 1 - x / n_bh : x % row_blocks) * kRows;
     const int64_t b = bh / p.heads_q, hq = bh % p.heads_q, hkv = hq / (p.heads_q / p.heads_kv);
@@ -192,7 +210,7 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
 #pragma unroll
         for (int c = 0; c < 2 * NC; ++c) z[r][c] = make_float2(0.f, 0.f);
 
-    const int64_t first = (int64_t)group * kRows, step = (int64_t)G * kRows;
+    const int64_t first = (int64_t)(rank * G + group) * kRows, step = (int64_t)(G * split) * kRows;
     load_tile<kRows, kGroup * G>(Qs, p.q + (bh * p.seq_q) * D, row0, p.seq_q, D, vec, q_share);
     if (first < k_loop) load_tile<kRows, kGroup>(Ks, kptr, first, k_hi, D, vec, share);
     cp_async_commit();
@@ -257,7 +275,7 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
             for (int i = 0; i < 8; ++i) ex[(8 * NC + i) * kGroup + tid] = make_float2(m[i], l[i]);
         }
         __syncthreads();
-        if (group == 1) return;
+        if (!kSplit && group == 1) return;
         float2 f0[4], f1[4];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -276,6 +294,52 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
                 z[r][c] = __ffma2_rn(f0[r], z[r][c], __fmul2_rn(f1[r], ex[(r * 2 * NC + c) * kGroup + tid]));
     }
 
+    if constexpr (kSplit) {
+        // ---- the cluster's partial rows, over the Q tile; (max, sum) of each where the second group's tiles were
+        float* const part = Qs;
+        float* const ml = smem + tile + 2 * tile + kWFloats;
+        const int pitch = pitch_of(D);
+        if (group == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float sum = row_sum(l[i]);
+                const int r = ln.g + 8 * i;
+                store_row<NC>(part + r * pitch, z, i, 1.f, 0, D, D % 2 == 0, ln);
+                if (ln.h == 0) ml[2 * r] = m[i], ml[2 * r + 1] = sum;
+            }
+        }
+        f32_cluster_sync();
+        const int rows = kRows / split;
+        for (int i = (int)threadIdx.x; i < rows * D; i += kGroup * G) {
+            const int r = rank * rows + i / D, d = i % D;
+            if (row0 + r >= p.seq_q) break;  // (rows ascend)
+            float ms[8], ls[8], zs[8], mm = -INFINITY;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (c < split) {
+                    ms[c] = f32_remote(ml + 2 * r, c);
+                    ls[c] = f32_remote(ml + 2 * r + 1, c);
+                    zs[c] = f32_remote(part + r * pitch + d, c);
+                    mm = fmaxf(mm, ms[c]);
+                }
+            const float m_use = (mm == -INFINITY) ? 0.f : mm;
+            float sum = 0.f, o = 0.f;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (c < split) {
+                    const float w = exp2f(ms[c] - m_use);
+                    sum = fmaf(ls[c], w, sum);  // (a NaN sum stays one: NaN * 0)
+                    o = fmaf(zs[c], w, o);
+                }
+            const bool ok = (sum > 0.f) && isfinite(sum);  // cpu_forward.rs:411
+            const int64_t qi = row0 + r;
+            p.out[(bh * p.seq_q + qi) * D + d] = o * (ok ? 1.f / sum : NAN);
+            if (p.lse && d == 0)
+                p.lse[bh * p.seq_q + qi] = (sum > 0.f) ? fmaf(mm, kLn2, logf(sum)) : (sum == 0.f ? -INFINITY : NAN);
+        }
+        f32_cluster_sync();  // no CTA leaves while its partial rows are being read
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const float sum = row_sum(l[i]);
@@ -288,21 +352,96 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
     }
 }
 
-template <int NC, int G>
-static cudaError_t launch_tiled(const SimtParams& p, int64_t batch, cudaStream_t stream) {
-    auto bytes = [](int dim) {
-        return sizeof(float) * ((1 + 2 * G) * (size_t)simt::tile_floats(simt::kRows, dim) + G * (size_t)simt::kWFloats);
-    };
+static size_t f32_tiled_bytes(int G, int dim) {
+    return sizeof(float) * ((1 + 2 * G) * (size_t)simt::tile_floats(simt::kRows, dim) + G * (size_t)simt::kWFloats);
+}
+
+template <int NC, int G, bool kSplit>
+static cudaError_t launch_tiled_s(const SimtParams& p, int64_t n, bool vec, bool pairs, int64_t row_blocks, cudaStream_t stream) {
     // the limit of the widest head dim of this instantiation, so that it is set once
-    cudaError_t e = set_max_dynamic_smem_once<prefill_f32_tiled_kernel<NC, G>>((int)bytes(NC * 32));
+    cudaError_t e = set_max_dynamic_smem_once<prefill_f32_tiled_kernel<NC, G, kSplit>>((int)f32_tiled_bytes(G, NC * 32));
     if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n * p.split));
+    cfg.blockDim = dim3(simt::kGroup * G);
+    cfg.dynamicSmemBytes = f32_tiled_bytes(G, p.dim);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    if (kSplit) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)p.split;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&cfg, prefill_f32_tiled_kernel<NC, G, kSplit>, p, vec, pairs, row_blocks);
+}
+
+// CTAs that clusters of `split` CTAs of the widest kernel can have resident on the current device (one CTA per SM; GPCs hold
+// whole clusters only).  Asked once per device and size.
+static int f32_cluster_slots(int split) {
+    static std::atomic<int> known[64][3];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::atomic<int>& slot = known[dev][split == 2 ? 0 : split == 4 ? 1 : 2];
+    const int have = slot.load(std::memory_order_relaxed);
+    if (have > 0) return have - 1;
+    int n = 0;
+    if (set_max_dynamic_smem_once<prefill_f32_tiled_kernel<4, 2, true>>((int)f32_tiled_bytes(2, 128)) == cudaSuccess) {
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)split;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(split * 256));
+        cfg.blockDim = dim3(simt::kGroup * 2);
+        cfg.dynamicSmemBytes = f32_tiled_bytes(2, 128);
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, prefill_f32_tiled_kernel<4, 2, true>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+    }
+    slot.store(n * split + 1, std::memory_order_relaxed);
+    return n * split;
+}
+
+template <int NC, int G>
+static cudaError_t launch_tiled(SimtParams p, int64_t batch, cudaStream_t stream) {
     const int64_t row_blocks = (p.seq_q + simt::kRows - 1) / simt::kRows, n = row_blocks * p.heads_q * batch;
     if (n > 0x7fffffff) return cudaErrorInvalidValue;
     const uintptr_t in = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v);
     const bool vec = p.dim % 4 == 0 && (in & 15) == 0;
     const bool pairs = p.dim % 2 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 7) == 0;
-    prefill_f32_tiled_kernel<NC, G><<<(unsigned)n, simt::kGroup * G, bytes(p.dim), stream>>>(p, vec, pairs, row_blocks);
-    return cudaGetLastError();
+    // How many CTAs share the keys of a row block: the launch lasts as long as its longest CTA or as the SMs' share of all,
+    // whichever is more (causal blocks are started heaviest first and fill up to within 8 %, equal ones come in whole waves).
+    // In us: a step of 64 keys per group, per CTA, and for the merge across a cluster.
+    p.split = 1;
+    if constexpr (G == 2) {
+        if (n < 2 * (int64_t)sm_count()) {
+            const double step = 1.0 + 0.1 * p.dim, cta = 3.0, merge = 4.0;
+            const int64_t all = (p.seq_kv + simt::kRows - 1) / simt::kRows,
+                          off = p.causal && p.q_offsets && p.seq_kv > p.seq_q ? p.seq_kv - p.seq_q : 0;
+            double best = 0;
+            for (int c = 1; c <= 8; c *= 2) {
+                const int64_t slots = c == 1 ? sm_count() : f32_cluster_slots(c) / c;
+                if (slots == 0 || all < 2 * c) break;
+                double sum = 0, mx = 0;
+                for (int64_t i = 0; i < row_blocks; ++i) {
+                    const int64_t tiles = p.causal ? std::min(all, (off + std::min((i + 1) * simt::kRows, p.seq_q) + simt::kRows - 1) / simt::kRows) : all;
+                    const double t = (double)((tiles + 2 * c - 1) / (2 * c)) * step + cta + (c > 1 ? merge : 0.0);
+                    sum += t;
+                    mx = std::max(mx, t);
+                }
+                const int64_t heads = n / row_blocks;
+                const double t = p.causal ? std::max(mx, 1.08 * sum * (double)heads / (double)slots) : mx * (double)((n + slots - 1) / slots);
+                if (c == 1 || t < best) best = t, p.split = c;
+            }
+        }
+        if (p.split > 1) return launch_tiled_s<NC, G, true>(p, n, vec, pairs, row_blocks, stream);
+    }
+    return launch_tiled_s<NC, G, false>(p, n, vec, pairs, row_blocks, stream);
 }
 
 cudaError_t launch_prefill_f32(const float* q, const float* k, const float* v, float* out, float* lse,
@@ -312,7 +451,7 @@ cudaError_t launch_prefill_f32(const float* q, const float* k, const float* v, f
                                float scale, cudaStream_t stream) {
     if (batch == 0 || heads_q == 0 || seq_q == 0) return cudaSuccess;
     SimtParams p{q, k, v, out, lse, heads_q, heads_kv, seq_q, seq_kv, dim, causal, kv_lens, q_offsets, key_keep,
-                 keep_batch_stride, scale};
+                 keep_batch_stride, scale, 1};
     // The register-tiled kernel is the path for 16 query rows and more; a decode-shaped call (a few rows against
     // a long cache) would waste most of its 64-row tile and keeps the warp-per-row kernel, which
     // RT_ATTN_PREFILL_F32_IMPL=rows selects for every shape (comparisons).
