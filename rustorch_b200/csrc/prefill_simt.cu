@@ -339,7 +339,7 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
         }
         f32_cluster_sync();  // no CTA leaves while its partial rows are being read
         return;
-    }
+    } else {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const float sum = row_sum(l[i]);
@@ -349,6 +349,7 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
         store_row<NC>(p.out + (bh * p.seq_q + qi) * D, z, i, ok ? 1.f / sum : NAN, 0, D, pairs, ln);
         if (p.lse && ln.h == 0)
             p.lse[bh * p.seq_q + qi] = (sum > 0.f) ? fmaf(m[i], kLn2, logf(sum)) : (sum == 0.f ? -INFINITY : NAN);
+    }
     }
 }
 
