@@ -295,9 +295,10 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
     }
 
     if constexpr (kSplit) {
-        // ---- the cluster's partial rows, over the Q tile; (max, sum) of each where the second group's tiles were
+        // ---- the cluster's partial rows, over the Q tile; (max, sum) of each behind what the groups have exchanged, which
+        // other warps may still be reading (at head dims of 8 and less that reaches into the second group's tiles)
         float* const part = Qs;
-        float* const ml = smem + tile + 2 * tile + kWFloats;
+        float* const ml = Qs + tile + (8 * NC + 8) * 2 * kGroup;
         const int pitch = pitch_of(D);
         if (group == 0) {
 #pragma unroll
