@@ -37,6 +37,10 @@ __global__ void __launch_bounds__(256) bwd_delta_kernel(const float* __restrict_
     if (lane == 0) delta[row] = acc;
 }
 
+// Tiles hold whole rows: the gradient columns of a launch with one column group, all 256 with two.
+template <int NC, int G>
+__host__ __device__ constexpr int bwd_pitch() { return simt::pitch_of(G == 1 ? 256 : NC * 32); }
+
 // One CTA's 64 rows of one side.  X1, X2 are its own rows of (Q, dO) or (K, V), Y1, Y2 the other side's tiles of
 // (K, V) or (Q, dO), 16 J rows at a time; col0 is the first of the NC x 32 gradient columns it accumulates.
 // Every step computes dP (Y2) before S (Y1) and accumulates with Y2 before Y1, so each single-buffered tile is
@@ -48,7 +52,7 @@ __device__ __forceinline__ void bwd_rows(const BwdParams& p, float* smem, int64_
     using namespace simt;
     const int D = p.dim;
     const int group = G == 1 ? 0 : (int)threadIdx.x >> 7, tid = (int)threadIdx.x & (kGroup - 1);
-    const int x_tile = tile_floats(kRows, D), y_tile = tile_floats(16 * J, D);
+    constexpr int kPitch = bwd_pitch<NC, G>(), x_tile = tile_floats(kRows, kPitch), y_tile = tile_floats(16 * J, kPitch);
     float* X1 = smem;
     float* X2 = X1 + x_tile;
     float* Y1 = X2 + x_tile + group * (2 * y_tile + kWFloats);
@@ -67,9 +71,9 @@ __device__ __forceinline__ void bwd_rows(const BwdParams& p, float* smem, int64_
     const int64_t t_hi = (!kKeySide && p.causal && own0 + kRows < N) ? own0 + kRows : N;
 
     const int64_t first = t_lo + group * 16 * J, step = (int64_t)G * 16 * J;
-    load_tile<kRows, kGroup * G>(X1, (kKeySide ? p.k : p.q) + base, own0, N, D, vec, x_share);
-    load_tile<kRows, kGroup * G>(X2, (kKeySide ? p.v : p.d_out) + base, own0, N, D, vec, x_share);
-    if (first < t_hi) load_tile<16 * J, kGroup>(Y2, oth2, first, N, D, vec, share);
+    load_tile<kRows, kGroup * G, kPitch>(X1, (kKeySide ? p.k : p.q) + base, own0, N, D, vec, x_share);
+    load_tile<kRows, kGroup * G, kPitch>(X2, (kKeySide ? p.v : p.d_out) + base, own0, N, D, vec, x_share);
+    if (first < t_hi) load_tile<16 * J, kGroup, kPitch>(Y2, oth2, first, N, D, vec, share);
     cp_async_commit();
 
     // LSE in units of log2.  A row without a visible key has LSE = -inf: +inf in its place makes every probability 0.
@@ -107,17 +111,17 @@ __device__ __forceinline__ void bwd_rows(const BwdParams& p, float* smem, int64_
         }
         cp_async_wait<0>();
         group_sync(group);  // Y2 is visible, the last step's Y1 is free
-        load_tile<16 * J, kGroup>(Y1, oth1, t0, N, D, vec, share);
+        load_tile<16 * J, kGroup, kPitch>(Y1, oth1, t0, N, D, vec, share);
         cp_async_commit();
         float dp[8][J], pr[8][J];
-        product<J>(dp, X2, Y2, D, ln);
+        product<J, kPitch>(dp, X2, Y2, D, ln);
         cp_async_wait<0>();
         group_sync(group);  // Y1 is visible (and, on the query side, Y2 free)
         if (!kKeySide && more) {
-            load_tile<16 * J, kGroup>(Y2, oth2, t0 + step, N, D, vec, share);
+            load_tile<16 * J, kGroup, kPitch>(Y2, oth2, t0 + step, N, D, vec, share);
             cp_async_commit();
         }
-        product<J>(pr, X1, Y1, D, ln);
+        product<J, kPitch>(pr, X1, Y1, D, ln);
 
 #pragma unroll
         for (int i = 0; i < 8; ++i)
@@ -140,14 +144,14 @@ __device__ __forceinline__ void bwd_rows(const BwdParams& p, float* smem, int64_
 #pragma unroll
             for (int j = 0; j < J; ++j) dp[i][j] = pr[i][j] * (dp[i][j] - (kKeySide ? c_delta[j] : r_delta[i]));
         if constexpr (kKeySide) {
-            accumulate<J, NC>(z2, pr, Y2 + col0, D, Ws, ln);  // dV += P^T dO
+            accumulate<J, NC, kPitch>(z2, pr, Y2 + col0, Ws, ln);  // dV += P^T dO
             group_sync(group);                                // Y2 is free
             if (more) {
-                load_tile<16 * J, kGroup>(Y2, oth2, t0 + step, N, D, vec, share);
+                load_tile<16 * J, kGroup, kPitch>(Y2, oth2, t0 + step, N, D, vec, share);
                 cp_async_commit();
             }
         }
-        accumulate<J, NC>(z1, dp, Y1 + col0, D, Ws, ln);  // dQ += dS K, or dK += dS^T Q
+        accumulate<J, NC, kPitch>(z1, dp, Y1 + col0, Ws, ln);  // dQ += dS K, or dK += dS^T Q
     }
 
     if (G == 2) {
@@ -178,7 +182,7 @@ __device__ __forceinline__ void bwd_rows(const BwdParams& p, float* smem, int64_
 
 // CTA order: rank (0 = most other-side tiles under a causal mask), then side, column group, head.
 // Against the kernel that gave every own row to one warp (a shared-memory load per multiply-add): B=2 H=8 N=1000 D=64
-// causal 1814 -> 205 us, B=4 H=16 N=1024 D=64 12.1 -> 1.47 ms (41 TFLOP/s executed), B=4 H=16 N=161 D=80 312 -> 63 us.
+// causal 1814 -> 193 us, B=4 H=16 N=1024 D=64 12.1 -> 1.35 ms (45 TFLOP/s executed), B=4 H=16 N=161 D=80 causal 312 -> 62 us.
 // Scalar multiply-adds in place of the packed ones were 4 % slower, one group per CTA (two CTAs an SM) 15 % at N=1000.
 template <int NC, int J, int G>
 __global__ void __launch_bounds__(simt::kGroup * G, 1)
@@ -196,11 +200,10 @@ bwd_tiled_kernel(const BwdParams p, const bool vec, const bool pairs, const int 
 
 template <int NC, int J, int G>
 static cudaError_t launch_bwd_tiled(const BwdParams& p, int64_t bh, cudaStream_t stream) {
-    auto bytes = [](int dim) {
-        return sizeof(float) * (2 * (size_t)simt::tile_floats(simt::kRows, dim) +
-                                G * (2 * (size_t)simt::tile_floats(16 * J, dim) + simt::kWFloats));
-    };
-    cudaError_t e = set_max_dynamic_smem_once<bwd_tiled_kernel<NC, J, G>>((int)bytes(G == 1 ? 256 : NC * 32));
+    constexpr int kPitch = bwd_pitch<NC, G>(),
+                  bytes = (int)sizeof(float) * (2 * simt::tile_floats(simt::kRows, kPitch) +
+                                                G * (2 * simt::tile_floats(16 * J, kPitch) + simt::kWFloats));
+    cudaError_t e = set_max_dynamic_smem_once<bwd_tiled_kernel<NC, J, G>>(bytes);
     if (e != cudaSuccess) return e;
     const int64_t n_tiles = (p.seq + simt::kRows - 1) / simt::kRows;
     const int groups = (p.dim + NC * 32 - 1) / (NC * 32);
@@ -210,7 +213,7 @@ static cudaError_t launch_bwd_tiled(const BwdParams& p, int64_t bh, cudaStream_t
                          reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.d_out);
     const uintptr_t outs = reinterpret_cast<uintptr_t>(p.dq) | reinterpret_cast<uintptr_t>(p.dk) | reinterpret_cast<uintptr_t>(p.dv);
     const bool vec = p.dim % 4 == 0 && (in & 15) == 0, pairs = p.dim % 2 == 0 && (outs & 7) == 0;
-    bwd_tiled_kernel<NC, J, G><<<(unsigned)n, simt::kGroup * G, bytes(p.dim), stream>>>(p, vec, pairs, (int)n_tiles,
+    bwd_tiled_kernel<NC, J, G><<<(unsigned)n, simt::kGroup * G, bytes, stream>>>(p, vec, pairs, (int)n_tiles,
                                                                                          (int)bh, groups);
     return cudaGetLastError();
 }

@@ -145,11 +145,12 @@ __global__ void __launch_bounds__(kSimtRows * 32) prefill_f32_kernel(const SimtP
 // next tile is copied while P V runs, V while Q K^T runs, so two group barriers per tile order everything.  The row
 // sum stays per thread until the end.  NC = ceil(D / 32) column groups of the output.
 // Against the 256-thread kernel with 4 x 4 scores a thread that this replaces (scalar loads transposed into shared
-// memory with 16-way conflicts): B=1 H=8 N=2048 D=64 causal 371 -> 120 us (36 TFLOP/s), B=2 H=16 N=1000 D=128 causal
-// 520 -> 232 us, B=4 H=16 N=1024 D=64 656 -> 435 us (40 TFLOP/s of the FP32 pipe's 74).
+// memory with 16-way conflicts): B=1 H=8 N=2048 D=64 causal 371 -> 113 us (38 TFLOP/s), B=2 H=16 N=1000 D=128 causal
+// 520 -> 218 us, B=4 H=16 N=1024 D=64 656 -> 408 us (42 TFLOP/s of the FP32 pipe's 74).
 // Launches of few row blocks leave SMs idle while each block walks its keys alone; there a cluster of 2, 4 or 8 CTAs shares
 // them (kSplit): each takes every split-th pair of tiles, leaves its partial rows in shared memory, and merges 64 / split rows out
-// of all of them.  (N=2048 D=64 causal, H=1 121 -> 40 us, H=2 122 -> 71; B=1 H=4 N=600 D=80 56 -> 44; the merge costs about half a step.)
+// of all of them.  (N=2048 D=64 causal, H=1 121 -> 40 us, H=2 122 -> 55; B=1 H=4 N=600 D=80 56 -> 44, 38, 52 and 41 since; the merge costs about half
+// a step.)
 __device__ __forceinline__ void f32_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -167,7 +168,8 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
     using namespace simt;
     extern __shared__ __align__(16) float smem[];
     const int group = G == 1 ? 0 : (int)threadIdx.x >> 7, tid = (int)threadIdx.x & (kGroup - 1);
-    const int D = p.dim, tile = tile_floats(kRows, D);
+    constexpr int kPitch = pitch_of(NC * 32), tile = tile_floats(kRows, kPitch);
+    const int D = p.dim;
     float* Qs = smem;
     float* Ks = Qs + tile + group * (2 * tile + kWFloats);
     float* Vs = Ks + tile;
@@ -211,22 +213,22 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
         for (int c = 0; c < 2 * NC; ++c) z[r][c] = make_float2(0.f, 0.f);
 
     const int64_t first = (int64_t)(rank * G + group) * kRows, step = (int64_t)(G * split) * kRows;
-    load_tile<kRows, kGroup * G>(Qs, p.q + (bh * p.seq_q) * D, row0, p.seq_q, D, vec, q_share);
-    if (first < k_loop) load_tile<kRows, kGroup>(Ks, kptr, first, k_hi, D, vec, share);
+    load_tile<kRows, kGroup * G, kPitch>(Qs, p.q + (bh * p.seq_q) * D, row0, p.seq_q, D, vec, q_share);
+    if (first < k_loop) load_tile<kRows, kGroup, kPitch>(Ks, kptr, first, k_hi, D, vec, share);
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();  // both groups have copied their share of Q
     for (int64_t kj = first; kj < k_loop; kj += step) {
         cp_async_wait<0>();
         group_sync(group);  // this tile's K is visible and nobody reads the last tile's V any more
-        load_tile<kRows, kGroup>(Vs, vptr, kj, k_hi, D, vec, share);
+        load_tile<kRows, kGroup, kPitch>(Vs, vptr, kj, k_hi, D, vec, share);
         cp_async_commit();
         float s[8][4];
-        product<4>(s, Qs, Ks, D, ln);
+        product<4, kPitch>(s, Qs, Ks, D, ln);
         cp_async_wait<0>();
         group_sync(group);  // V is visible, K is free
         if (kj + step < k_loop) {
-            load_tile<kRows, kGroup>(Ks, kptr, kj + step, k_hi, D, vec, share);
+            load_tile<kRows, kGroup, kPitch>(Ks, kptr, kj + step, k_hi, D, vec, share);
             cp_async_commit();
         }
         // ---- masks, in tiles that the length, the diagonal or flags cut
@@ -262,7 +264,7 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int c = 0; c < 2 * NC; ++c) z[r][c] = __fmul2_rn(z[r][c], alpha[r]);
-        accumulate<4, NC>(z, s, Vs, D, Ws, ln);
+        accumulate<4, NC, kPitch>(z, s, Vs, Ws, ln);
     }
 
     // ---- the two groups' partial rows: the second hands over (max, per-thread sum, output), the first merges
@@ -299,13 +301,12 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
         // other warps may still be reading (at head dims of 8 and less that reaches into the second group's tiles)
         float* const part = Qs;
         float* const ml = Qs + tile + (8 * NC + 8) * 2 * kGroup;
-        const int pitch = pitch_of(D);
         if (group == 0) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float sum = row_sum(l[i]);
                 const int r = ln.g + 8 * i;
-                store_row<NC>(part + r * pitch, z, i, 1.f, 0, D, D % 2 == 0, ln);
+                store_row<NC>(part + r * kPitch, z, i, 1.f, 0, D, D % 2 == 0, ln);
                 if (ln.h == 0) ml[2 * r] = m[i], ml[2 * r + 1] = sum;
             }
         }
@@ -320,7 +321,7 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
                 if (c < split) {
                     ms[c] = f32_remote(ml + 2 * r, c);
                     ls[c] = f32_remote(ml + 2 * r + 1, c);
-                    zs[c] = f32_remote(part + r * pitch + d, c);
+                    zs[c] = f32_remote(part + r * kPitch + d, c);
                     mm = fmaxf(mm, ms[c]);
                 }
             const float m_use = (mm == -INFINITY) ? 0.f : mm;
@@ -354,19 +355,19 @@ prefill_f32_tiled_kernel(const SimtParams p, const bool vec, const bool pairs, c
     }
 }
 
-static size_t f32_tiled_bytes(int G, int dim) {
-    return sizeof(float) * ((1 + 2 * G) * (size_t)simt::tile_floats(simt::kRows, dim) + G * (size_t)simt::kWFloats);
+template <int NC, int G>
+constexpr int f32_tiled_bytes() {
+    return (int)sizeof(float) * ((1 + 2 * G) * simt::tile_floats(simt::kRows, simt::pitch_of(NC * 32)) + G * simt::kWFloats);
 }
 
 template <int NC, int G, bool kSplit>
 static cudaError_t launch_tiled_s(const SimtParams& p, int64_t n, bool vec, bool pairs, int64_t row_blocks, cudaStream_t stream) {
-    // the limit of the widest head dim of this instantiation, so that it is set once
-    cudaError_t e = set_max_dynamic_smem_once<prefill_f32_tiled_kernel<NC, G, kSplit>>((int)f32_tiled_bytes(G, NC * 32));
+    cudaError_t e = set_max_dynamic_smem_once<prefill_f32_tiled_kernel<NC, G, kSplit>>(f32_tiled_bytes<NC, G>());
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n * p.split));
     cfg.blockDim = dim3(simt::kGroup * G);
-    cfg.dynamicSmemBytes = f32_tiled_bytes(G, p.dim);
+    cfg.dynamicSmemBytes = f32_tiled_bytes<NC, G>();
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     if (kSplit) {
@@ -389,7 +390,7 @@ static int f32_cluster_slots(int split) {
     const int have = slot.load(std::memory_order_relaxed);
     if (have > 0) return have - 1;
     int n = 0;
-    if (set_max_dynamic_smem_once<prefill_f32_tiled_kernel<4, 2, true>>((int)f32_tiled_bytes(2, 128)) == cudaSuccess) {
+    if (set_max_dynamic_smem_once<prefill_f32_tiled_kernel<4, 2, true>>(f32_tiled_bytes<4, 2>()) == cudaSuccess) {
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = (unsigned)split;
@@ -397,7 +398,7 @@ static int f32_cluster_slots(int split) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(split * 256));
         cfg.blockDim = dim3(simt::kGroup * 2);
-        cfg.dynamicSmemBytes = f32_tiled_bytes(2, 128);
+        cfg.dynamicSmemBytes = f32_tiled_bytes<4, 2>();
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         if (cudaOccupancyMaxActiveClusters(&n, prefill_f32_tiled_kernel<4, 2, true>, &cfg) != cudaSuccess) {

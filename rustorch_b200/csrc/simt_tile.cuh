@@ -12,8 +12,12 @@
 //     16-byte bank groups;
 //   * a score row lives in 16 lanes of one warp: the row maximum is four shuffles, and the scores reach the second
 //     product through a warp-private piece of shared memory without a CTA barrier.
-// Bound: the FP32 pipe (128 multiply-adds per clock and SM) and, next to it, shared-memory wavefronts; with two warps
-// per scheduler the products run at three quarters of the pipe.
+// Bound: the FP32 pipe (128 multiply-adds per clock and SM) and, next to it, shared-memory wavefronts (2.7 per 16-byte read);
+// with two warps per scheduler the products run at three quarters of the pipe.  What two warps do not hide is the latency of
+// the first reads behind a loop's end and the integer work on row addresses: products unrolled 4 and 16 deep over tiles of
+// constant pitch take 6 % less than 2 and 4 deep over a pitch that follows the head dim.  (8 deep, or the next step's operands
+// read ahead, spill: level and 2 % slower.  A third group at 168 registers 3 % slower; lanes h and h ^ 8 sharing 8 x 8
+// scores over half of d each, a third fewer reads per multiply-add but scalar ones, 6 %.)
 #pragma once
 #include "common.cuh"
 
@@ -24,13 +28,11 @@ constexpr int kGroup = 128, kRows = 64;
 constexpr int kWKeys = 32, kWPitch = 20;                // one warp's exchange buffer: [32 keys][16 rows + pad]
 constexpr int kWFloats = 4 * kWKeys * kWPitch;          // of a group
 
-// Floats between rows of a tile: D rounded up to 4, then to an odd multiple of 4.
-__host__ __device__ inline int pitch_of(int dim) {
-    const int d4 = (dim + 3) / 4;
-    return 4 * (d4 | 1);
-}
-// Floats of a tile; the slack covers the column groups of the accumulating product beyond the last row's end.
-__host__ __device__ inline int tile_floats(int rows, int dim) { return rows * pitch_of(dim) + 32; }
+// Floats between rows of a tile for head dims up to `cols`, an odd multiple of 4.  It is a constant of the kernel, not of
+// the call: row offsets are immediates of the loads then and take no registers.
+__host__ __device__ constexpr int pitch_of(int cols) { return 4 * ((cols + 3) / 4 | 1); }
+// Floats of a tile.
+__host__ __device__ constexpr int tile_floats(int rows, int pitch) { return rows * pitch; }
 
 struct Lane {
     int warp, g, h;
@@ -93,10 +95,9 @@ struct Share {
 // Starts the copy of rows [r0, r0 + kTileRows) of a [n_rows, dim] matrix; rows beyond n_rows and the padding up to a
 // multiple of 4 columns become zero.  vec: dim is a multiple of 4 and the matrix 16-byte aligned.  The copy is the work
 // of kThreads threads, each doing its share; the caller commits.
-template <int kTileRows, int kThreads>
+template <int kTileRows, int kThreads, int pitch>
 __device__ __forceinline__ void load_tile(float* tile, const float* src, int64_t r0, int64_t n_rows, int dim, bool vec,
                                           const Share& sh) {
-    const int pitch = pitch_of(dim);
     const int n = (int)(n_rows - r0 < kTileRows ? n_rows - r0 : kTileRows);  // rows that exist (may be negative)
     if (vec) {
         const float* g = src + r0 * dim + sh.c * 4;
@@ -113,9 +114,9 @@ __device__ __forceinline__ void load_tile(float* tile, const float* src, int64_t
 }
 
 // t[i][j] = sum over d of X[g + 8 i][d] Y[h + 16 j][d].  Even and odd d accumulate in the two halves of an f32x2.
-template <int J>
+template <int J, int pitch>
 __device__ __forceinline__ void product(float (&t)[8][J], const float* X, const float* Y, int dim, const Lane& ln) {
-    const int pitch = pitch_of(dim), steps = (dim + 3) / 4;
+    const int steps = (dim + 3) / 4;
     const float* x = X + ln.g * pitch;
     const float* y = Y + ln.h * pitch;
     float2 acc[8][J];
@@ -123,7 +124,7 @@ __device__ __forceinline__ void product(float (&t)[8][J], const float* X, const 
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < J; ++j) acc[i][j] = make_float2(0.f, 0.f);
-#pragma unroll 2
+#pragma unroll 4
     for (int s = 0; s < steps; ++s) {
         float4 b[J];
 #pragma unroll
@@ -146,10 +147,9 @@ __device__ __forceinline__ void product(float (&t)[8][J], const float* X, const 
 
 // z[p][c] (+)= sum over the other tile's rows k of t[row][k] Y[k][col]: p = row pair (g + 16 p, g + 16 p + 8), c = 2 cc + e
 // stands for column pair_col(cc) + e.  t goes through the warp's exchange buffer, 32 rows of Y at a time.
-template <int J, int NC>
-__device__ __forceinline__ void accumulate(float2 (&z)[4][2 * NC], const float (&t)[8][J], const float* Y, int dim,
-                                           float* w_sm, const Lane& ln) {
-    const int pitch = pitch_of(dim);
+template <int J, int NC, int pitch>
+__device__ __forceinline__ void accumulate(float2 (&z)[4][2 * NC], const float (&t)[8][J], const float* Y, float* w_sm,
+                                           const Lane& ln) {
     float* w = w_sm + ln.warp * kWKeys * kWPitch;
     const float* wr = w + (ln.g & 1) * 8;
 #pragma unroll
@@ -164,7 +164,7 @@ __device__ __forceinline__ void accumulate(float2 (&z)[4][2 * NC], const float (
         }
         __syncwarp();
         const float* y = Y + half * 32 * pitch;
-#pragma unroll 4
+#pragma unroll 16
         for (int k = 0; k < kWKeys; ++k) {
             const float4 a = *reinterpret_cast<const float4*>(wr + k * kWPitch);
             const float4 b = *reinterpret_cast<const float4*>(wr + k * kWPitch + 4);
