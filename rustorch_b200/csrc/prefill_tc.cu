@@ -25,8 +25,8 @@
 // steps; P (bf16) overwrites the first 32 columns of its S buffer and feeds the PV MMA from TMEM.
 // S = Q K^T is an SS MMA with both operands K-major in 128-byte-swizzled shared memory; O += P V
 // is a TS MMA whose B operand (V) is MN-major, i.e. V is used exactly as TMA lands it.
-// The normalised O tile is staged in the tile's own (by then idle) Q buffer and leaves through
-// TMA stores.  Every mbarrier wait is bounded; on expiry the kernel records a code in the device
+// The normalised O tile is staged in shared memory (at D = 64 in a buffer of its own, at D = 128, where the rings
+// leave no room, in the tile's by then idle Q buffer) and leaves through TMA stores.  Every mbarrier wait is bounded; on expiry the kernel records a code in the device
 // status word, drains its own copies and MMAs, frees TMEM and returns.
 #include <algorithm>
 #include <atomic>
@@ -315,12 +315,14 @@ __device__ __forceinline__ void merge_cluster(const TcParams& p, const TcItem& i
 // Pipeline, per Q tile w and 64-key step u (buffer b = u & 1):
 //   MMA:     S_w(u) -> TMEM S[w][b]            (SS, N = 64, D/16 k-steps)       commit s_full[w][b]
 //   softmax: S[w][b] -> registers -> P (bf16) over the first 32 columns of S[w][b]   arrive p_full[w][b]
-//   MMA:     O_w += P V(u)                      (TS, N = D, 4 k-steps)           commit o_full[w]
-//            then S_w(u+2) into the same buffer (in-order after the PV that read P from it)
-// S is double-buffered, so the softmax of step u+1 never waits for the PV of step u.
+//   MMA:     O_w += P V(u)                      (TS, N = D, 4 k-steps)
+//            then S_w(u+2) into the same buffer (in-order after the PV that read P from it)   commit s_full[w][b]
+// S is double-buffered, so the softmax of step u+1 never waits for the PV of step u.  One commit a step: S_w(u+2) has
+// retired only if PV(u) has, so a softmax warp that moves the reference maximum at step u+1 reads 'O is at rest' off
+// the barrier of the next scores; only an item's last step but one has a commit for it (o_full).
 // Per item and tile: q_full (Q landed) -> ... -> o_done (last PV retired) -> epilogue reads O
-// (o_free: the next item's first PV may overwrite it), stages it in the Q buffer (stage_full),
-// one thread stores it (q_empty: the next item's Q may land).  A tile that sees no key in an
+// (o_free: the next item's first PV may overwrite it), stages it (stage_full), and one thread stores it.  q_empty, the
+// next item's Q may land: at D = 64 behind the item's last score MMA, at D = 128 when the store has read the staged tile.  A tile that sees no key in an
 // item takes no part in these (its rows are written as NaN directly).
 template <int D, bool kCausal, bool kKeep, bool kSingle, bool kSplit, bool kByLength>
 __global__ void __launch_bounds__(384, 1)
