@@ -284,7 +284,13 @@ __device__ __forceinline__ void merge_decode_cluster(const DecodeTcParams& p, in
         const bool any = l > 0.f;
         o = any ? make_float4(o.x / l, o.y / l, o.z / l, o.w / l) : make_float4(0.f, 0.f, 0.f, 0.f);
         const int64_t row = row0 + gg;
-        if (p.out_bf16) *reinterpret_cast<uint2*>(p.out_bf16 + row * D + d) = make_uint2(float2_to_bf16x2(o.x, o.y), float2_to_bf16x2(o.z, o.w));
+        if (p.out_bf16) {  // (only its element size is asked of the output's address)
+            __nv_bfloat16* dst = p.out_bf16 + row * D + d;
+            if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0)
+                *reinterpret_cast<uint2*>(dst) = make_uint2(float2_to_bf16x2(o.x, o.y), float2_to_bf16x2(o.z, o.w));
+            else
+                dst[0] = __float2bfloat16(o.x), dst[1] = __float2bfloat16(o.y), dst[2] = __float2bfloat16(o.z), dst[3] = __float2bfloat16(o.w);
+        }
         if (p.out_f32) {
             float* dst = p.out_f32 + row * p.of_stride + d;  // (records: rows of D + 1 floats)
             dst[0] = o.x, dst[1] = o.y, dst[2] = o.z, dst[3] = o.w;

@@ -43,6 +43,23 @@ def test_cluster_parts(oracle, D, G, Hkv):
     util.check_lse(util.to_np(lse1), ref_lse[-1:])
 
 
+@pytest.mark.parametrize("offset", [1, 2, 3])
+@pytest.mark.parametrize("n,D", [(1000, 64), (1000, 128), (1000, 256), (40, 128)])
+def test_output_of_any_element_alignment(n, D, offset):
+    """An output that starts 1, 2 or 3 elements into a buffer gets the bits of an aligned one: lengths that clusters take,
+    and one that a single CTA does."""
+    import torch
+    import rustorch_b200 as rt
+    g = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v = (torch.randn(s, dtype=torch.bfloat16, device="cuda", generator=g) for s in ((2, 8, D), (2, 2, n, D), (2, 2, n, D)))
+    want, _ = rt.gqa_decode(q, k, v, kv_len=n)
+    buf = torch.full((q.numel() + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
+    out, _ = rt.gqa_decode(q, k, v, kv_len=n, out=buf[offset:offset + q.numel()].view(q.shape))
+    torch.cuda.synchronize()
+    assert out.data_ptr() % 8 == 2 * offset and torch.equal(out, want)
+    assert bool((buf[:offset] == 7.0).all()) and bool((buf[offset + q.numel():] == 7.0).all())
+
+
 @pytest.mark.skipif("RT_ATTN_DECODE_CLUSTER" in os.environ, reason="the child process itself")
 @pytest.mark.parametrize("size", ["2", "4", "8", "16"])
 def test_every_cluster_size(size):
