@@ -947,7 +947,10 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
     if (span < 1) span = 1;
     const bool tc = decode_use_tensor_cores() && batch * n_kv * max_seq < (1ll << 31) - 64;
     p.split = pick_split(batch, n_kv, head_dim, max_seq, span, kv_lens != nullptr);
-    if (tc) {
+    // A cluster's record goes to the peers through the copy kernel, whose 16-byte pieces want it aligned; merge_partials_kernel
+    // delivers a record at any address.
+    const bool record_aligned = !push || (reinterpret_cast<uintptr_t>(out_f32) & 15) == 0;
+    if (tc && record_aligned) {
         const int64_t groups = batch * n_kv, slots = (int64_t)sm_count() * (head_dim == 64 ? 4 : head_dim == 128 ? 2 : 1);
         pick_cluster(p.split, groups, head_dim, span, kv_lens != nullptr && batch > 1, std::max<int64_t>(1, slots / groups));
     }

@@ -60,6 +60,37 @@ def test_output_of_any_element_alignment(n, D, offset):
     assert bool((buf[:offset] == 7.0).all()) and bool((buf[offset + q.numel():] == 7.0).all())
 
 
+def test_pushed_record_of_any_alignment():
+    """rt_gqa_decode_record_push_bf16 with a record that is no slot and lies 4 to 12 bytes off a 16-byte boundary: taken at a
+    length that clusters serve for an aligned one, delivered to every peer, and equal up to the roundings of P."""
+    import ctypes
+    import torch
+    import rustorch_b200 as rt
+    from rustorch_b200 import _lib
+    B, Hq, Hkv, D, S, world = 1, 8, 2, 128, 1000, 2
+    rows = B * Hq
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn(s, dtype=torch.bfloat16, device="cuda", generator=g) for s in ((B, Hq, D), (B, Hkv, S, D), (B, Hkv, S, D)))
+    want = rt.gqa_decode_record(q, k, v, kv_len=S)
+    ws = torch.empty(rt.decode_workspace_bytes(B, Hq, Hkv, D, S), dtype=torch.uint8, device="cuda")
+    buf = torch.empty(rows * (D + 1) + 4, dtype=torch.float32, device="cuda")
+    done = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for off in range(4):
+        slots = [torch.full((rows, D + 1), float("nan"), device="cuda") for _ in range(world)]
+        flags = torch.zeros(world, dtype=torch.int32, device="cuda")
+        p_slots = (ctypes.c_void_p * world)(*[t.data_ptr() for t in slots])
+        p_flags = (ctypes.c_void_p * world)(*[flags.data_ptr() + 4 * r for r in range(world)])
+        rc = _lib.lib().rt_gqa_decode_record_push_bf16(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), buf.data_ptr() + 4 * off, p_slots, p_flags, world, 5, done.data_ptr(), B, Hq, Hkv,
+            D, S, None, S, 0, -1, -1.0, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        torch.cuda.synchronize()
+        rec = buf[off:off + rows * (D + 1)].view(rows, D + 1)
+        # another cut rounds P to bf16 against other running maxima: 2^-9 a weight, 2^-9 / sqrt(keys) an element, times 16
+        assert (rec - want).abs().max().item() < 1e-3
+        assert all(torch.equal(t, rec) for t in slots) and flags.tolist() == [5] * world and int(done.item()) == 0
+
+
 @pytest.mark.skipif("RT_ATTN_DECODE_CLUSTER" in os.environ, reason="the child process itself")
 @pytest.mark.parametrize("size", ["2", "4", "8", "16"])
 def test_every_cluster_size(size):
