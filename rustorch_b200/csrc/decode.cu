@@ -946,7 +946,8 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
     if (kv_end >= 0 && kv_end - kv_begin < span) span = kv_end - kv_begin;
     if (span < 1) span = 1;
     const bool tc = decode_use_tensor_cores() && batch * n_kv * max_seq < (1ll << 31) - 64;
-    p.split = pick_split(batch, n_kv, head_dim, max_seq, span, kv_lens != nullptr);
+    const DecodeSplit chunks = pick_split(batch, n_kv, head_dim, max_seq, span, kv_lens != nullptr);
+    p.split = chunks;
     // A cluster's record goes to the peers through the copy kernel, whose 16-byte pieces want it aligned; merge_partials_kernel
     // delivers a record at any address.
     const bool record_aligned = !push || (reinterpret_cast<uintptr_t>(out_f32) & 15) == 0;
@@ -965,18 +966,14 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
     int* counters = p.part_lse ? reinterpret_cast<int*>(p.part_lse + (int64_t)decode_num_chunks(batch, n_kv, max_seq) * p.rows)
                                : nullptr;
     bool merged = false;
-    if (tail) {  // the caller merges the chunk partials itself (split-KV row exchange)
-        counters = nullptr;
-        tail->n_chunks = p.split.mode == kSplitCluster ? 1 : p.split.n_chunks;  // (a cluster writes the merged rows)
-        tail->part_o = p.part_o;
-        tail->part_lse = p.part_lse;
-    }
+    if (tail) counters = nullptr;  // the caller merges the chunk partials itself (split-KV row exchange)
     cudaError_t e = cudaErrorNotSupported;
     if (decode_use_tensor_cores())
         e = launch_gqa_decode_tc(q, k, v, out_bf16, out_f32, lse, batch, n_heads, n_kv, head_dim, max_seq, kv_lens,
                                  kv_len_uniform, kv_begin, kv_end, scale, p.part_o, p.part_lse, counters, p.split,
                                  p.of_stride, p.lse_stride, &merged, push, stream);
-    if (e == cudaErrorNotSupported) {  // a cache too large for 32-bit TMA row coordinates, or RT_ATTN_DECODE_IMPL=simt
+    if (e == cudaErrorNotSupported) {  // a cache too large for 32-bit TMA row coordinates, no tensor map, or RT_ATTN_DECODE_IMPL=simt
+        p.split = chunks;              // this kernel has no clusters, and a cluster may have more parts than the scratch holds
         switch (head_dim) {
             case 64: e = launch_decode_d<64>(p, group, batch, stream); break;
             case 128: e = launch_decode_d<128>(p, group, batch, stream); break;
@@ -985,6 +982,11 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
         }
     }
     if (e != cudaSuccess) return e;
+    if (tail) {
+        tail->n_chunks = p.split.mode == kSplitCluster ? 1 : p.split.n_chunks;  // (a cluster writes the merged rows)
+        tail->part_o = p.part_o;
+        tail->part_lse = p.part_lse;
+    }
     if (merged && p.split.mode != kSplitCluster && push && push->world > 0 && pushed) *pushed = true;  // delivered by the decode kernel itself
     if (p.split.n_chunks > 1 && !merged && !tail) {
         e = launch_merge_partials(p.part_o, p.part_lse, p.split.n_chunks, p.rows, head_dim, head_dim, 1, p.out_bf16, p.out_f32, lse,

@@ -695,7 +695,7 @@ cudaError_t launch_gqa_decode_tc(const void* q, const void* k, const void* v, vo
                                  float scale, float* part_o, float* part_lse, int* counters, const DecodeSplit& split,
                                  int64_t of_stride, int64_t lse_stride, bool* merged, const MergePush* push,
                                  cudaStream_t stream) {
-    *merged = split.mode == kSplitCluster;
+    *merged = false;
     const int64_t cache_rows = batch * n_kv * max_seq;
     if ((head_dim != 64 && head_dim != 128 && head_dim != 256) || cache_rows >= (1ll << 31) - 64)
         return cudaErrorNotSupported;
@@ -760,6 +760,7 @@ cudaError_t launch_gqa_decode_tc(const void* q, const void* k, const void* v, vo
         *merged = true;
         if (push) p.push = *push;
     }
+    if (split.mode == kSplitCluster) *merged = true;
     return head_dim == 256   ? launch_d<256>(mk, mv, p, n_heads / n_kv, batch, stream)
            : head_dim == 128 ? launch_d<128>(mk, mv, p, n_heads / n_kv, batch, stream)
                              : launch_d<64>(mk, mv, p, n_heads / n_kv, batch, stream);
