@@ -974,6 +974,7 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
                                  p.of_stride, p.lse_stride, &merged, push, stream);
     if (e == cudaErrorNotSupported) {  // a cache too large for 32-bit TMA row coordinates, no tensor map, or RT_ATTN_DECODE_IMPL=simt
         p.split = chunks;              // this kernel has no clusters, and a cluster may have more parts than the scratch holds
+        merged = false;
         switch (head_dim) {
             case 64: e = launch_decode_d<64>(p, group, batch, stream); break;
             case 128: e = launch_decode_d<128>(p, group, batch, stream); break;
