@@ -107,10 +107,10 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
                                          const Bwd5Params& p, uint8_t* smem, int warp, int lane, int cta, int n_ctas) {
     using C = BwdCfg<D>;
     constexpr int TILE = C::TILE_BYTES, SUB = C::SUB_BYTES, STAGES = C::STAGES, HALFT = C::HALF_BYTES, HSUB = C::HSUB_BYTES;
-    // Where TMEM has room behind the accumulators, the A operands have columns of their own (per buffer P^T and dS^T, or
-    // dS, 32 each): the score MMAs of step u + 2 then follow the reading of T(u), not the accumulating MMAs of step u.
+    // On the query side at D = 128 dS has columns of its own behind the accumulator (32 per buffer): the score MMAs of step
+    // u + 2 then follow the reading of T(u), not the accumulating MMAs of step u.
     constexpr bool kApart = !kKeySide && D == 128;
-    constexpr uint32_t COL_A = C::COL_ACC + (kKeySide ? 2 : 1) * D, A_BUF = kKeySide ? 64 : 32;
+    constexpr uint32_t COL_A = C::COL_ACC + D, A_BUF = 32;
     static_assert(!kApart || COL_A + 2 * A_BUF <= 512, "TMEM columns");
     uint8_t* sX1 = smem;
     uint8_t* sX2 = sX1 + TILE;
@@ -335,9 +335,8 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t y1 = dy + (uint64_t)((st * 2 * HALFT) >> 4), y2 = y1 + (uint64_t)(HALFT >> 4);
-                    // P^T, dS^T (or dS): contiguous, or the first 16 of every 32 columns of T1 and T2
-                    const uint32_t a1 = kApart ? tmem_base + COL_A + b * A_BUF : tT + b * 128;
-                    const uint32_t a2 = kApart ? (kKeySide ? a1 + 32 : a1) : a1 + 64;
+                    // P^T and dS^T (or dS): the first 16 of every 32 columns of T1 and T2, or contiguous
+                    const uint32_t a1 = tT + b * 128, a2 = kApart ? tmem_base + COL_A + b * A_BUF : a1 + 64;
                     auto k16 = [](int kk) { return (uint32_t)(kk * 8 + (!kApart && kk >= 2 ? 16 : 0)); };
                     const uint32_t acc0 = u > 0 ? 1u : 0u;
                     if (kKeySide) {
@@ -468,11 +467,9 @@ __device__ __forceinline__ void bwd_side(const CUtensorMap* tm_x1, const CUtenso
                 if (diag || ragged) columns(std::true_type{});
                 else columns(std::false_type{});
                 if constexpr (kApart) {
-                    const uint32_t to = tmem_base + lane_sel + COL_A + buf * A_BUF + half * 16;
-                    if (kKeySide) tmem_st16(to, pk_p);
-                    tmem_st16(to + (kKeySide ? 32 : 0), pk_ds);
+                    tmem_st16(tmem_base + lane_sel + COL_A + buf * A_BUF + half * 16, pk_ds);
                 } else {  // into the first 16 of this thread's own 32 columns (in registers by now)
-                    tmem_st16(t1 + cbase, pk_p);
+                    if (kKeySide) tmem_st16(t1 + cbase, pk_p);
                     tmem_st16(t2 + cbase, pk_ds);
                 }
             }
