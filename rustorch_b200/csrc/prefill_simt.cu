@@ -422,7 +422,15 @@ static cudaError_t launch_tiled(SimtParams p, int64_t batch, cudaStream_t stream
     // In us: a step of 64 keys per group, per CTA, and for the merge across a cluster.
     p.split = 1;
     if constexpr (G == 2) {
-        if (n < 2 * (int64_t)sm_count()) {
+        // RT_ATTN_PREFILL_F32_CLUSTER=1|2|4|8 takes that many for every launch (read once per process).
+        static const int env = [] {
+            const char* e = getenv("RT_ATTN_PREFILL_F32_CLUSTER");
+            const int c = e ? atoi(e) : 0;
+            return c == 1 || c == 2 || c == 4 || c == 8 ? c : 0;
+        }();
+        if (env > 0) {
+            if (n * env <= 0x7fffffff && (env == 1 || f32_cluster_slots(env) > 0)) p.split = env;
+        } else if (n < 2 * (int64_t)sm_count()) {
             const double step = 1.0 + 0.1 * p.dim, cta = 3.0, merge = 4.0;
             const int64_t all = (p.seq_kv + simt::kRows - 1) / simt::kRows,
                           off = p.causal && p.q_offsets && p.seq_kv > p.seq_q ? p.seq_kv - p.seq_q : 0;

@@ -14,6 +14,23 @@ from tests.test_gpu_overrides import run_tests_with
 pytestmark = pytest.mark.gpu
 
 
+def _check_scratch(q, k, v, lens, want):
+    """Under an override that sets a cluster's size no chunk partial is written: the launch took clusters."""
+    import torch
+    import rustorch_b200 as rt
+    from rustorch_b200 import _lib
+    size = int(os.environ.get("RT_ATTN_DECODE_CLUSTER", "0"))
+    if size == 0:
+        return
+    (B, Hq, D), (Hkv, S) = q.shape, k.shape[1:3]
+    ws = torch.full((rt.decode_workspace_bytes(B, Hq, Hkv, D, S),), 0xff, dtype=torch.uint8, device="cuda")
+    out = torch.empty_like(want)
+    rc = _lib.lib().rt_gqa_decode_bf16(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), None, None, B, Hq, Hkv, D, S,
+                                       lens.data_ptr(), 0, 0, -1, -1.0, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0 and torch.equal(out, want) and ws.numel() > 0 and bool((ws == 0xff).all())
+
+
 @pytest.mark.parametrize("D", [64, 128, 256])
 @pytest.mark.parametrize("G,Hkv", [(1, 2), (2, 1), (4, 2), (8, 1)])
 def test_cluster_parts(oracle, D, G, Hkv):
@@ -29,14 +46,19 @@ def test_cluster_parts(oracle, D, G, Hkv):
     for b, n in enumerate(lens):
         dk[b, :, n:] = float("nan")
         dv[b, :, n:] = float("nan")
-    out, lse = rt.gqa_decode(dq, dk, dv, kv_lens=util.to_cuda(lens))
-    f32, _ = rt.gqa_decode(dq, dk, dv, kv_lens=util.to_cuda(lens), out_dtype=torch.float32)
-    rec = rt.gqa_decode_record(dq, dk, dv, kv_lens=util.to_cuda(lens))
-    torch.cuda.synchronize()
-    util.check_output(util.to_np(out), ref)
-    util.check_lse(util.to_np(lse), ref_lse)
-    assert torch.equal(f32.to(torch.bfloat16), out)
-    assert torch.equal(rec[:, :D], f32.reshape(-1, D)) and torch.equal(rec[:, D], lse.reshape(-1))
+    # all of them, and pairs: 16 CTAs of D = 256 for each of 16 (sequence, KV head) groups are not resident at once
+    for part in [slice(0, B)] + [slice(i, i + 2) for i in range(0, B, 2)]:
+        tq, tk, tv, tl = dq[part], dk[part], dv[part], util.to_cuda(lens[part])
+        out, lse = rt.gqa_decode(tq, tk, tv, kv_lens=tl)
+        f32, _ = rt.gqa_decode(tq, tk, tv, kv_lens=tl, out_dtype=torch.float32)
+        rec = rt.gqa_decode_record(tq, tk, tv, kv_lens=tl)
+        torch.cuda.synchronize()
+        util.check_output(util.to_np(out), ref[part])
+        util.check_lse(util.to_np(lse), ref_lse[part])
+        assert torch.equal(f32.to(torch.bfloat16), out)
+        assert torch.equal(rec[:, :D], f32.reshape(-1, D)) and torch.equal(rec[:, D], lse.reshape(-1))
+        if part.stop - part.start == 2:
+            _check_scratch(tq, tk, tv, tl, out)
     # one sequence, the length known to the host
     out1, lse1 = rt.gqa_decode(dq[-1:], dk[-1:], dv[-1:], kv_len=int(lens[-1]))
     util.check_output(util.to_np(out1), ref[-1:])
