@@ -34,9 +34,10 @@
 // results go back into the first 16 of its OWN columns, so the two threads of a row never touch each other's
 // inputs, and the accumulating MMAs take K elements 0-31 from columns [0,16) and 32-63 from [32,48));
 // warp 8 TMA producer, warp 9 TMEM allocation and the accumulating MMAs, warp 10 the score MMAs, warp 11 the columns' statistics.
-// What bounds a step: the MMAs on the key side at D = 128 (1270 clocks of 1280), MMAs and their hand-over on its query side (1140 of
-// 1024), the element-wise chain at D = 64 (1030 and 980 for 640 and 512 of MMA); between two items the read-out, 4000 clocks of f32
-// stores at D = 128, and the refill.
+// What bounds a step, by its clocks and those of its MMAs at the rates of back-to-back issue: the MMAs on the key side at
+// D = 128 (1270 and 1280: the pipe does not idle), MMAs and their hand-over on its query side (1140 and 1024), the element-wise
+// chain at D = 64 (key side 1030 and 640, query side 980 and 512); between two items the read-out, 4000 clocks of f32 stores at
+// D = 128, and the refill.
 // Every mbarrier wait is bounded; on expiry the kernel records a code in the device status word and
 // leaves through the common teardown.
 #include <cuda.h>

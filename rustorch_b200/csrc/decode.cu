@@ -839,7 +839,6 @@ static cudaError_t launch_decode_d(const DecodeParams& p, int group, int64_t bat
 //    lengths fill the cache).  Up to 2048 tokens at fixed places.
 static DecodeSplit pick_split(int64_t batch, int n_kv, int head_dim, int64_t max_seq, int64_t span, bool ragged) {
     DecodeSplit sp{};
-
     sp.chunk = decode_chunk_tokens(batch, n_kv, max_seq);
     const int64_t groups = batch * (int64_t)n_kv, slots = (int64_t)sm_count() * (head_dim == 64 ? 4 : head_dim == 128 ? 2 : 1);
     const int64_t whole = (span + 63) / 64 * 64, group_bytes = span * head_dim * 4;
@@ -972,8 +971,10 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
         e = launch_gqa_decode_tc(q, k, v, out_bf16, out_f32, lse, batch, n_heads, n_kv, head_dim, max_seq, kv_lens,
                                  kv_len_uniform, kv_begin, kv_end, scale, p.part_o, p.part_lse, counters, p.split,
                                  p.of_stride, p.lse_stride, &merged, push, stream);
-    if (e == cudaErrorNotSupported) {  // a cache too large for 32-bit TMA row coordinates, no tensor map, or RT_ATTN_DECODE_IMPL=simt
-        p.split = chunks;              // this kernel has no clusters, and a cluster may have more parts than the scratch holds
+    // A cache too large for 32-bit TMA row coordinates, no tensor map, or RT_ATTN_DECODE_IMPL=simt.  This kernel has no clusters,
+    // and a cluster may have more parts than the scratch holds.
+    if (e == cudaErrorNotSupported) {
+        p.split = chunks;
         merged = false;
         switch (head_dim) {
             case 64: e = launch_decode_d<64>(p, group, batch, stream); break;
@@ -988,7 +989,8 @@ cudaError_t launch_gqa_decode(const void* q, const void* k, const void* v, void*
         tail->part_o = p.part_o;
         tail->part_lse = p.part_lse;
     }
-    if (merged && p.split.mode != kSplitCluster && push && push->world > 0 && pushed) *pushed = true;  // delivered by the decode kernel itself
+    // delivered by the decode kernel itself
+    if (merged && p.split.mode != kSplitCluster && push && push->world > 0 && pushed) *pushed = true;
     if (p.split.n_chunks > 1 && !merged && !tail) {
         e = launch_merge_partials(p.part_o, p.part_lse, p.split.n_chunks, p.rows, head_dim, head_dim, 1, p.out_bf16, p.out_f32, lse,
                                   stream, nullptr, push, p.of_stride, p.lse_stride);

@@ -14,9 +14,10 @@
 //     (warp-uniformly) when no row maximum moved.
 // One CTA = 4 independent warps = one (sequence, KV head, chunk); warp states are merged through
 // shared memory and written as a normalised (O f32, LSE) partial, or as the final output when
-// the launch has a single chunk.  With kCluster > 0 the sequence's CTAs are a cluster that merges its partial rows
-// through distributed shared memory (merge_decode_cluster; which launches: pick_cluster in decode.cu).  Rows past the visible range are masked in the scores and
-// zeroed in V (uninitialised cache memory may hold NaN bit patterns).  Waits are bounded.
+// the launch has a single chunk.  With kCluster > 0 the sequence's CTAs are a cluster that merges its
+// partial rows through distributed shared memory (merge_decode_cluster; which launches: pick_cluster in
+// decode.cu).  Rows past the visible range are masked in the scores and zeroed in V (uninitialised
+// cache memory may hold NaN bit patterns).  Waits are bounded.
 #include <atomic>
 #include <cuda.h>
 #include <cstdlib>

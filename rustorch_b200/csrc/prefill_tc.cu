@@ -25,9 +25,10 @@
 // steps; P (bf16) overwrites the first 32 columns of its S buffer and feeds the PV MMA from TMEM.
 // S = Q K^T is an SS MMA with both operands K-major in 128-byte-swizzled shared memory; O += P V
 // is a TS MMA whose B operand (V) is MN-major, i.e. V is used exactly as TMA lands it.
-// The normalised O tile is staged in shared memory (at D = 64 in a buffer of its own, at D = 128, where the rings
-// leave no room, in the tile's by then idle Q buffer) and leaves through TMA stores.  Every mbarrier wait is bounded; on expiry the kernel records a code in the device
-// status word, drains its own copies and MMAs, frees TMEM and returns.
+// The normalised O tile is staged in shared memory (at D = 64 in a buffer of its own, at D = 128, where
+// the rings leave no room, in the tile's by then idle Q buffer) and leaves through TMA stores.  Every
+// mbarrier wait is bounded; on expiry the kernel records a code in the device status word, drains its
+// own copies and MMAs, frees TMEM and returns.
 #include <algorithm>
 #include <atomic>
 #include <cuda.h>
@@ -321,9 +322,10 @@ __device__ __forceinline__ void merge_cluster(const TcParams& p, const TcItem& i
 // retired only if PV(u) has, so a softmax warp that moves the reference maximum at step u+1 reads 'O is at rest' off
 // the barrier of the next scores; only an item's last step but one has a commit for it (o_full).
 // Per item and tile: q_full (Q landed) -> ... -> o_done (last PV retired) -> epilogue reads O
-// (o_free: the next item's first PV may overwrite it), stages it (stage_full), and one thread stores it.  q_empty, the
-// next item's Q may land: at D = 64 behind the item's last score MMA, at D = 128 when the store has read the staged tile.  A tile that sees no key in an
-// item takes no part in these (its rows are written as NaN directly).
+// (o_free: the next item's first PV may overwrite it), stages it (stage_full), and one thread stores it.
+// q_empty, the next item's Q may land: at D = 64 behind the item's last score MMA, at D = 128 when the store has
+// read the staged tile.  A tile that sees no key in an item takes no part in these (its rows are written as
+// NaN directly).
 template <int D, bool kCausal, bool kKeep, bool kSingle, bool kSplit, bool kByLength>
 __global__ void __launch_bounds__(384, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
