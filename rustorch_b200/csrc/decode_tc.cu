@@ -296,7 +296,7 @@ __device__ __forceinline__ void merge_decode_cluster(const DecodeTcParams& p, in
             float* dst = p.out_f32 + row * p.of_stride + d;  // (records: rows of D + 1 floats)
             dst[0] = o.x, dst[1] = o.y, dst[2] = o.z, dst[3] = o.w;
         }
-        if (d == 0 && p.lse) p.lse[row * p.lse_stride] = any ? (m + fast_log2(l)) * kLn2 : -INFINITY;
+        if (d == 0 && p.lse) p.lse[row * p.lse_stride] = any ? fmaf(m, kLn2, logf(l)) : -INFINITY;
     }
     decode_cluster_sync();  // no CTA leaves while its partial rows are being read
 }
