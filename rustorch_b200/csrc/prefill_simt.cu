@@ -149,8 +149,8 @@ __global__ void __launch_bounds__(kSimtRows * 32) prefill_f32_kernel(const SimtP
 // 520 -> 218 us, B=4 H=16 N=1024 D=64 656 -> 408 us (42 TFLOP/s of the FP32 pipe's 74).
 // Launches of few row blocks leave SMs idle while each block walks its keys alone; there a cluster of 2, 4 or 8 CTAs shares
 // them (kSplit): each takes every split-th pair of tiles, leaves its partial rows in shared memory, and merges 64 / split rows out
-// of all of them.  (N=2048 D=64 causal, H=1 121 -> 40 us, H=2 122 -> 55; B=1 H=4 N=600 D=80 56 -> 44, 38, 52 and 41 since; the merge costs about half
-// a step.)
+// of all of them.  (N=2048 D=64 causal, H=1 112 -> 37 us, H=2 112 -> 52; H=4 N=600 D=80 without a mask 51 -> 41; H=2 64 rows
+// against 4096 keys D=128 402 -> 64; the merge costs about half a step.)
 __device__ __forceinline__ void f32_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
